@@ -1,9 +1,9 @@
-// APIC particle-to-grid and grid-to-particle transfers, one thread per
-// particle, accumulating straight into HBM with atomics.  This is the plain
-// form of Picasso_APIC.hpp (and the path taken for unsorted particles); the
-// per-particle bodies are in plain.cuh, the shared-memory tiled kernels for
-// binned particles in tiled.cu.
+// APIC particle-to-grid and grid-to-particle transfers of the plain form of
+// Picasso_APIC.hpp, for particles in any order: FP64 P2G by warps (warp_p2g.cuh),
+// the fixed-point P2G and the G2P by one thread per particle (plain.cuh).  The
+// shared-memory tiled FP32 kernels for binned particles are in tiled.cu.
 #include "plain.cuh"
+#include "warp_p2g.cuh"
 
 namespace pb {
 
@@ -31,6 +31,32 @@ apic_g2p_kernel(MeshP mp, int64_t n, PField x, GField u, PField c, int stag, int
                                                                    &adv);
 }
 
+// FP64 P2G: 4-warp CTAs, each warp one segment of `seg` consecutive particles.
+constexpr int kWarpP2GWarps = 4;
+
+template <int ORDER, int NC, bool STAG>
+__global__ void __launch_bounds__(32 * kWarpP2GWarps, ORDER == 3 ? 3 : 4)
+apic_p2g_warp_kernel(MeshP mp, int64_t n, int64_t seg, PField x, PField m, PField c, bool wide,
+                     GField gm, GField gmu, int stag, int* err)
+{
+    using W = WarpP2G<ORDER, NC, STAG>;
+    __shared__ __align__(16) double sm[kWarpP2GWarps][W::DOUBLES];
+    const int warp = threadIdx.x >> 5;
+    const int64_t a = ((int64_t)blockIdx.x * kWarpP2GWarps + warp) * seg;
+    if (a < n)
+        apic_p2g_warp<ORDER, NC, STAG>(mp, a, min(a + seg, n), x, m, c, wide, gm, gmu, stag, err,
+                                       sm[warp]);
+}
+
+// Particles per warp: 256 (long enough that the flush at a segment's end is a
+// small part, 108 grid additions per quadratic segment), less -- at least 8 --
+// when the particles would not give every SM 16 warps.
+static int64_t warp_segment(int64_t n)
+{
+    const int64_t seg = (n / (148 * 16) + 7) / 8 * 8;
+    return seg < 8 ? 8 : (seg > 32 ? (seg > 256 ? 256 : seg / 32 * 32) : seg);
+}
+
 // ---------------------------------------------------------------------------
 // dispatch
 // ---------------------------------------------------------------------------
@@ -42,8 +68,10 @@ static void launch_p2g(Form form, const MeshP& mp, int64_t n, const PField& x, c
     const int threads = 256;
     const unsigned blocks = grid_for(n, threads);
     if (form == Form::F64) {
-        apic_p2g_kernel<ORDER, NC, STAG, double, double, AccF64><<<blocks, threads, 0, st>>>(
-            mp, n, x, m, c, gm, gmu, stag, 0.0, 0.0, err);
+        const int64_t seg = warp_segment(n);
+        const int64_t ctas = (n + seg * kWarpP2GWarps - 1) / (seg * kWarpP2GWarps);
+        apic_p2g_warp_kernel<ORDER, NC, STAG><<<(unsigned)ctas, 32 * kWarpP2GWarps, 0, st>>>(
+            mp, n, seg, x, m, c, wide_rows<STAG ? 3 : NC>(c), gm, gmu, stag, err);
     } else if (form == Form::F32Fixed) {
         apic_p2g_kernel<ORDER, NC, STAG, float, float, AccFixed><<<blocks, threads, 0, st>>>(
             mp, n, x, m, c, gm, gmu, stag, ldexpf(1.0f, gm.fixed_bits),

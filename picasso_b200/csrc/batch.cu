@@ -21,8 +21,8 @@
 // registers of its own phase only).
 //
 // Work items reuse the single-call bodies: tiled P2G / G2P (tiled.cuh) for the
-// precision form, the per-particle plain transfers (plain.cuh) on sorted
-// particles for FP64, the per-node velocity update (gridops.cuh).
+// precision form, the warp P2G (warp_p2g.cuh) and the per-particle plain G2P
+// (plain.cuh) for FP64, the per-node velocity update (gridops.cuh).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -33,6 +33,7 @@
 #include "gridops.cuh"
 #include "plain.cuh"
 #include "tiled.cuh"
+#include "warp_p2g.cuh"
 
 namespace pb {
 
@@ -158,12 +159,35 @@ __device__ __noinline__ void g2p_item_call(const G2PArgs& A, int64_t t, int64_t 
     g2p_item<ORDER, NT>(A, t, a, b, tile, tid);
 }
 
+// FP64 P2G item: each warp takes a contiguous part of it (apic_p2g_warp); smem
+// holds one table per warp.
 template <int ORDER, int NT>
-__device__ __noinline__ void plain_p2g_call(const BInst& I, int64_t a, int64_t b, int tid)
+__device__ __forceinline__ void warp_p2g_item(const BInst& I, int64_t a, int64_t b, float* smem,
+                                              int tid)
 {
-    for (int64_t p = a + tid; p < b; p += NT)
-        apic_p2g_particle<ORDER, 3, false, double, double, AccF64>(
-            I.p2g.mp, p, I.x, I.m, I.c, I.gm, I.gmu, -1, 0.0, 0.0, I.p2g.err);
+    using W = WarpP2G<ORDER, 3, false>;
+    const int64_t seg = (b - a + NT - 1) / NT * 32;
+    const int64_t lo = a + (tid >> 5) * seg;
+    if (lo < b)
+        apic_p2g_warp<ORDER, 3, false>(I.p2g.mp, lo, min(lo + seg, b), I.x, I.m, I.c, true, I.gm,
+                                       I.gmu, -1, I.p2g.err,
+                                       reinterpret_cast<double*>(smem) + (tid >> 5) * W::DOUBLES);
+}
+
+template <int ORDER, int NT>
+__device__ __noinline__ void warp_p2g_call(const BInst& I, int64_t a, int64_t b, float* smem,
+                                           int tid)
+{
+    warp_p2g_item<ORDER, NT>(I, a, b, smem, tid);
+}
+
+// Shared bytes of one warp's FP64 P2G table.
+static int warp_p2g_bytes(int order)
+{
+    const int d = order == 1 ? WarpP2G<1, 3, false>::DOUBLES
+                             : (order == 2 ? WarpP2G<2, 3, false>::DOUBLES
+                                           : WarpP2G<3, 3, false>::DOUBLES);
+    return d * (int)sizeof(double);
 }
 
 template <int ORDER, int NT>
@@ -205,9 +229,7 @@ __device__ void p2g_batch_item(const BInst& I, uint32_t local, float* smem, int*
             const P2GArgs& A = stage_args<P2GArgs, NT>(I.p2g, args, tid);
             p2g_item<O, kVarLanes[VAR]>(A, t, a, b, smem, stage_base);
         } else {
-            for (int64_t p = a + tid; p < b; p += NT)
-                apic_p2g_particle<O, 3, false, double, double, AccF64>(
-                    I.p2g.mp, p, I.x, I.m, I.c, I.gm, I.gmu, -1, 0.0, 0.0, I.p2g.err);
+            warp_p2g_item<O, NT>(I, a, b, smem, tid);
         }
     } else if constexpr (F32) {
         static_assert(!F32 || NT == 32, "tiled P2G items are single-warp");
@@ -223,9 +245,9 @@ __device__ void p2g_batch_item(const BInst& I, uint32_t local, float* smem, int*
             default: p2g_item_call<3, 4>(A, t, a, b, smem, stage_base); break;
         }
     } else {
-        if (I.order == 1) plain_p2g_call<1, NT>(I, a, b, tid);
-        else if (I.order == 2) plain_p2g_call<2, NT>(I, a, b, tid);
-        else plain_p2g_call<3, NT>(I, a, b, tid);
+        if (I.order == 1) warp_p2g_call<1, NT>(I, a, b, smem, tid);
+        else if (I.order == 2) warp_p2g_call<2, NT>(I, a, b, smem, tid);
+        else warp_p2g_call<3, NT>(I, a, b, smem, tid);
     }
 }
 
@@ -542,6 +564,8 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     if (f32) {
         *smem_p2g = std::max(*smem_p2g, (int)p2g_warp_bytes(order, lpp, tp.P));
         *smem_g2p = std::max(*smem_g2p, (int)(sizeof(float4) * (size_t)tp.nodes));
+    } else {
+        *smem_p2g = std::max(*smem_p2g, warp_p2g_bytes(order));  // one warp's
     }
     return PICASSO_OK;
 }
@@ -570,7 +594,9 @@ extern "C" picasso_status picasso_batch_create(const picasso_batch_instance* ins
     b->count = count;
     b->f32 = f32;
     b->mode = mode;
-    b->smem[1] = smem_p2g;
+    // FP64 P2G CTAs of the phased step run several warps, each with a table
+    constexpr int kF64Warps = BatchShape<false, 0x2>::threads / 32;
+    b->smem[1] = f32 ? smem_p2g : kF64Warps * smem_p2g;
     b->smem[3] = smem_g2p;
     b->smem[kPhases] = std::max(smem_p2g, smem_g2p);
     b->inst.assign(instances, instances + count);
@@ -600,10 +626,10 @@ extern "C" picasso_status picasso_batch_create(const picasso_batch_instance* ins
                 const int v = var[i];
                 if (b->var_lo[v] == b->var_hi[v]) b->var_lo[v] = (uint32_t)q;
                 b->var_hi[v] = (uint32_t)(q + hinst[i].nitems[p]);
-                if (f32)
-                    b->var_smem[v] = std::max(b->var_smem[v],
-                                              (int)p2g_warp_bytes(hinst[i].order, hinst[i].lpp,
-                                                                  hinst[i].p2g.tp.P));
+                b->var_smem[v] =
+                    f32 ? std::max(b->var_smem[v], (int)p2g_warp_bytes(hinst[i].order, hinst[i].lpp,
+                                                                       hinst[i].p2g.tp.P))
+                        : kF64Warps * warp_p2g_bytes(hinst[i].order);
             }
             q += hinst[i].nitems[p];
         }

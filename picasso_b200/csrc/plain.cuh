@@ -1,7 +1,8 @@
 // Per-particle bodies of the plain APIC transfers: one thread handles one
-// particle and accumulates straight into HBM with atomics (the form of
-// Picasso_APIC.hpp applied per particle by GridOperator::apply).  Used by the
-// plain kernels (apic.cu) and by the batched kernel (batch.cu).
+// particle (the form of Picasso_APIC.hpp applied per particle by
+// GridOperator::apply); the fixed-point P2G accumulates straight into HBM with
+// atomics.  Used by the plain kernels (apic.cu), the G2P also by the batched
+// kernel (batch.cu).
 #pragma once
 
 #include "common.cuh"
