@@ -1,7 +1,9 @@
 // APIC particle-to-grid and grid-to-particle transfers of the plain form of
-// Picasso_APIC.hpp, for particles in any order: FP64 P2G by warps (warp_p2g.cuh),
-// the fixed-point P2G and the G2P by one thread per particle (plain.cuh).  The
-// shared-memory tiled FP32 kernels for binned particles are in tiled.cu.
+// Picasso_APIC.hpp, for particles in any order: FP64 by warps (warp_p2g.cuh,
+// g2p_f64.cuh; the latter with a node tile for binned particles), the fixed-point
+// P2G and FP32 G2P by one thread per particle (plain.cuh).  The shared-memory
+// tiled FP32 kernels for binned particles are in tiled.cu.
+#include "g2p_f64.cuh"
 #include "plain.cuh"
 #include "warp_p2g.cuh"
 
@@ -27,8 +29,51 @@ apic_g2p_kernel(MeshP mp, int64_t n, PField x, GField u, PField c, int stag, int
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
-        apic_g2p_particle<ORDER, NC, STAG, GT, PT, R, false, ADV>(mp, p, x, u, c, stag, err,
-                                                                   &adv);
+        apic_g2p_particle<ORDER, NC, STAG, GT, PT, R, ADV>(mp, p, x, u, c, stag, err, &adv);
+}
+
+// FP64 G2P: grid-stride over 32 particles per warp.
+template <int ORDER, int NC, bool STAG, bool ADV, bool UNIT>
+__global__ void __launch_bounds__(128, 4)
+apic_g2p_f64_kernel(MeshP mp, int64_t n, PField x, GField u, PField c, int stag, int* err,
+                    Advect adv, bool packed)
+{
+    using R = WarpRows<STAG ? 3 : NC, ADV>;
+    __shared__ double rows[4][R::DOUBLES];
+    const int warp = threadIdx.x >> 5;
+    double* mine = packed ? rows[warp] : nullptr;
+    const int64_t stride = (int64_t)gridDim.x * 128;
+    for (int64_t p0 = (int64_t)blockIdx.x * 128 + warp * 32; p0 < n; p0 += stride)
+        apic_g2p_warp<ORDER, NC, STAG, false, ADV, UNIT, false>(
+            mp, p0, (int)min((int64_t)32, n - p0), x, u, c, stag, err, &adv, mine);
+}
+
+// FP64 G2P of cell-sorted particles: one CTA per work item of the bins.  The
+// particles past the last item (out of the mesh at the sort) are taken from
+// global memory by all CTAs.
+template <int ORDER, bool ADV>
+__global__ void __launch_bounds__(128, 4)
+apic_g2p_tiled_f64_kernel(MeshP mp, TileP tp, int64_t n, PField x, GField u, PField c, int* err,
+                          Advect adv, bool packed)
+{
+    using R = WarpRows<3, ADV>;
+    extern __shared__ __align__(16) double g2p_nodes[];  // 3 per tile node
+    __shared__ double rows[4][R::DOUBLES];
+    const int tid = threadIdx.x;
+    int64_t t, a, b;
+    if (item_range(tp, blockIdx.x, t, a, b)) {
+        b = min(b, n);
+        if (a < b)
+            g2p_item_f64<ORDER, 128, false, ADV>(mp, tp, t, a, b, x, u, c, err, &adv, g2p_nodes,
+                                                       packed ? rows[0] : nullptr, tid);
+    }
+    const int64_t rest = __ldg(tp.off + tp.ntiles) + (int64_t)blockIdx.x * 128 + tid;
+    for (int64_t p = rest; p < n; p += (int64_t)gridDim.x * 128) {
+        const double xp[3] = {x.get<double>(p, 0), x.get<double>(p, 1), x.get<double>(p, 2)};
+        double up[3], B[3][3];
+        if (g2p_stray<ORDER, false>(mp, xp, u, up, B)) g2p_set<ADV>(p, xp, up, B, x, c, &adv);
+        else if (err) atomicAdd(err, 1);
+    }
 }
 
 // FP64 P2G: 4-warp CTAs, each warp one segment of `seg` consecutive particles.
@@ -88,26 +133,64 @@ template <int ORDER, int NC, bool STAG>
 static void launch_g2p(bool f32, const MeshP& mp, int64_t n, const PField& x, const GField& u,
                        const PField& c, int stag, int* err, const Advect* adv, cudaStream_t st)
 {
+    const Advect a = adv ? *adv : Advect{};
+    if (!f32) {
+        const unsigned blocks = grid_for(n, 128, 148LL * 64);
+        const bool packed = packed_rows_f64(x, c, 4 * (STAG ? 3 : NC), adv != nullptr);
+        auto launch = [&](auto kern) {
+            kern<<<blocks, 128, 0, st>>>(mp, n, x, u, c, stag, err, a, packed);
+        };
+        if constexpr (STAG || NC == 1) {  // one component: nothing to be adjacent
+            launch(apic_g2p_f64_kernel<ORDER, NC, STAG, false, true>);
+        } else {
+            const bool unit = u.s[3] == 1;
+            if constexpr (NC == 3) {
+                if (adv) {
+                    if (unit) launch(apic_g2p_f64_kernel<ORDER, NC, STAG, true, true>);
+                    else launch(apic_g2p_f64_kernel<ORDER, NC, STAG, true, false>);
+                    return;
+                }
+            }
+            if (unit) launch(apic_g2p_f64_kernel<ORDER, NC, STAG, false, true>);
+            else launch(apic_g2p_f64_kernel<ORDER, NC, STAG, false, false>);
+        }
+        return;
+    }
     const int threads = 256;
     const unsigned blocks = grid_for(n, threads);
-    const Advect a = adv ? *adv : Advect{};
     if constexpr (NC == 3 && !STAG) {
         if (adv) {
-            if (f32)
-                apic_g2p_kernel<ORDER, NC, STAG, float, float, float, true>
-                    <<<blocks, threads, 0, st>>>(mp, n, x, u, c, stag, err, a);
-            else
-                apic_g2p_kernel<ORDER, NC, STAG, double, double, double, true>
-                    <<<blocks, threads, 0, st>>>(mp, n, x, u, c, stag, err, a);
+            apic_g2p_kernel<ORDER, NC, STAG, float, float, float, true>
+                <<<blocks, threads, 0, st>>>(mp, n, x, u, c, stag, err, a);
             return;
         }
     }
-    if (f32)
-        apic_g2p_kernel<ORDER, NC, STAG, float, float, float, false><<<blocks, threads, 0, st>>>(
-            mp, n, x, u, c, stag, err, a);
-    else
-        apic_g2p_kernel<ORDER, NC, STAG, double, double, double, false>
-            <<<blocks, threads, 0, st>>>(mp, n, x, u, c, stag, err, a);
+    apic_g2p_kernel<ORDER, NC, STAG, float, float, float, false><<<blocks, threads, 0, st>>>(
+        mp, n, x, u, c, stag, err, a);
+}
+
+// FP64 G2P with bins (3 collocated components); *handled stays false when the
+// node tile does not fit in shared memory.
+template <int ORDER>
+static picasso_status launch_g2p_tiled_f64(const MeshP& mp, const TileP& tp, int64_t n,
+                                           const PField& x, const GField& u, const PField& c,
+                                           int* err, const Advect* adv, cudaStream_t st,
+                                           bool* handled)
+{
+    const size_t smem = 3 * sizeof(double) * (size_t)tp.nodes;
+    const size_t rows = 4 * sizeof(double) * (size_t)(adv ? WarpRows<3, true>::DOUBLES
+                                                          : WarpRows<3, false>::DOUBLES);
+    if ((int64_t)(smem + rows) > device_smem_optin()) return PICASSO_OK;
+    *handled = true;
+    const bool packed = packed_rows_f64(x, c, 12, adv != nullptr);
+    const int64_t items = tp.ntiles + (n + tp.chunk - 1) / tp.chunk;
+    auto launch = [&](auto kern) -> picasso_status {
+        PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, u, c, err, adv ? *adv : Advect{}, packed);
+        return check_launch();
+    };
+    if (adv) return launch(apic_g2p_tiled_f64_kernel<ORDER, true>);
+    return launch(apic_g2p_tiled_f64_kernel<ORDER, false>);
 }
 
 #define PB_ORDER_SWITCH(order, ...)               \
@@ -254,6 +337,12 @@ static picasso_status apic_g2p_entry(const picasso_spline* sd, int64_t num_parti
         st = apic_g2p_tiled(mp, sd->order, ncomp, f32, num_particles, x, u, c, *exec->bins, err,
                             ap, s, &handled, stag);
         if (st || handled) return st;
+        TileP tp;
+        if (!f32 && stag < 0 && ncomp == 3 && make_tilep(mp, sd->order, *exec->bins, &tp)) {
+            PB_ORDER_SWITCH(sd->order, st = launch_g2p_tiled_f64<O_>(mp, tp, num_particles, x, u, c,
+                                                                     err, ap, s, &handled));
+            if (st || handled) return st;
+        }
     }
     return apic_g2p_plain(mp, sd->order, stag, ncomp, f32, num_particles, x, u, c, err, ap, s);
 }

@@ -21,8 +21,8 @@
 // registers of its own phase only).
 //
 // Work items reuse the single-call bodies: tiled P2G / G2P (tiled.cuh) for the
-// precision form, the warp P2G (warp_p2g.cuh) and the per-particle plain G2P
-// (plain.cuh) for FP64, the per-node velocity update (gridops.cuh).
+// precision form, the warp P2G (warp_p2g.cuh) and G2P (g2p_f64.cuh) for
+// FP64, the per-node velocity update (gridops.cuh).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -30,8 +30,8 @@
 #include <numeric>
 #include <vector>
 
+#include "g2p_f64.cuh"
 #include "gridops.cuh"
-#include "plain.cuh"
 #include "tiled.cuh"
 #include "warp_p2g.cuh"
 
@@ -190,12 +190,18 @@ static int warp_p2g_bytes(int order)
     return d * (int)sizeof(double);
 }
 
-template <int ORDER, int NT>
-__device__ __noinline__ void plain_g2p_call(const BInst& I, int64_t a, int64_t b, int tid)
+// FP64 G2P item (g2p_item_f64); smem: a WarpRows buffer per warp, then the node
+// tile.  CG: u_i was written in this launch.
+constexpr int kWarpG2PBytes = WarpRows<3, false>::DOUBLES * (int)sizeof(double);
+
+template <int ORDER, int NT, bool CG>
+__device__ __noinline__ void g2p_f64_call(const BInst& I, int64_t t, int64_t a, int64_t b,
+                                          float* smem, int tid)
 {
-    for (int64_t p = a + tid; p < b; p += NT)
-        apic_g2p_particle<ORDER, 3, false, double, double, double, true>(I.g2p.mp, p, I.x, I.gu,
-                                                                         I.c, -1, I.g2p.err);
+    double* rows = reinterpret_cast<double*>(smem);
+    double* nodes = rows + NT / 32 * WarpRows<3, false>::DOUBLES;
+    g2p_item_f64<ORDER, NT, CG, false>(I.g2p.mp, I.g2p.tp, t, a, b, I.x, I.gu, I.c, I.g2p.err,
+                                       nullptr, nodes, rows, tid);
 }
 
 // Copies an argument block into shared memory with the NT threads of the
@@ -251,7 +257,7 @@ __device__ void p2g_batch_item(const BInst& I, uint32_t local, float* smem, int*
     }
 }
 
-template <bool F32, int NT>
+template <bool F32, int NT, bool CG>
 __device__ void g2p_batch_item(const BInst& I, uint32_t local, float* smem, G2PArgs* args,
                                int tid)
 {
@@ -267,9 +273,9 @@ __device__ void g2p_batch_item(const BInst& I, uint32_t local, float* smem, G2PA
         if (NT == 32) __syncwarp();  // the next item rewrites args
         else __syncthreads();
     } else {
-        if (I.order == 1) plain_g2p_call<1, NT>(I, a, b, tid);
-        else if (I.order == 2) plain_g2p_call<2, NT>(I, a, b, tid);
-        else plain_g2p_call<3, NT>(I, a, b, tid);
+        if (I.order == 1) g2p_f64_call<1, NT, CG>(I, t, a, b, smem, tid);
+        else if (I.order == 2) g2p_f64_call<2, NT, CG>(I, t, a, b, smem, tid);
+        else g2p_f64_call<3, NT, CG>(I, t, a, b, smem, tid);
     }
 }
 
@@ -338,7 +344,7 @@ batch_kernel(BatchDev B, uint32_t qlo, uint32_t qhi, int slot)
             if constexpr ((PMASK & 0x4) != 0)
                 if (ph == 2) velocity_item<F32, NT>(I, local, tid);
             if constexpr ((PMASK & 0x8) != 0)
-                if (ph == 3) g2p_batch_item<F32, NT>(I, local, smem, &s_g2p, tid);
+                if (ph == 3) g2p_batch_item<F32, NT, PMASK == 0xF>(I, local, smem, &s_g2p, tid);
         }
         if (PMASK == 0xF) {
             __threadfence();  // this item's writes before its completion count
@@ -566,6 +572,7 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
         *smem_g2p = std::max(*smem_g2p, (int)(sizeof(float4) * (size_t)tp.nodes));
     } else {
         *smem_p2g = std::max(*smem_p2g, warp_p2g_bytes(order));  // one warp's
+        *smem_g2p = std::max(*smem_g2p, 3 * (int)sizeof(double) * tp.nodes);  // the tile's
     }
     return PICASSO_OK;
 }
@@ -587,18 +594,22 @@ extern "C" picasso_status picasso_batch_create(const picasso_batch_instance* ins
         picasso_status st = make_instance(instances[i], f32, &hinst[i], &smem_p2g, &smem_g2p);
         if (st) return st;
     }
-    if (std::max(smem_p2g, smem_g2p) > device_smem_optin()) return PICASSO_ERR_UNSUPPORTED;
+    // FP64 CTAs of the phased transfers run several warps, each with its buffer
+    constexpr int kF64Warps = BatchShape<false, 0x2>::threads / 32;
+    const int p2g_bytes = f32 ? smem_p2g : kF64Warps * smem_p2g;
+    const int g2p_bytes = f32 ? smem_g2p : kF64Warps * kWarpG2PBytes + smem_g2p;
+    const int fused_bytes = std::max(smem_p2g, f32 ? smem_g2p : kWarpG2PBytes + smem_g2p);
+    if (std::max(std::max(p2g_bytes, g2p_bytes), fused_bytes) > device_smem_optin())
+        return PICASSO_ERR_UNSUPPORTED;
 
     picasso_batch* b = new (std::nothrow) picasso_batch();
     if (!b) return PICASSO_ERR_OUT_OF_RANGE;
     b->count = count;
     b->f32 = f32;
     b->mode = mode;
-    // FP64 P2G CTAs of the phased step run several warps, each with a table
-    constexpr int kF64Warps = BatchShape<false, 0x2>::threads / 32;
-    b->smem[1] = f32 ? smem_p2g : kF64Warps * smem_p2g;
-    b->smem[3] = smem_g2p;
-    b->smem[kPhases] = std::max(smem_p2g, smem_g2p);
+    b->smem[1] = p2g_bytes;
+    b->smem[3] = g2p_bytes;
+    b->smem[kPhases] = fused_bytes;
     b->inst.assign(instances, instances + count);
     // queue: phase-major, instances by decreasing particle count; in the P2G
     // phase grouped by variant first (one phased launch per variant)

@@ -1,8 +1,8 @@
 // Per-particle bodies of the plain APIC transfers: one thread handles one
 // particle (the form of Picasso_APIC.hpp applied per particle by
 // GridOperator::apply); the fixed-point P2G accumulates straight into HBM with
-// atomics.  Used by the plain kernels (apic.cu), the G2P also by the batched
-// kernel (batch.cu).
+// atomics.  Used by the plain kernels (apic.cu); FP64 has its own bodies
+// (warp_p2g.cuh, g2p_f64.cuh).
 #pragma once
 
 #include "common.cuh"
@@ -130,18 +130,15 @@ __device__ __forceinline__ void apic_p2g_particle(const MeshP& mp, int64_t p, co
 // G2P
 // ---------------------------------------------------------------------------
 // GT: grid storage type of u_i; PT: particle storage type of c_p.
-// CG: load u_i through L2 only (for grids written earlier in the same launch).
 // ADV (collocated, 3 components): then moves the particle, x += dt u_p with
 // the stored (PT-rounded) u_p, exactly as picasso_advect would afterwards.
-template <int ORDER, int NC, bool STAG, class GT, class PT, class R, bool CG = false,
-          bool ADV = false>
+template <int ORDER, int NC, bool STAG, class GT, class PT, class R, bool ADV = false>
 __device__ __forceinline__ void apic_g2p_particle(const MeshP& mp, int64_t p, const PField& x,
                                                   const GField& u, const PField& c, int stag,
                                                   int* err, const Advect* adv = nullptr)
 {
     constexpr int K = SplineTraits<ORDER>::K;
     constexpr int NCO = STAG ? 3 : NC;
-    auto load = [](const GT* a) { return CG ? __ldcg(a) : __ldg(a); };
     Spline1D<ORDER, R> sp[3];
     int idx[3][K];
     bool ok = true;
@@ -175,7 +172,7 @@ __device__ __forceinline__ void apic_g2p_particle(const MeshP& mp, int64_t p, co
                     R ue[NC];
 #pragma unroll
                     for (int d = 0; d < NC; ++d)
-                        ue[d] = (R)load(u.ptr<GT>(idx[0][i], idx[1][j], idx[2][k], d));
+                        ue[d] = (R)__ldg(u.ptr<GT>(idx[0][i], idx[1][j], idx[2][k], d));
 #pragma unroll
                     for (int d = 0; d < NC; ++d) {
                         up[d] = up[d] + w * ue[d];
@@ -184,7 +181,7 @@ __device__ __forceinline__ void apic_g2p_particle(const MeshP& mp, int64_t p, co
                         for (int a = 0; a < 3; ++a) B[d][a] += wu * dist[a];
                     }
                 } else {
-                    const R ue = (R)load(u.ptr<GT>(idx[0][i], idx[1][j], idx[2][k], 0));
+                    const R ue = (R)__ldg(u.ptr<GT>(idx[0][i], idx[1][j], idx[2][k], 0));
                     const R wu = w * ue;
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {

@@ -104,26 +104,6 @@ inline bool wide_rows(const PField& c)
            reinterpret_cast<uintptr_t>(c.data) % 16 == 0;
 }
 
-// First stencil node of a particle along d, counted from the owned box in a
-// periodic dimension; false if the stencil leaves a non-periodic mesh.
-template <int K>
-__device__ __forceinline__ bool stencil_start(const MeshP& mp, int d, int s0, int& r)
-{
-    if (!mp.periodic[d]) {
-        r = s0;
-        return s0 >= 0 && s0 <= mp.ext[d] - K;
-    }
-    const int n = mp.own_n[d];
-    r = s0 - mp.own_lo[d];
-    if (r < 0) r += n;         // one period covers every particle inside or
-    else if (r >= n) r -= n;   // next to the owned box
-    if ((unsigned)r >= (unsigned)n) {
-        r %= n;
-        if (r < 0) r += n;
-    }
-    return true;
-}
-
 // Adds the particles [a, b) to the grid; called by a whole warp.  sm:
 // WarpP2G::DOUBLES doubles of the warp.  wide: wide_rows(c).
 template <int ORDER, int NC, bool STAG>
@@ -357,21 +337,10 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
         };
         changes();
         if (__popc(chg & ~step) > 8) {
-            // bitonic sort of (stencil, lane); the lane's particle becomes the
-            // one of its rank.  Stencils more than 2^27 apart may share a key:
-            // then they are only not merged.
-            unsigned key = lane < cnt
-                               ? ((((unsigned)s[0] * (unsigned)mp.ext[1] + (unsigned)s[1]) *
-                                       (unsigned)mp.ext[2] + (unsigned)s[2]) << 5) | lane
-                               : 0xFFFFFFE0u | lane;
-#pragma unroll
-            for (int size = 2; size <= 32; size *= 2)
-#pragma unroll
-                for (int st = size / 2; st > 0; st /= 2) {
-                    const unsigned other = __shfl_xor_sync(kAll, key, st);
-                    const bool up = (lane & size) == 0 || size == 32;
-                    key = ((lane & st) == 0) == up ? min(key, other) : max(key, other);
-                }
+            // the lane's particle becomes the one of its rank
+            const unsigned key = warp_sort_by_stencil(
+                lane < cnt, ((unsigned)s[0] * (unsigned)mp.ext[1] + (unsigned)s[1]) *
+                                    (unsigned)mp.ext[2] + (unsigned)s[2]);
             const int src = key & 31;
             p = p0 + src;
             ok = __shfl_sync(kAll, ok, src);
