@@ -143,11 +143,12 @@ typedef struct picasso_bins {
     int32_t order;               /* spline order the bins were built for */
     int32_t location;            /* picasso_location the bins were built for */
     int32_t chunk;               /* particles per work item */
-    int32_t p2g_lanes;           /* lanes per particle of the tiled P2G: 1, 2 or
-                                    4 for orders 1-2 (the 4 grid fields are
-                                    split between them), 4 for order 3 (one
-                                    stencil i-plane each); 0 = the library's
-                                    choice; set to 0 by the sort */
+    int32_t p2g_lanes;           /* 0, or 1, 2 or 4 for orders 1-2 (staggered
+                                    locations: 1 or 2), 4 for order 3; other
+                                    values are refused.  The tiled P2G's lanes
+                                    per particle follow from the order (one per
+                                    k-row of the stencil) whatever its value;
+                                    set to 0 by the sort */
     const int64_t* tile_offset;  /* device, num_tiles_total + 1 particle offsets */
     const uint32_t* tile_items;  /* device, num_tiles_total + 1: first work item
                                     of each tile (exclusive prefix of
@@ -500,8 +501,7 @@ typedef struct picasso_tune_result {
 /* Autotuner of the precision-form tiled step (FP32 m_p / c_p, 64-bit
  * fixed-point m_i / mu_i, FP32 u_i; collocated, 3 components) on the
  * caller's own particles: for tiles (4,4,4) (4,4,8) (4,8,8) (8,8,8), work items
- * of 1024 and 4096 particles and 1 or 2 P2G lanes per particle (4 for cubic)
- * it sorts and permutes copies of the particles and times `trials` steps of
+ * of 1024 and 4096 particles it sorts and permutes copies of the particles and times `trials` steps of
  * grid fill -> P2G -> grid velocity -> G2P with CUDA events on the stream,
  * and writes the fastest candidate to *best.  The particle members are not
  * modified; m_i, mu_i and u_i serve as the step's grids and hold the last

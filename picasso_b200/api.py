@@ -548,8 +548,8 @@ def cell_sort(sd, tile=(4, 8, 8), chunk=4096, stream=None, workspace=None, p2g_l
     """Stable sort of the spline's particles by (tile, bin).  Returns
     (key, perm, bins): keys and permutation as int32 tensors holding uint32
     values, and the Bins to pass to the transfers once the particle members
-    have been permuted (see permute / permute_members).  `p2g_lanes` (1, 2, 4;
-    0 = library choice) is the tiled P2G's lanes per particle.  `keys`: the
+    have been permuted (see permute / permute_members).  `p2g_lanes` (0, 1, 2
+    or 4) is accepted where the order allows it and changes nothing.  `keys`: the
     particles' keys for this tile shape as APIC.g2p_advect(key_tile=tile)
     returned them; the sort then starts from them instead of the positions.
     `out`: a SortBuffers for this spline and tile shape whose tensors receive

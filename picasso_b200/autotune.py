@@ -1,11 +1,12 @@
 """Autotuner for the sorted (tiled) transfers.
 
 For an instance shape -- mesh edge, particles per cell, spline order and
-form -- it picks the three launch knobs of the tiled path:
+form -- it picks the launch knobs of the tiled path:
   * ``tile``: bins per tile (the sort's tile shape, which sets the node tile
     a work item stages in shared memory),
   * ``chunk``: particles per work item,
-  * ``lanes``: lanes per particle of the tiled P2G (precision form only).
+  * ``lanes``: the ``p2g_lanes`` value of the order (the tiled P2G's lanes per
+    particle follow from it; precision form only).
 Each candidate is timed on a synthetic instance of the shape's class (uniform
 positions, v ~ N(0, 1), m ~ U[0.5, 1.5], C ~ N(0, 0.1)) on the current GPU:
 sort + permute once per (tile, chunk), then the median of a few
@@ -35,7 +36,7 @@ PPC_BUCKETS = [(0, 4), (5, 10), (11, 1 << 20)]
 def lanes_for(order, f32):
     if not f32:
         return [0]
-    return [4] if order == 3 else [1, 2]
+    return [4] if order == 3 else [1]
 
 
 def _bucket(v, buckets):

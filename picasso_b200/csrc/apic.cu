@@ -183,7 +183,7 @@ static picasso_status launch_g2p_tiled_f64(const MeshP& mp, const TileP& tp, int
     if ((int64_t)(smem + rows) > device_smem_optin()) return PICASSO_OK;
     *handled = true;
     const bool packed = packed_rows_f64(x, c, 12, adv != nullptr);
-    const int64_t items = tp.ntiles + (n + tp.chunk - 1) / tp.chunk;
+    const int64_t items = item_bound(tp, n);
     auto launch = [&](auto kern) -> picasso_status {
         PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, u, c, err, adv ? *adv : Advect{}, packed);
@@ -338,7 +338,7 @@ static picasso_status apic_g2p_entry(const picasso_spline* sd, int64_t num_parti
                             ap, s, &handled, stag);
         if (st || handled) return st;
         TileP tp;
-        if (!f32 && stag < 0 && ncomp == 3 && make_tilep(mp, sd->order, *exec->bins, &tp)) {
+        if (!f32 && stag < 0 && ncomp == 3 && make_tilep(mp, sd->order, *exec->bins, num_particles, &tp)) {
             PB_ORDER_SWITCH(sd->order, st = launch_g2p_tiled_f64<O_>(mp, tp, num_particles, x, u, c,
                                                                      err, ap, s, &handled));
             if (st || handled) return st;

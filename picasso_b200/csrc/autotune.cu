@@ -1,11 +1,11 @@
 // Native autotuner of the sorted (tiled) transfer step: for one instance's
 // own particles it measures fill -> P2G -> velocity -> G2P for every
-// candidate tile shape, work-item size and P2G lanes-per-particle, and
+// candidate tile shape and work-item size, and
 // returns the fastest.  A host-side composition of the public entry points
 // (cell sort, permute, grid fill, APIC P2G, grid velocity, APIC G2P) on
 // sorted copies of the particles, timed with CUDA events on the caller's
 // stream.  Candidates: tiles (4,4,4) (4,4,8) (4,8,8) (8,8,8), work items of
-// 1024 and 4096 particles, 1 or 2 lanes per particle (orders 1-2), 4 (order 3).
+// 1024 and 4096 particles (p2g_lanes is the order's: 1, or 4 for order 3).
 #include <vector>
 
 #include "common.cuh"
@@ -98,9 +98,7 @@ extern "C" picasso_status picasso_autotune(const picasso_spline* sd, int64_t num
 
     const int32_t tiles[4][3] = {{4, 4, 4}, {4, 4, 8}, {4, 8, 8}, {8, 8, 8}};
     const int32_t chunks[2] = {1024, 4096};
-    const int32_t lanes_lo[2] = {1, 2}, lanes_cubic[1] = {4};
-    const int32_t* lanes = sd->order == 3 ? lanes_cubic : lanes_lo;
-    const int nlanes = sd->order == 3 ? 1 : 2;
+    const int32_t lanes = sd->order == 3 ? 4 : 1;
     float best_ms = -1.f;
 
     for (const auto& tile : tiles) {
@@ -125,39 +123,37 @@ extern "C" picasso_status picasso_autotune(const picasso_spline* sd, int64_t num
                 return st;
             if ((st = picasso_permute(n, 3, perm, x_p, xf, &ex))) return st;
             if ((st = picasso_permute(n, 1, perm, m_p, mf, &ex))) return st;
-            for (int li = 0; li < nlanes; ++li) {
-                bins.p2g_lanes = lanes[li];
-                picasso_exec bex = ex;
-                bex.bins = &bins;
-                // c_p is re-gathered before each candidate: G2P overwrites it
-                auto step = [&]() -> picasso_status {
-                    picasso_status r;
-                    if ((r = picasso_grid_fill(&sd->mesh, 1, m_i, 0.0, &ex))) return r;
-                    if ((r = picasso_grid_fill(&sd->mesh, 3, mu_i, 0.0, &ex))) return r;
-                    if ((r = picasso_apic_p2g(sd, n, 3, xf, mf, cf, m_i, mu_i, &bex))) return r;
-                    picasso_grid_field none{};
-                    if ((r = picasso_grid_velocity(&sd->mesh, 3, m_i, mu_i, mass_threshold, u_i,
-                                                   none, &ex)))
-                        return r;
-                    return picasso_apic_g2p(sd, n, 3, xf, u_i, cf, &bex);
-                };
-                if ((st = picasso_permute(n, 12, perm, c_p, cf, &ex))) return st;
-                if ((st = step())) return st;  // warm-up
-                PB_CUDA_TRY(cudaEventRecord(e0, s));
-                for (int t = 0; t < trials; ++t)
-                    if ((st = step())) return st;
-                PB_CUDA_TRY(cudaEventRecord(e1, s));
-                PB_CUDA_TRY(cudaEventSynchronize(e1));
-                float ms_total = 0.f;
-                PB_CUDA_TRY(cudaEventElapsedTime(&ms_total, e0, e1));
-                const float per = ms_total / trials;
-                if (best_ms < 0.f || per < best_ms) {
-                    best_ms = per;
-                    for (int d = 0; d < 3; ++d) best->tile[d] = tile[d];
-                    best->chunk = chunk;
-                    best->p2g_lanes = lanes[li];
-                    best->step_ms = per;
-                }
+            bins.p2g_lanes = lanes;
+            picasso_exec bex = ex;
+            bex.bins = &bins;
+            // c_p is re-gathered before each candidate: G2P overwrites it
+            auto step = [&]() -> picasso_status {
+                picasso_status r;
+                if ((r = picasso_grid_fill(&sd->mesh, 1, m_i, 0.0, &ex))) return r;
+                if ((r = picasso_grid_fill(&sd->mesh, 3, mu_i, 0.0, &ex))) return r;
+                if ((r = picasso_apic_p2g(sd, n, 3, xf, mf, cf, m_i, mu_i, &bex))) return r;
+                picasso_grid_field none{};
+                if ((r = picasso_grid_velocity(&sd->mesh, 3, m_i, mu_i, mass_threshold, u_i,
+                                               none, &ex)))
+                    return r;
+                return picasso_apic_g2p(sd, n, 3, xf, u_i, cf, &bex);
+            };
+            if ((st = picasso_permute(n, 12, perm, c_p, cf, &ex))) return st;
+            if ((st = step())) return st;  // warm-up
+            PB_CUDA_TRY(cudaEventRecord(e0, s));
+            for (int t = 0; t < trials; ++t)
+                if ((st = step())) return st;
+            PB_CUDA_TRY(cudaEventRecord(e1, s));
+            PB_CUDA_TRY(cudaEventSynchronize(e1));
+            float ms_total = 0.f;
+            PB_CUDA_TRY(cudaEventElapsedTime(&ms_total, e0, e1));
+            const float per = ms_total / trials;
+            if (best_ms < 0.f || per < best_ms) {
+                best_ms = per;
+                for (int d = 0; d < 3; ++d) best->tile[d] = tile[d];
+                best->chunk = chunk;
+                best->p2g_lanes = lanes;
+                best->step_ms = per;
             }
         }
         PB_CUDA_TRY(cudaStreamSynchronize(s));  // before the tile's buffers are freed

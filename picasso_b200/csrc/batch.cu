@@ -38,18 +38,9 @@
 namespace pb {
 
 constexpr int kPhases = 4;
-// P2G variants: the phased step runs one P2G kernel per variant, each with the
-// registers of that variant alone.  Precision form: (order, lanes per
-// particle); FP64: order.
-constexpr int kVariants = 7;
-constexpr int kVarOrder[kVariants] = {1, 1, 1, 2, 2, 2, 3};
-constexpr int kVarLanes[kVariants] = {1, 2, 4, 1, 2, 4, 4};
-
-__host__ __device__ constexpr int p2g_variant(bool f32, int order, int lpp)
-{
-    return f32 ? (order == 3 ? 6 : (order - 1) * 3 + (lpp == 1 ? 0 : (lpp == 2 ? 1 : 2)))
-               : order - 1;
-}
+// P2G variants: the phased step runs one P2G kernel per spline order, each with
+// the registers of that order alone.
+constexpr int kVariants = 3;
 constexpr int kNodeItem = 4096;           // nodes per fill / velocity item
 constexpr unsigned kWaitPolls = 1u << 22;  // default bound: ~1-2 s of polling
 
@@ -61,7 +52,7 @@ struct BInst {
     Box full, owned;
     double thr, inv_m, inv_mu;
     int64_t n;
-    int order, lpp;
+    int order;
     uint32_t nitems[kPhases];
 };
 
@@ -145,11 +136,11 @@ __device__ void velocity_item(const BInst& I, uint32_t local, int tid)
 
 // Item bodies called out of line: each variant gets its own register
 // allocation instead of one allocation for the union of all inlined variants.
-template <int ORDER, int LPP>
+template <int ORDER>
 __device__ __noinline__ void p2g_item_call(const P2GArgs& A, int64_t t, int64_t a, int64_t b,
-                                           float* smem, int* stage_base)
+                                           float* smem)
 {
-    p2g_item<ORDER, LPP>(A, t, a, b, smem, stage_base);
+    p2g_item<ORDER>(A, t, a, b, smem);
 }
 
 template <int ORDER, int NT>
@@ -223,33 +214,25 @@ __device__ __forceinline__ const T& stage_args(const T& src, T* dst, int tid)
 // VAR >= 0: every item of this kernel is of P2G variant VAR (inlined body);
 // VAR < 0: any variant (out-of-line bodies).
 template <bool F32, int NT, int VAR>
-__device__ void p2g_batch_item(const BInst& I, uint32_t local, float* smem, int* stage_base,
-                               P2GArgs* args, int tid)
+__device__ void p2g_batch_item(const BInst& I, uint32_t local, float* smem, P2GArgs* args, int tid)
 {
     int64_t t, a, b;
     if (!item_range(I.p2g.tp, local, t, a, b)) return;
     if constexpr (VAR >= 0) {
-        constexpr int O = F32 ? kVarOrder[VAR] : VAR + 1;
+        constexpr int O = VAR + 1;
         if constexpr (F32) {
             static_assert(NT == 32, "tiled P2G items are single-warp");
             const P2GArgs& A = stage_args<P2GArgs, NT>(I.p2g, args, tid);
-            p2g_item<O, kVarLanes[VAR]>(A, t, a, b, smem, stage_base);
+            p2g_item<O>(A, t, a, b, smem);
         } else {
             warp_p2g_item<O, NT>(I, a, b, smem, tid);
         }
     } else if constexpr (F32) {
         static_assert(!F32 || NT == 32, "tiled P2G items are single-warp");
-        const int key = I.order * 8 + I.lpp;
         const P2GArgs& A = stage_args<P2GArgs, NT>(I.p2g, args, tid);
-        switch (key) {
-            case 1 * 8 + 1: p2g_item_call<1, 1>(A, t, a, b, smem, stage_base); break;
-            case 1 * 8 + 2: p2g_item_call<1, 2>(A, t, a, b, smem, stage_base); break;
-            case 1 * 8 + 4: p2g_item_call<1, 4>(A, t, a, b, smem, stage_base); break;
-            case 2 * 8 + 1: p2g_item_call<2, 1>(A, t, a, b, smem, stage_base); break;
-            case 2 * 8 + 2: p2g_item_call<2, 2>(A, t, a, b, smem, stage_base); break;
-            case 2 * 8 + 4: p2g_item_call<2, 4>(A, t, a, b, smem, stage_base); break;
-            default: p2g_item_call<3, 4>(A, t, a, b, smem, stage_base); break;
-        }
+        if (I.order == 1) p2g_item_call<1>(A, t, a, b, smem);
+        else if (I.order == 2) p2g_item_call<2>(A, t, a, b, smem);
+        else p2g_item_call<3>(A, t, a, b, smem);
     } else {
         if (I.order == 1) warp_p2g_call<1, NT>(I, a, b, smem, tid);
         else if (I.order == 2) warp_p2g_call<2, NT>(I, a, b, smem, tid);
@@ -291,9 +274,7 @@ struct BatchShape {
     // a single-variant precision-form P2G kernel gets the occupancy of the
     // single-call kernel of that variant
     static constexpr int min_blocks =
-        threads == 32 ? ((VAR >= 0 && F32) ? P2GOccupancy<kVarOrder[VAR >= 0 ? VAR : 0],
-                                                          kVarLanes[VAR >= 0 ? VAR : 0]>::value
-                                           : 8)
+        threads == 32 ? ((VAR >= 0 && F32) ? kP2GOccupancy : 8)
                       : (!F32 && threads == 128 ? 3 : 4);
 };
 
@@ -304,7 +285,6 @@ batch_kernel(BatchDev B, uint32_t qlo, uint32_t qhi, int slot)
 {
     constexpr int NT = BatchShape<F32, PMASK, VAR>::threads;
     extern __shared__ __align__(16) float smem[];
-    __shared__ int stage_base[kStageBases];
     __shared__ uint32_t s_item;
     __shared__ __align__(16) P2GArgs s_p2g;
     __shared__ __align__(16) G2PArgs s_g2p;
@@ -340,7 +320,7 @@ batch_kernel(BatchDev B, uint32_t qlo, uint32_t qhi, int slot)
                 if (ph == 0) fill_item<F32, NT>(I, local, tid);
             if constexpr ((PMASK & 0x2) != 0)
                 if (ph == 1)
-                    p2g_batch_item<F32, NT, VAR>(I, local, smem, stage_base, &s_p2g, tid);
+                    p2g_batch_item<F32, NT, VAR>(I, local, smem, &s_p2g, tid);
             if constexpr ((PMASK & 0x4) != 0)
                 if (ph == 2) velocity_item<F32, NT>(I, local, tid);
             if constexpr ((PMASK & 0x8) != 0)
@@ -398,14 +378,11 @@ picasso_status configure_kernel(int smem, int items, int* blocks)
     return PICASSO_OK;
 }
 
-// FP64 has variants 0..2 (orders 1..3) only.
 template <bool F32, int VAR>
 picasso_status configure_variant(picasso_batch* b)
 {
-    if constexpr (F32 || VAR < 3) {
-        const int n = (int)(b->var_hi[VAR] - b->var_lo[VAR]);
-        if (n) return configure_kernel<F32, 0x2, VAR>(b->var_smem[VAR], n, &b->var_blocks[VAR]);
-    }
+    const int n = (int)(b->var_hi[VAR] - b->var_lo[VAR]);
+    if (n) return configure_kernel<F32, 0x2, VAR>(b->var_smem[VAR], n, &b->var_blocks[VAR]);
     return PICASSO_OK;
 }
 
@@ -425,23 +402,17 @@ picasso_status configure(picasso_batch* b)
     if ((st = configure_kernel<F32, 0x8>(b->smem[3], items[3], &b->blocks[3]))) return st;
     if ((st = configure_variant<F32, 0>(b))) return st;
     if ((st = configure_variant<F32, 1>(b))) return st;
-    if ((st = configure_variant<F32, 2>(b))) return st;
-    if ((st = configure_variant<F32, 3>(b))) return st;
-    if ((st = configure_variant<F32, 4>(b))) return st;
-    if ((st = configure_variant<F32, 5>(b))) return st;
-    return configure_variant<F32, 6>(b);
+    return configure_variant<F32, 2>(b);
 }
 
 template <bool F32, int VAR>
 void launch_p2g_variant(const picasso_batch* b, cudaStream_t s)
 {
-    if constexpr (F32 || VAR < 3) {
-        const uint32_t lo = b->var_lo[VAR], hi = b->var_hi[VAR];
-        if (lo == hi) return;
-        batch_kernel<F32, 0x2, VAR>
-            <<<b->var_blocks[VAR], BatchShape<F32, 0x2, VAR>::threads, b->var_smem[VAR], s>>>(
-                b->dev, lo, hi, kPhases + VAR);
-    }
+    const uint32_t lo = b->var_lo[VAR], hi = b->var_hi[VAR];
+    if (lo == hi) return;
+    batch_kernel<F32, 0x2, VAR>
+        <<<b->var_blocks[VAR], BatchShape<F32, 0x2, VAR>::threads, b->var_smem[VAR], s>>>(
+            b->dev, lo, hi, kPhases + VAR);
 }
 
 template <bool F32>
@@ -453,10 +424,6 @@ void launch_phase(const picasso_batch* b, int p, cudaStream_t s)
         launch_p2g_variant<F32, 0>(b, s);
         launch_p2g_variant<F32, 1>(b, s);
         launch_p2g_variant<F32, 2>(b, s);
-        launch_p2g_variant<F32, 3>(b, s);
-        launch_p2g_variant<F32, 4>(b, s);
-        launch_p2g_variant<F32, 5>(b, s);
-        launch_p2g_variant<F32, 6>(b, s);
         return;
     }
 #define PB_PHASE(P, M)                                                                  \
@@ -515,10 +482,9 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     if (bins.order != in.spline.order || bins.location != in.spline.location)
         return PICASSO_ERR_INVALID_ARGUMENT;
     const int order = in.spline.order;
-    const int lpp = bins.p2g_lanes ? bins.p2g_lanes : default_lpp(order);
-    if (f32 && !valid_lpp(order, lpp)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (f32 && !valid_lanes(order, bins.p2g_lanes)) return PICASSO_ERR_INVALID_ARGUMENT;
     TileP tp;
-    if (!make_tilep(mp, order, bins, &tp, f32 ? lpp : 0)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, order, bins, in.num_particles, &tp, f32)) return PICASSO_ERR_INVALID_ARGUMENT;
 
     std::memset(static_cast<void*>(I), 0, sizeof(BInst));
     I->p2g.mp = mp;
@@ -557,9 +523,7 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     I->inv_mu = f32 ? ldexp(1.0, -in.mu_i.fixed_bits) : 1.0;
     I->n = in.num_particles;
     I->order = order;
-    I->lpp = lpp;
-    const int64_t work = in.num_particles ? tp.ntiles + (in.num_particles + tp.chunk - 1) / tp.chunk
-                                          : 0;
+    const int64_t work = in.num_particles ? item_bound(tp, in.num_particles) : 0;
     const int64_t fill = (I->full.count() + kNodeItem - 1) / kNodeItem;
     const int64_t vel = (I->owned.count() + kNodeItem - 1) / kNodeItem;
     if (work > (1LL << 30) || fill > (1LL << 30)) return PICASSO_ERR_OUT_OF_RANGE;
@@ -568,7 +532,7 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     I->nitems[2] = (uint32_t)vel;
     I->nitems[3] = (uint32_t)work;
     if (f32) {
-        *smem_p2g = std::max(*smem_p2g, (int)p2g_warp_bytes(order, lpp, tp.P));
+        *smem_p2g = std::max(*smem_p2g, (int)p2g_warp_bytes(order, tp.P));
         *smem_g2p = std::max(*smem_g2p, (int)(sizeof(float4) * (size_t)tp.nodes));
     } else {
         *smem_p2g = std::max(*smem_p2g, warp_p2g_bytes(order));  // one warp's
@@ -614,7 +578,7 @@ extern "C" picasso_status picasso_batch_create(const picasso_batch_instance* ins
     // queue: phase-major, instances by decreasing particle count; in the P2G
     // phase grouped by variant first (one phased launch per variant)
     std::vector<int> var(count);
-    for (int i = 0; i < count; ++i) var[i] = p2g_variant(f32, hinst[i].order, hinst[i].lpp);
+    for (int i = 0; i < count; ++i) var[i] = hinst[i].order - 1;
     std::vector<int32_t> by_size(count);
     std::iota(by_size.begin(), by_size.end(), 0);
     std::stable_sort(by_size.begin(), by_size.end(), [&](int a, int c) {
@@ -638,8 +602,8 @@ extern "C" picasso_status picasso_batch_create(const picasso_batch_instance* ins
                 if (b->var_lo[v] == b->var_hi[v]) b->var_lo[v] = (uint32_t)q;
                 b->var_hi[v] = (uint32_t)(q + hinst[i].nitems[p]);
                 b->var_smem[v] =
-                    f32 ? std::max(b->var_smem[v], (int)p2g_warp_bytes(hinst[i].order, hinst[i].lpp,
-                                                                       hinst[i].p2g.tp.P))
+                    f32 ? std::max(b->var_smem[v],
+                                   (int)p2g_warp_bytes(hinst[i].order, hinst[i].p2g.tp.P))
                         : kF64Warps * warp_p2g_bytes(hinst[i].order);
             }
             q += hinst[i].nitems[p];

@@ -586,7 +586,7 @@ static picasso_status launch_pp_p2g_tiled(const MeshP& mp, const TileP& tp, int6
     const size_t smem = 3 * sizeof(unsigned int) * (1 + NC) * (size_t)tp.nodes;
     auto kern = polypic_p2g_tiled_kernel<ORDER, NC>;
     PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t items = tp.ntiles + (n + tp.chunk - 1) / tp.chunk;
+    const int64_t items = item_bound(tp, n);
     kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, m, u, c, gmu, gm, (float)dt,
                                              ldexpf(1.f, gmu.fixed_bits), ldexpf(1.f, gm.fixed_bits),
                                              err);
@@ -602,7 +602,7 @@ static picasso_status launch_pp_g2p_tiled(const MeshP& mp, const TileP& tp, int6
     const bool ws = packed_record<ORDER, NC, float>(c);
     const size_t smem = ((sizeof(float4) * tp.nodes + 15) & ~size_t(15)) +
                         (ws ? 4 * WarpRecords<float, NV>::kBytesPerWarp : 0);
-    const int64_t items = tp.ntiles + (n + tp.chunk - 1) / tp.chunk;
+    const int64_t items = item_bound(tp, n);
     if (ws) {
         auto kern = polypic_g2p_tiled_kernel<ORDER, NC, true>;
         PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -709,7 +709,7 @@ static picasso_status polypic_common(const picasso_spline* sd, int64_t n, int32_
 // locations; the bins must match the spline.  *tiled stays false (plain
 // kernels) when not eligible or when the node tile of `node_bytes` per node
 // does not fit in shared memory.
-static picasso_status polypic_tiles(const picasso_spline* sd, const picasso_exec* exec,
+static picasso_status polypic_tiles(const picasso_spline* sd, const picasso_exec* exec, int64_t n,
                                     bool eligible, const MeshP& mp, int node_bytes, bool* tiled,
                                     TileP* tp)
 {
@@ -718,7 +718,7 @@ static picasso_status polypic_tiles(const picasso_spline* sd, const picasso_exec
     if (exec->bins->order != sd->order || exec->bins->location != sd->location)
         return PICASSO_ERR_INVALID_ARGUMENT;
     if (!eligible) return PICASSO_OK;
-    if (!make_tilep(mp, sd->order, *exec->bins, tp)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, sd->order, *exec->bins, n, tp)) return PICASSO_ERR_INVALID_ARGUMENT;
     // records of four warps on top of the node tile in the G2P (at most)
     const int64_t extra = 4 * 32 * 82 * 4;
     if ((int64_t)node_bytes * tp->nodes + extra > device_smem_optin()) return PICASSO_OK;
@@ -760,7 +760,7 @@ extern "C" picasso_status picasso_polypic_p2g(const picasso_spline* sd, int64_t 
     // (the tile's 32-bit slice sums are exact for work items of at most
     // 65536 particles)
     const bool p2g_ok = form == 1 && stag < 0 && exec && exec->bins && exec->bins->chunk <= 65536;
-    if ((st = polypic_tiles(sd, exec, p2g_ok, mp, 12 * (1 + ncomp), &tiled, &tp))) return st;
+    if ((st = polypic_tiles(sd, exec, num_particles, p2g_ok, mp, 12 * (1 + ncomp), &tiled, &tp))) return st;
     if (tiled) {
         if (sd->order == 1) {
             PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g_tiled<1, NC_>(mp, tp, num_particles, x, m,
@@ -805,7 +805,7 @@ extern "C" picasso_status picasso_polypic_g2p(const picasso_spline* sd, int64_t 
     GField u = make_gfield(u_i);
     bool tiled = false;
     TileP tp;
-    if ((st = polypic_tiles(sd, exec, f32 && stag < 0, mp, 16, &tiled, &tp))) return st;
+    if ((st = polypic_tiles(sd, exec, num_particles, f32 && stag < 0, mp, 16, &tiled, &tp))) return st;
     if (tiled) {
         if (sd->order == 1) {
             PB_PP_NC_SWITCH(ncomp, return launch_pp_g2p_tiled<1, NC_>(mp, tp, num_particles, x, u,

@@ -3,9 +3,9 @@
 // bodies are in tiled.cuh.
 //
 // P2G runs single-warp CTAs (warps finish their items independently; a
-// 4-warp CTA would wait for its slowest warp) with LPP lanes per particle.
+// 4-warp CTA would wait for its slowest warp).
 // G2P runs 128-thread CTAs sharing one node tile.
-#include <mutex>
+#include <algorithm>
 
 #include "tiled.cuh"
 
@@ -19,20 +19,21 @@ struct G2PThreads {
     static constexpr int value = ORDER == 3 ? 32 : 64;
 };
 
-template <int ORDER, int LPP, bool REC, bool FUSED, bool STAG>
-__global__ void __launch_bounds__(32, (P2GOccupancy<ORDER, LPP>::value))
+template <int ORDER, bool REC, bool FUSED, bool STAG>
+__global__ void __launch_bounds__(32, kP2GOccupancy)
 p2g_tiled_kernel(P2GArgs A, FusedUpdate F, int64_t n)
 {
     extern __shared__ __align__(16) float smem[];
-    __shared__ int stage_base[kStageBases];
     if (blockIdx.x == 0 && threadIdx.x == 0 && A.err) {
         const int64_t n_valid = __ldg(A.tp.off + A.tp.ntiles);
         if (n > n_valid) atomicAdd(A.err, (int)(n - n_valid));
     }
     int64_t t, a, b;
-    if (!item_range(A.tp, blockIdx.x, t, a, b)) return;
-    p2g_item<ORDER, LPP, REC, STAG>(A, t, a, b, smem, stage_base);
-    if constexpr (FUSED) fused_update_arrive<ORDER>(A, F, t);
+    const bool any = item_range(A.tp, blockIdx.x, t, a, b);
+    if (any) p2g_item<ORDER, REC, STAG>(A, t, a, b, smem);
+    if constexpr (FUSED) {
+        if (t >= 0) fused_update_arrive<ORDER>(A, F, t);
+    }
 }
 
 template <int ORDER, bool ADV, bool REC, bool STAG>
@@ -53,126 +54,63 @@ __global__ void __launch_bounds__(G2PThreads<ORDER>::value) g2p_tiled_kernel(G2P
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-// Padded node-tile strides for the P2G merge: value v = lane + 32 r of a
-// staged lane (field v / FS of its F fields, stencil node v % FS) lands at
-// f * P + a * SI + b * SJ + c; pick the smallest padding that maximises the
-// number of distinct banks per merge instruction.  The search takes a fraction
-// of a millisecond, so results are cached per (tile nodes, K, F) for callers
-// that alternate between tile shapes (batches of meshes).
-struct StrideKey {
-    int NT[3], K, F, split;
-    bool operator==(const StrideKey& o) const
-    {
-        return NT[0] == o.NT[0] && NT[1] == o.NT[1] && NT[2] == o.NT[2] && K == o.K &&
-               F == o.F && split == o.split;
-    }
-};
-
-// Tile strides (SJ, SI, P) that spread the tile offsets of one merge round
-// (32 staged values added by 32 lanes) over as many shared-memory banks as
-// possible; the smallest tile among equals.  `split`: the staging of the
-// i-plane split (F fields of K^2 nodes per lane, whose k-plane merges are
-// counted as well).
-static void search_strides(const StrideKey& key, int* SJ, int* SI, int* P)
+// Node-tile strides of the P2G: the nodes (i, j, k0) of a plane are added by the
+// lanes of a stream at once, 16 bytes each, 8 lanes per shared-memory cycle; the
+// smallest padding (fewer than 8 nodes per row and per plane) that puts the most
+// of 8 consecutive rows' nodes on distinct banks.
+static void choose_strides(const int NT[3], int K, int* SJ, int* SI)
 {
-    const int* NT = key.NT;
-    const int K = key.K, F = key.F;
-    const int NL = key.split ? K * K : K * K * K, FS = (NL + 3) & ~3, SV = F * FS;
-    const int R = (SV + 31) / 32;
-    const int ROWS = NL / K, PV = F * ROWS, RP = key.split ? (PV + 31) / 32 : 0;
-    int best = -1, bsj = NT[2], bsi = NT[1] * NT[2], bp = NT[0] * NT[1] * NT[2];
-    long best_size = 0;
+    int best = -1, size = 0;
     for (int sj = NT[2]; sj < NT[2] + 8; ++sj)
-        for (int si = NT[1] * sj; si < NT[1] * sj + 16; ++si)
-            for (int pp = NT[0] * si; pp < NT[0] * si + 16; ++pp) {
-                int distinct = 0;
-                for (int r = 0; r < R; ++r) {
-                    unsigned banks = 0;
-                    for (int lane = 0; lane < 32; ++lane) {
-                        const int v = lane + 32 * r, f = v / FS, nn = v % FS;
-                        if (v >= SV || nn >= NL) continue;
-                        const int a = nn / (K * K), b = (nn / K) % K, c = nn % K;
-                        const int off = f * pp + a * si + b * sj + c;
-                        // 8-byte tile words: a half warp per bank cycle
-                        const unsigned bit = kTileWords == 2
-                                                 ? (1u << ((off & 15) + 16 * (lane >> 4)))
-                                                 : (1u << (off & 31));
-                        if (!(banks & bit)) ++distinct;
-                        banks |= bit;
-                    }
-                }
-                for (int r = 0; r < RP; ++r) {
-                    unsigned banks = 0;
-                    for (int lane = 0; lane < 32; ++lane) {
-                        const int v = lane + 32 * r;
-                        if (v >= PV) continue;
-                        const int ij = v % ROWS;
-                        const int off = (v / ROWS) * pp + (ij / K) * si + (ij % K) * sj;
-                        const unsigned bit = kTileWords == 2
-                                                 ? (1u << ((off & 15) + 16 * (lane >> 4)))
-                                                 : (1u << (off & 31));
-                        if (!(banks & bit)) ++distinct;
-                        banks |= bit;
-                    }
-                }
-                const long size = 4L * pp * kTileWords;
-                if (distinct > best || (distinct == best && size < best_size)) {
-                    best = distinct;
-                    best_size = size;
-                    bsj = sj;
-                    bsi = si;
-                    bp = pp;
-                }
+        for (int si = NT[1] * sj; si < NT[1] * sj + 8; ++si) {
+            int distinct = 0;
+            for (int r0 = 0; r0 < K * K; r0 += 8) {
+                unsigned banks = 0;
+                for (int r = r0; r < r0 + 8 && r < K * K; ++r) banks |= 1u << ((r / K * si + r % K * sj) & 7);
+                for (; banks; banks &= banks - 1) ++distinct;
             }
-    *SJ = bsj;
-    *SI = bsi;
-    *P = bp;
-}
-
-static void choose_strides(const int NT[3], int K, int F, int split, int* SJ, int* SI, int* P)
-{
-    constexpr int kSlots = 64;
-    static std::mutex mu;
-    static StrideKey keys[kSlots];
-    static int vals[kSlots][3];
-    static int used = 0, next = 0;
-    const StrideKey key{{NT[0], NT[1], NT[2]}, K, F, split};
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        for (int i = 0; i < used; ++i)
-            if (keys[i] == key) {
-                *SJ = vals[i][0];
-                *SI = vals[i][1];
-                *P = vals[i][2];
-                return;
+            if (distinct > best || (distinct == best && si < size)) {
+                best = distinct;
+                size = si;
+                *SJ = sj;
+                *SI = si;
             }
-    }
-    search_strides(key, SJ, SI, P);
-    std::lock_guard<std::mutex> lock(mu);
-    const int slot = used < kSlots ? used++ : (next++ % kSlots);
-    keys[slot] = key;
-    vals[slot][0] = *SJ;
-    vals[slot][1] = *SI;
-    vals[slot][2] = *P;
+        }
 }
 
-static_assert(P2GCfg<3, 4>::ISPLIT && !P2GCfg<2, 4>::ISPLIT && !P2GCfg<1, 4>::ISPLIT &&
-                  !P2GCfg<1, 2>::ISPLIT,
-              "make_tilep's stride choice follows the accumulator split");
-
-int default_lpp(int order) { return order == 3 ? 4 : 1; }
-
-// Orders 1 and 2 take 1, 2 or 4 lanes per particle (staggered locations, with
-// two grid fields: 1 or 2); order 3 (4 x 64 accumulators) takes 4.
-bool valid_lpp(int order, int lpp, bool stag)
+// Values of picasso_bins.p2g_lanes a call accepts (the P2G's lanes per particle
+// follow from the order: one per k-row of the stencil): orders 1 and 2 take 1, 2
+// or 4 (staggered locations 1 or 2), order 3 takes 4; 0 always.
+bool valid_lanes(int order, int lanes, bool stag)
 {
-    if (order == 3) return lpp == 4;
-    return lpp == 1 || lpp == 2 || (lpp == 4 && !stag);
+    if (lanes == 0) return true;
+    if (order == 3) return lanes == 4;
+    return lanes == 1 || lanes == 2 || (lanes == 4 && !stag);
 }
 
-// Tile geometry for the bins; lpp > 0 also picks the P2G tile strides for nf
-// grid fields.
-bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, TileP* tp, int lpp, int nf)
+// Parts an item of the bins is cut into: 1 where the items give every SM 4 warps;
+// less particles than that are latency-bound (12^3 cells of 4, quadratic FP32
+// form: 12 items, one warp each: P2G 69 us, G2P 21 us; 8 parts: 20 and 9 us), so
+// their items are cut into up to 8 parts of at least 64 particles on average.  A
+// function of the sizes alone: every call on the same bins, single or batched,
+// cuts the same way and sums in the same order.
+static int item_split(int64_t ntiles, int64_t n, int chunk)
+{
+    const int64_t items = ntiles + n / chunk;
+    if (items >= 148 * 4) return 1;
+    const int64_t parts = std::min<int64_t>(148 * 4 / items, n / ntiles / 64);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(parts, 8));
+}
+
+int64_t item_bound(const TileP& tp, int64_t n)
+{
+    return (tp.ntiles + (n + tp.chunk - 1) / tp.chunk) * tp.split;
+}
+
+// Tile geometry for the bins of n particles, with the strides of the P2G node
+// tile if asked.
+bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n, TileP* tp,
+                bool p2g_strides)
 {
     const int K = order + 1;
     int64_t nt = 1;
@@ -191,20 +129,17 @@ bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, TileP* tp,
     }
     tp->tsize = (uint32_t)bins.tile[0] * (uint32_t)bins.tile[1] * (uint32_t)bins.tile[2];
     tp->nodes = tp->NT[0] * tp->NT[1] * tp->NT[2];
-    if (lpp > 0) {
-        // the accumulator split of p2g_item (P2GCfg::ISPLIT, F)
-        const int split = order == 3 && lpp == 4;
-        choose_strides(tp->NT, K, split ? nf : nf / lpp, split, &tp->SJ, &tp->SI, &tp->P);
-    } else {
-        tp->SJ = tp->NT[2];
-        tp->SI = tp->NT[1] * tp->NT[2];
-        tp->P = tp->nodes;
-    }
+    tp->SJ = tp->NT[2];
+    tp->SI = tp->NT[1] * tp->NT[2];
+    if (p2g_strides) choose_strides(tp->NT, K, &tp->SJ, &tp->SI);
+    tp->P = tp->NT[0] * tp->SI;
     tp->ntiles = nt;
     tp->off = bins.tile_offset;
     tp->items = bins.tile_items;
     tp->chunk = bins.chunk;
-    return bins.tile_offset && bins.tile_items && bins.chunk >= 32;
+    if (!bins.tile_offset || !bins.tile_items || bins.chunk < 32) return false;
+    tp->split = item_split(nt, n, bins.chunk);
+    return true;
 }
 
 // The fused update needs every tile (the last one included) to hold at least
@@ -242,53 +177,34 @@ bool packed_c(const PField& c)
            (reinterpret_cast<uintptr_t>(c.data) % 16) == 0;
 }
 
-size_t p2g_warp_bytes(int order, int lpp, int P, bool rec, bool stag)
+size_t p2g_warp_bytes(int order, int P, bool stag)
 {
-#define PB_CASE(O, L, S)                                                                \
-    if (order == O && lpp == L && stag == S)                                            \
-        return sizeof(float) * (size_t)(rec ? p2g_warp_floats<O, L, true, S>(P)         \
-                                            : p2g_warp_floats<O, L, false, S>(P));
-    PB_CASE(1, 1, false) PB_CASE(1, 2, false) PB_CASE(1, 4, false)
-    PB_CASE(2, 1, false) PB_CASE(2, 2, false) PB_CASE(2, 4, false)
-    PB_CASE(3, 4, false)
-    PB_CASE(1, 1, true) PB_CASE(1, 2, true) PB_CASE(2, 1, true) PB_CASE(2, 2, true)
-    PB_CASE(3, 4, true)
-#undef PB_CASE
-    return 0;
+    const int floats = order == 1 ? (stag ? p2g_warp_floats<1, true>(P) : p2g_warp_floats<1>(P))
+                       : order == 2 ? (stag ? p2g_warp_floats<2, true>(P) : p2g_warp_floats<2>(P))
+                                    : (stag ? p2g_warp_floats<3, true>(P) : p2g_warp_floats<3>(P));
+    return sizeof(float) * (size_t)floats;
 }
 
-static int64_t item_bound(const TileP& tp, int64_t n)
-{
-    return tp.ntiles + (n + tp.chunk - 1) / tp.chunk;
-}
-
-template <int ORDER, int LPP, bool REC, bool STAG>
+template <int ORDER, bool REC, bool STAG>
 static picasso_status launch_p2g_tiled(const P2GArgs& args, const FusedUpdate* fu, int64_t n,
                                        cudaStream_t st)
 {
     P2GArgs A = args;
-    // the bulk flush rounds rows into the ring and staging area: one k-row
-    // at least must fit
-    if (P2GCfg<ORDER, LPP, REC, STAG>::TILE_OFF / 8 < A.tp.NT[2]) A.bulk_flush = 0;
-    const size_t smem = p2g_warp_bytes(ORDER, LPP, A.tp.P, REC, STAG);
+    // the bulk flush rounds rows into the table: one k-row at least must fit
+    if (P2GCfg<ORDER, STAG>::TILE_OFF / 8 < A.tp.NT[2]) A.bulk_flush = 0;
+    const size_t smem = p2g_warp_bytes(ORDER, A.tp.P, STAG);
     const int64_t items = item_bound(A.tp, n);
+    auto launch = [&](auto kern, const FusedUpdate& F) -> picasso_status {
+        PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kern<<<(unsigned)(items ? items : 1), 32, smem, st>>>(A, F, n);
+        return check_launch();
+    };
     if constexpr (!STAG) {
-        if (fu) {
-            PB_CUDA_TRY(cudaFuncSetAttribute(p2g_tiled_kernel<ORDER, LPP, REC, true, false>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem));
-            p2g_tiled_kernel<ORDER, LPP, REC, true, false>
-                <<<(unsigned)(items ? items : 1), 32, smem, st>>>(A, *fu, n);
-            return check_launch();
-        }
+        if (fu) return launch(p2g_tiled_kernel<ORDER, REC, true, false>, *fu);
     } else if (fu) {
         return PICASSO_ERR_UNSUPPORTED;  // the fused update is collocated
     }
-    PB_CUDA_TRY(cudaFuncSetAttribute(p2g_tiled_kernel<ORDER, LPP, REC, false, STAG>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    p2g_tiled_kernel<ORDER, LPP, REC, false, STAG>
-        <<<(unsigned)(items ? items : 1), 32, smem, st>>>(A, FusedUpdate{}, n);
-    return check_launch();
+    return launch(p2g_tiled_kernel<ORDER, REC, false, STAG>, FusedUpdate{});
 }
 
 template <int ORDER, bool ADV, bool REC, bool STAG>
@@ -333,13 +249,12 @@ picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, 
     if (form != Form::F32Fixed || ncomp != 3 || !packed_x(x) || !packed_m(m) || !packed_c(c))
         return PICASSO_OK;
     const bool sg = stag >= 0;
-    const int lpp = bins.p2g_lanes ? bins.p2g_lanes : default_lpp(order);
-    if (!valid_lpp(order, lpp, sg)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!valid_lanes(order, bins.p2g_lanes, sg)) return PICASSO_ERR_INVALID_ARGUMENT;
     P2GArgs A;
-    if (!make_tilep(mp, order, bins, &A.tp, lpp, sg ? 2 : 4)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, order, bins, n, &A.tp, true)) return PICASSO_ERR_INVALID_ARGUMENT;
     A.rec = bins_records(bins);
     const bool rec = A.rec != nullptr;
-    const size_t smem = p2g_warp_bytes(order, lpp, A.tp.P, rec, sg);
+    const size_t smem = p2g_warp_bytes(order, A.tp.P, sg);
     if ((int64_t)smem > device_smem_optin()) return PICASSO_OK;  // tile too large: plain path
     *handled = true;
     A.mp = mp;
@@ -356,15 +271,13 @@ picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, 
     // the fused update counts its arrivals after element-wise reductions; a
     // neighbour's rows take element-wise reductions too
     A.bulk_flush = !sg && !fu && !A.hp.on && packed_accumulator(gm, gmu);
-#define PB_CASE(O, L, S)                                                                \
-    if (order == O && lpp == L && sg == S)                                              \
-        return rec ? launch_p2g_tiled<O, L, true, S>(A, fu, n, st)                      \
-                   : launch_p2g_tiled<O, L, false, S>(A, fu, n, st);
-    PB_CASE(1, 1, false) PB_CASE(1, 2, false) PB_CASE(1, 4, false)
-    PB_CASE(2, 1, false) PB_CASE(2, 2, false) PB_CASE(2, 4, false)
-    PB_CASE(3, 4, false)
-    PB_CASE(1, 1, true) PB_CASE(1, 2, true) PB_CASE(2, 1, true) PB_CASE(2, 2, true)
-    PB_CASE(3, 4, true)
+#define PB_CASE(O)                                                                         \
+    if (order == O)                                                                        \
+        return sg ? (rec ? launch_p2g_tiled<O, true, true>(A, fu, n, st)                   \
+                         : launch_p2g_tiled<O, false, true>(A, fu, n, st))                 \
+                  : (rec ? launch_p2g_tiled<O, true, false>(A, fu, n, st)                  \
+                         : launch_p2g_tiled<O, false, false>(A, fu, n, st));
+    PB_CASE(1) PB_CASE(2) PB_CASE(3)
 #undef PB_CASE
     return PICASSO_ERR_INVALID_ARGUMENT;
 }
@@ -391,7 +304,7 @@ picasso_status apic_g2p_tiled(const MeshP& mp, int order, int ncomp, bool f32, i
     if (!f32 || ncomp != 3 || !packed_x(x) || !packed_c(c)) return PICASSO_OK;
     if (adv && stag >= 0) return PICASSO_OK;
     G2PArgs A;
-    if (!make_tilep(mp, order, bins, &A.tp)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, order, bins, n, &A.tp)) return PICASSO_ERR_INVALID_ARGUMENT;
     const size_t smem = sizeof(float4) * (size_t)A.tp.nodes;
     if ((int64_t)smem > device_smem_optin()) return PICASSO_OK;
     *handled = true;
@@ -550,7 +463,7 @@ extern "C" picasso_status picasso_apic_p2g_update(
     if (f_i.data && (st = validate_gfield(f_i, PICASSO_F64))) return st;
     if (u64_i.data && (st = validate_gfield(u64_i, PICASSO_F64))) return st;
     TileP tp;
-    if (!make_tilep(mp, sd->order, *bins, &tp)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, sd->order, *bins, num_particles, &tp)) return PICASSO_ERR_INVALID_ARGUMENT;
     int64_t need = 0;
     if ((st = picasso_apic_p2g_update_workspace(bins, &need))) return st;
     if (!fused_update_fits(tp, sd->order)) return separate();

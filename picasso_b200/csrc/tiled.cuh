@@ -6,18 +6,18 @@
 // Work items are chunks of at most `chunk` particles of one tile (the sort
 // writes the per-tile item prefix).
 //
-// P2G item (one warp): particles are processed in runs -- contiguous ranges
-// of the sorted item, so consecutive particles of a run mostly share a
-// stencil -- and each run is handled by LPP lanes (1, 2 or 4) that split the
-// four grid fields (mass, 3 momentum components) between them.  A lane keeps
-// the K^3 sums of its fields for the run's current bin in registers.
-// Particle records arrive through a cp.async ring in shared memory a few
-// particles ahead of use.  When a run's bin changes its lanes stage their
-// partial sums and the warp adds the staged partials into its FP32 node tile
-// ((T + K - 1)^3 nodes) one staged lane after the other: a fixed order without
-// atomics, so the tile sums are reproducible.  At the end of the item the
-// touched box of the tile is rounded to 64-bit fixed point and added to HBM
-// with integer reductions, whose result does not depend on their order; P2G
+// P2G item (one warp): the item's sorted particles are cut into S contiguous
+// streams (3 for quadratic, 2 for cubic, 8 for linear splines) that the warp
+// sweeps side by side.  The lanes first evaluate the next 32 / S particles of
+// every stream, one particle each (splines, the affine velocity relative to the
+// stencil's centre knot), into a shared table; then, step by step, K^2 lanes per
+// stream -- one for every k-row of the stencil -- add the stream's next particle
+// to their K nodes' sums in registers.  When a stream's stencil moves, its lanes
+// add the nodes that are finished (one k-plane for a move along k, else all) to
+// the warp's FP32 node tile ((T + K - 1)^3 nodes), stream after stream: a fixed
+// order without atomics, so the tile sums are reproducible.  At the end of the
+// item the touched box of the tile is rounded to 64-bit fixed point and added to
+// HBM with integer reductions, whose result does not depend on their order; P2G
 // is deterministic for a given particle order.
 //
 // G2P item (one warp or one CTA): the item's node velocities are staged once
@@ -39,16 +39,7 @@
 
 namespace pb {
 
-constexpr int kStageLanes = 8;   // lanes staged per full merge round
-constexpr int kStageBases = 32;  // stage_base entries (k-plane merges stage every lane at once)
 constexpr unsigned kFull = 0xFFFFFFFFu;
-
-// Element type of the P2G node tile that sums the lanes' FP32 partials.
-#ifndef PB_P2G_TILE_F64
-#define PB_P2G_TILE_F64 0
-#endif
-using TileVal = std::conditional<PB_P2G_TILE_F64 != 0, double, float>::type;
-constexpr int kTileWords = sizeof(TileVal) / sizeof(float);
 
 struct TileP {
     int T[3];    // bins per tile
@@ -57,9 +48,10 @@ struct TileP {
     int NT[3];   // nodes per tile dimension (T + K - 1)
     int nodes;   // NT0 * NT1 * NT2
     int SJ, SI;  // P2G node-tile strides along j and i (k stride 1), padded so
-    int P;       // that a merge's stencil nodes hit distinct banks; P = stride
-                 // between the 4 field planes
+                 // that a plane's nodes fall on distinct banks
+    int P;       // node slots of the P2G tile (NT0 * SI)
     int chunk;
+    int split;       // parts an item of the bins is cut into (item_split)
     int tsh[3];      // log2(T[d]) when T[d] is a power of two, else -1
     uint32_t tsize;  // bins per tile (sort keys of tile t start at t * tsize)
     int64_t ntiles;
@@ -162,10 +154,17 @@ __device__ __forceinline__ int node_global(const MeshP& mp, const TileP& tp, int
     return g;
 }
 
-// Work item w -> tile t and particle range [a, b).  False past the last item.
+// Work item w -- part w % split of item w / split of the bins -> tile t (-1 past
+// the last item) and particle range [a, b).  False if it has no particles.
 __device__ __forceinline__ bool item_range(const TileP& tp, int64_t w, int64_t& t, int64_t& a,
                                            int64_t& b)
 {
+    int part = 0;
+    if (tp.split > 1) {
+        part = (int)(w % tp.split);
+        w /= tp.split;
+    }
+    t = -1;
     if (w >= (int64_t)__ldg(tp.items + tp.ntiles)) return false;
     int64_t lo = 0, hi = tp.ntiles - 1;  // last t with items[t] <= w
     while (lo < hi) {
@@ -176,6 +175,11 @@ __device__ __forceinline__ bool item_range(const TileP& tp, int64_t w, int64_t& 
     t = lo;
     a = __ldg(tp.off + t) + (w - (int64_t)__ldg(tp.items + t)) * tp.chunk;
     b = min(a + (int64_t)tp.chunk, (int64_t)__ldg(tp.off + t + 1));
+    if (tp.split > 1) {  // parts of whole warps
+        const int64_t len = ((b - a + tp.split - 1) / tp.split + 31) & ~int64_t(31);
+        a += part * len;
+        b = min(a + len, b);
+    }
     return a < b;
 }
 
@@ -205,33 +209,13 @@ __device__ __forceinline__ bool locate(const MeshP& mp, const TileP& tp, const d
 }
 
 // ---------------------------------------------------------------------------
-// cp.async (asynchronous global -> shared copies)
+// bulk reductions (shared -> global through the tensor memory accelerator;
+// both addresses 16-byte aligned, size a multiple of 16 bytes)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned smem_addr(const void* p)
 {
     return (unsigned)__cvta_generic_to_shared(p);
 }
-template <int BYTES>
-__device__ __forceinline__ void cp_async(void* dst, const void* src)
-{
-    if constexpr (BYTES == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem_addr(dst)),
-                     "l"(src));
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(smem_addr(dst)),
-                     "l"(src), "n"(BYTES));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
-}
-
-// ---------------------------------------------------------------------------
-// bulk reductions (shared -> global through the tensor memory accelerator;
-// both addresses 16-byte aligned, size a multiple of 16 bytes)
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ void bulk_add_u64(long long* dst, const long long* src, int bytes)
 {
     asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.u64 [%0], [%1], %2;\n"
@@ -254,96 +238,47 @@ __device__ __forceinline__ void fence_proxy_async_smem()
 // ---------------------------------------------------------------------------
 // P2G
 // ---------------------------------------------------------------------------
-// Shared-memory layout of one P2G warp: particle-record ring, staging area,
-// node tile.  Field g of a node n = (a, b, c) of a bin receives
+// Field g of a node n = (a, b, c) of a bin receives
 //   w_n m (e_d + sum_q G_dq (n_q - n0))                     (order 2 / 3)
-//   m * (c0 www + cx gww + cy wgw + cz wwg)                  (order 1)
+//   m (c0 www + cx gww + cy wgw + cz wwg)                    (order 1)
 // for the momentum components d = g - 1 and w_n m for the mass (g = 0), with
 // n0 the stencil's centre knot, e_d = v_d + D sum_q B_dq dist_q(n0) and
 // G_dq = D dx B_dq: the affine term D B dist (APIC.hpp:110-139) written
 // relative to the centre knot, where dist_q(n) - dist_q(n0) = (n_q - n0) dx,
 // so the nodes next to the centre need one addition and the centre none.
-// Order 1: APIC.hpp:287-318 with D = 1.
+// Order 1: APIC.hpp:287-318 with D = 1; the gradients are +-w w / dx, so a k-row
+// (a, b) of weight w_ab = w_a w_b receives (c0 m w_ab + cx m gx_a w_b + cy m gy_b
+// w_a) w_c +- (cz m / dx) w_ab.
 //
-// REC: the particle's position arrives as a spline record (in-cell fraction
-// of the logical position along each dimension in FP32, and the sort key
-// of its bin) instead of the FP64 position.
 // STAG: a staggered location (Face<D> / Edge<D>, APIC.hpp:148-232): two
 // grid fields, the mass and the one momentum component of the entity's
 // dimension, which comes from column `stag` of c_p.
-template <int ORDER, int LPP, bool REC = false, bool STAG = false>
+template <int ORDER, bool STAG>
 struct P2GCfg {
     static constexpr int K = SplineTraits<ORDER>::K;
-    static constexpr int NF = STAG ? 2 : 4;  // grid fields
-    static constexpr int KKK = K * K * K;
-    static constexpr int N0 = 1;  // centre knot of the quadratic and cubic stencils
-    // Cubic stencils with 4 lanes per particle split the stencil by its
-    // i-planes (lane h sums all four fields of the 16 nodes (h, j, k)); the
-    // other splits are by field (lane h sums fields h F .. h F + F - 1 of all
-    // K^3 nodes).  The plane split needs one x-weight per lane and shares the
-    // affine products of a (j, k) node between the three momentum fields.
-    static constexpr bool ISPLIT = ORDER == 3 && LPP == 4;
-    static constexpr int NL = ISPLIT ? K * K : KKK;  // nodes per lane
-    static constexpr int ROWS = NL / K;              // k-rows per lane
-    static constexpr int FS = (NL + 3) & ~3;         // staged floats per field
-    static constexpr int F = ISPLIT ? NF : NF / LPP;  // fields per lane
-    static constexpr int RUNS = 32 / LPP;            // runs per warp
-    static constexpr int SV = F * FS;                // staged values per lane
-    // staging stride: a multiple of 4 floats whose quarter is odd keeps the
-    // float4 stores of 8 staged lanes on distinct banks
-    static constexpr int SS = ((SV / 4) % 2 == 0) ? SV + 4 : SV;
-    static constexpr int R = (SV + 31) / 32;  // merge rounds per staged lane
-    // k-plane merges (a lane's bin advanced by one along k): the K^2 nodes of
-    // the stencil's first k-plane, F fields, packed
-    static constexpr int PV = F * ROWS;
-    static constexpr int PV4 = (PV + 3) & ~3;
-    static constexpr int PS = ((PV4 / 4) % 2 == 0) ? PV4 + 4 : PV4;
-    static constexpr int RP = (PV + 31) / 32;
-    static_assert(PS <= SS, "a plane stages inside a full stage slot");
-    // ring per stage: position (6 floats: 3 doubles; REC: one 16-byte
-    // record) | c (12 floats) | m (1 float) per run
-    static constexpr int XS = REC ? 4 : 6;
-    static constexpr int RING_X = 0, RING_C = XS * RUNS, RING_M = (XS + 12) * RUNS;
-    static constexpr int RING =
-        (XS + 13) * RUNS + (((XS + 13) * RUNS) % 4 ? 4 - ((XS + 13) * RUNS) % 4 : 0);
-    // ring depth: records of DEPTH - 1 particles are in flight per run; the
-    // warps with fewer runs (more lanes per particle) need more to keep the
-    // same bytes in flight.  Deeper rings cost shared memory, which costs
-    // warps (measured: depth 4 fastest for one lane per particle, and for
-    // cubic stencils, whose ~600 instructions per lane and particle hide the
-    // loads: 256^3 8 ppc, tile (4, 4, 8): depth 4 14.6 ms, 6 14.7, 10 15.7).
-    static constexpr int DEPTH = LPP == 1 ? 4 : (LPP == 2 ? 8 : (ORDER == 3 ? 4 : 10));
-    static constexpr int STAGE_OFF = DEPTH * RING;
-    // staging area: kStageLanes full stencils, or the first k-plane of every
-    // lane (used one after the other)
-    static constexpr int STAGE_FLOATS = 32 * PS > kStageLanes * SS ? 32 * PS : kStageLanes * SS;
-    static constexpr int TILE_OFF = STAGE_OFF + STAGE_FLOATS;
-    // plane split with records, collocated: the lanes of a run evaluate the
-    // splines and affine form of the run's next LPP particles once (one
-    // particle each) and share them through a table after the node tile
-    // (p2g_item)
-    static constexpr bool SHARE = ISPLIT && REC && !STAG;
-    static constexpr int ENTRY = 28;  // floats of one particle's table entry
-    // entries of sub-step q start 8 q floats later (bank skew, p2g_item)
-    static constexpr int TABLE = SHARE ? 32 * ENTRY + 8 * (LPP - 1) : 0;
-    static_assert(LPP == 1 || LPP == 2 || LPP == 4, "1, 2 or 4 lanes per particle");
-    static_assert(F >= 1, "at least one field per lane");
+    static constexpr int KK = K * K;            // lanes per stream, a k-row each
+    static constexpr int NV = STAG ? 1 : 3;     // momentum components
+    static constexpr int NF = 1 + NV;           // grid fields
+    static constexpr int S = 32 / KK;           // streams
+    static constexpr int B = 32 / S;            // table slots per stream
+    // Table entry of a particle: (E, G_x, G_y, G_z) per component (linear: m times
+    // c0 and the gradient coefficients), w_z, (linear: m), the tile offset of its
+    // stencil's first node (-1: skipped).  20 floats: the 16-byte stores of 8
+    // lanes fall on distinct banks.
+    static constexpr int ENTRY = 20, WZ = 4 * NV, AT = WZ + K + (ORDER == 1 ? 1 : 0);
+    static_assert(AT < ENTRY, "a particle's entry");
+    // then w_x w_y m per k-row (linear: w_x, w_y) in rows of 33
+    static constexpr int WROWS = ORDER == 1 ? 2 * K : KK, WROW = 33;
+    static constexpr int TILE_OFF = (32 * ENTRY + WROWS * WROW + 3) & ~3;
 };
 
-// Single-warp CTAs per SM the P2G register budget is sized for: 1 lane per
-// particle holds 4 x K^3 accumulators (~255 registers), 2 and 4 lanes a half
-// and a quarter of them; cubic 4-lane items also hold a 64-node stencil.
-template <int ORDER, int LPP>
-struct P2GOccupancy {
-    static constexpr int value = LPP == 1 ? 8 : (LPP == 2 ? 12 : (ORDER == 3 ? 12 : 16));
-};
+// Single-warp CTAs per SM the P2G register budget is sized for.
+constexpr int kP2GOccupancy = 16;
 
-template <int ORDER, int LPP, bool REC = false, bool STAG = false>
+template <int ORDER, bool STAG = false>
 __host__ __device__ constexpr int p2g_warp_floats(int P)
 {
-    return P2GCfg<ORDER, LPP, REC, STAG>::TILE_OFF +
-           P2GCfg<ORDER, LPP, REC, STAG>::NF * P * kTileWords +
-           P2GCfg<ORDER, LPP, REC, STAG>::TABLE;
+    return P2GCfg<ORDER, STAG>::TILE_OFF + P2GCfg<ORDER, STAG>::NF * P;
 }
 
 // p + s g for a small integer s (s = 0: p exactly).  Called with unrolled
@@ -354,312 +289,6 @@ __device__ __forceinline__ float add_steps(int s, float p, float g)
     if (s == 1) return p + g;
     if (s == -1) return p - g;
     return fmaf((float)s, g, p);
-}
-
-template <int ORDER, int LPP, bool STAG = false>
-struct P2GAcc {
-    using C = P2GCfg<ORDER, LPP, false, STAG>;
-    float acc[C::F][C::NL];
-
-    __device__ __forceinline__ void zero()
-    {
-#pragma unroll
-        for (int f = 0; f < C::F; ++f)
-#pragma unroll
-            for (int n = 0; n < C::NL; ++n) acc[f][n] = 0.f;
-    }
-
-    // Orders 2 / 3.  E[f], G[f][q]: the centre-knot form of field f of the
-    // lane (mass: E = 1, G = 0); h: the lane's share of the particle (its
-    // i-plane when C::ISPLIT).  `mass_first`: field 0 of the lane is the
-    // mass (known at compile time for one lane per particle and for the
-    // plane split).
-    __device__ __forceinline__ void add(const Spline1D<ORDER, float> sp[3], float mass,
-                                        const float E[C::F], const float G[C::F][3], int h)
-    {
-        constexpr int K = C::K;
-        constexpr int N0 = C::N0;
-        constexpr bool MASS0 = C::ISPLIT || LPP == 1;
-        if constexpr (C::ISPLIT) {
-            float wx = 0.f;
-#pragma unroll
-            for (int i = 0; i < K; ++i)
-                if (i == h) wx = sp[0].w[i];
-            add_isplit(wx, sp[1].w, sp[2].w, mass, E, G, h);
-        } else {
-#pragma unroll
-            for (int i = 0; i < K; ++i) {
-                const float wi = sp[0].w[i] * mass;
-                float pi[C::F];
-#pragma unroll
-                for (int f = 0; f < C::F; ++f) pi[f] = add_steps(i - N0, E[f], G[f][0]);
-#pragma unroll
-                for (int j = 0; j < K; ++j) {
-                    const float wij = wi * sp[1].w[j];
-                    float pij[C::F];
-#pragma unroll
-                    for (int f = 0; f < C::F; ++f) pij[f] = add_steps(j - N0, pi[f], G[f][1]);
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const int n = (i * K + j) * K + k;
-                        const float w = wij * sp[2].w[k];
-#pragma unroll
-                        for (int f = 0; f < C::F; ++f) {
-                            if (MASS0 && f == 0) acc[f][n] += w;
-                            else
-                                acc[f][n] =
-                                    fmaf(w, add_steps(k - N0, pij[f], G[f][2]), acc[f][n]);
-                        }
-                    }
-                }
-            }
-        }
-    }
-
-    // Plane split: the lane's i-plane h, x-weight wx = w_x[h]; node (h, j, k)
-    // receives w = wx m wy_j wz_k.
-    __device__ __forceinline__ void add_isplit(float wx, const float* wy, const float* wz,
-                                               float mass, const float E[C::F],
-                                               const float G[C::F][3], int h)
-    {
-        constexpr int K = C::K;
-        constexpr int N0 = C::N0;
-        const float wxm = wx * mass;
-        const float hs = (float)(h - N0);
-        float pi[C::F];
-#pragma unroll
-        for (int f = 1; f < C::F; ++f) pi[f] = fmaf(hs, G[f][0], E[f]);
-#pragma unroll
-        for (int j = 0; j < K; ++j) {
-            const float wij = wxm * wy[j];
-            float pij[C::F];
-#pragma unroll
-            for (int f = 1; f < C::F; ++f) pij[f] = add_steps(j - N0, pi[f], G[f][1]);
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const int n = j * K + k;
-                const float w = wij * wz[k];
-                acc[0][n] += w;
-#pragma unroll
-                for (int f = 1; f < C::F; ++f)
-                    acc[f][n] = fmaf(w, add_steps(k - N0, pij[f], G[f][2]), acc[f][n]);
-            }
-        }
-    }
-
-    // Order 1 (gradient form); co[f] = (c0, cx, cy, cz) of field f.
-    __device__ __forceinline__ void add_linear(const Spline1D<ORDER, float> sp[3], float mass,
-                                               const float co[C::F][4])
-    {
-        constexpr int K = C::K;
-#pragma unroll
-        for (int i = 0; i < K; ++i)
-#pragma unroll
-            for (int j = 0; j < K; ++j)
-#pragma unroll
-                for (int k = 0; k < K; ++k) {
-                    const int n = (i * K + j) * K + k;
-                    const float www = sp[0].w[i] * sp[1].w[j] * sp[2].w[k] * mass;
-                    const float gww = sp[0].g[i] * sp[1].w[j] * sp[2].w[k] * mass;
-                    const float wgw = sp[0].w[i] * sp[1].g[j] * sp[2].w[k] * mass;
-                    const float wwg = sp[0].w[i] * sp[1].w[j] * sp[2].g[k] * mass;
-#pragma unroll
-                    for (int f = 0; f < C::F; ++f) {
-                        if (LPP == 1 && f == 0) acc[f][n] += www;  // mass
-                        else
-                            acc[f][n] += co[f][0] * www + co[f][1] * gww + co[f][2] * wgw +
-                                         co[f][3] * wwg;
-                    }
-                }
-    }
-
-    // st[f * FS + n] <- acc[f][n] with 16-byte stores.
-    __device__ __forceinline__ void stage(float* st) const
-    {
-#pragma unroll
-        for (int f = 0; f < C::F; ++f)
-#pragma unroll
-            for (int q = 0; q < C::FS / 4; ++q) {
-                float4 v;
-                v.x = (4 * q + 0 < C::NL) ? acc[f][4 * q + 0] : 0.f;
-                v.y = (4 * q + 1 < C::NL) ? acc[f][4 * q + 1] : 0.f;
-                v.z = (4 * q + 2 < C::NL) ? acc[f][4 * q + 2] : 0.f;
-                v.w = (4 * q + 3 < C::NL) ? acc[f][4 * q + 3] : 0.f;
-                *reinterpret_cast<float4*>(st + f * C::FS + 4 * q) = v;
-            }
-    }
-
-    // value v of the first k-plane: field v / ROWS, k-row v % ROWS (the row
-    // (i, j) with i * K + j = v % ROWS, or (h, j) with j = v % ROWS for the
-    // plane split), its node k = 0
-    __device__ __forceinline__ float plane_value(int v) const
-    {
-        return acc[v / C::ROWS][(v % C::ROWS) * C::K];
-    }
-
-    // st[v] <- plane_value(v) with 16-byte stores.
-    __device__ __forceinline__ void stage_plane(float* st) const
-    {
-#pragma unroll
-        for (int q = 0; q < C::PV4 / 4; ++q) {
-            float4 v;
-            v.x = (4 * q + 0 < C::PV) ? plane_value(4 * q + 0) : 0.f;
-            v.y = (4 * q + 1 < C::PV) ? plane_value(4 * q + 1) : 0.f;
-            v.z = (4 * q + 2 < C::PV) ? plane_value(4 * q + 2) : 0.f;
-            v.w = (4 * q + 3 < C::PV) ? plane_value(4 * q + 3) : 0.f;
-            *reinterpret_cast<float4*>(st + 4 * q) = v;
-        }
-    }
-
-    // Moves the sums one node down along k (the stencil moved up by one):
-    // planes 1 .. K-1 become 0 .. K-2, the last plane starts at zero.
-    __device__ __forceinline__ void shift_k()
-    {
-        constexpr int K = C::K;
-#pragma unroll
-        for (int f = 0; f < C::F; ++f)
-#pragma unroll
-            for (int ij = 0; ij < C::ROWS; ++ij) {
-#pragma unroll
-                for (int k = 0; k + 1 < K; ++k) acc[f][ij * K + k] = acc[f][ij * K + k + 1];
-                acc[f][ij * K + K - 1] = 0.f;
-            }
-    }
-};
-
-// Merge plan of one lane: staged value v = lane + 32 r of a staged lane that
-// handles fields hh F .. hh F + F - 1 (plane split: i-plane hh) lands at tile
-// offset moff[r] + hh * fstride from the stencil start.
-template <int ORDER, int LPP, bool STAG = false>
-struct MergePlan {
-    using C = P2GCfg<ORDER, LPP, false, STAG>;
-    int moff[C::R];
-    int poff[C::RP];  // the same for the values of a k-plane stage
-    int fstride;      // F * P (plane split: SI)
-    unsigned valid;   // bit r: value lane + 32 r exists
-    unsigned pvalid;
-    __device__ __forceinline__ void init(const TileP& tp, int lane)
-    {
-        constexpr int K = C::K;
-        valid = 0;
-        // the plane split offsets a staged lane's values by its i-plane
-        fstride = C::ISPLIT ? tp.SI : C::F * tp.P;
-#pragma unroll
-        for (int r = 0; r < C::R; ++r) {
-            const int v = lane + 32 * r;
-            const int fs = v / C::FS, nn = v - (v / C::FS) * C::FS;
-            moff[r] = 0;
-            if (v < C::SV && nn < C::NL) {
-                const int a = nn / (K * K), b = (nn / K) % K, c = nn % K;
-                moff[r] = fs * tp.P + a * tp.SI + b * tp.SJ + c;
-                valid |= 1u << r;
-            }
-        }
-        pvalid = 0;
-#pragma unroll
-        for (int r = 0; r < C::RP; ++r) {
-            const int v = lane + 32 * r;
-            poff[r] = 0;
-            if (v < C::PV) {
-                const int fs = v / C::ROWS, ij = v % C::ROWS;
-                poff[r] = fs * tp.P + (ij / K) * tp.SI + (ij % K) * tp.SJ;
-                pvalid |= 1u << r;
-            }
-        }
-    }
-};
-
-// The warp adds staged values into the node tile: lane l adds value l + 32 r
-// of each staged slot at tile offset base + off[r], slot after slot in a
-// fixed order (so the tile sums are reproducible): slots 0 .. n - 1 (LANES
-// false, n = `slots`) or the set bits of `slots`, lowest first (LANES true,
-// not empty).  The next slot's base and values are read before this slot's
-// tile updates, so only the tile read-add-write is on the dependency chain.
-template <int NR, int SLOT, int LPP, bool LANES>
-__device__ __forceinline__ void add_staged(unsigned slots, const float* stage,
-                                           const int* stage_base, const int (&off)[NR],
-                                           unsigned valid, int fstride, TileVal* tile, int lane)
-{
-    int q = LANES ? __ffs(slots) - 1 : 0;
-    unsigned rest = LANES ? slots & (slots - 1u) : slots - 1u;  // LANES false: slots left
-    int sb = stage_base[q];
-    float v[NR];
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-        v[r] = ((valid >> r) & 1u) ? stage[q * SLOT + lane + 32 * r] : 0.f;
-    for (;;) {
-        const int qn = rest ? (LANES ? __ffs(rest) - 1 : q + 1) : q;
-        const int sbn = stage_base[qn];
-        float vn[NR];
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
-            vn[r] = ((valid >> r) & 1u) ? stage[qn * SLOT + lane + 32 * r] : 0.f;
-        const int base = (sb & 0x0FFFFFFF) + (LPP > 1 ? (sb >> 28) * fstride : 0);
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
-            if ((valid >> r) & 1u) tile[base + off[r]] += v[r];
-        __syncwarp();
-        if (!rest) break;
-        rest = LANES ? rest & (rest - 1u) : rest - 1u;
-        q = qn;
-        sb = sbn;
-#pragma unroll
-        for (int r = 0; r < NR; ++r) v[r] = vn[r];
-    }
-}
-
-// Lanes in `mask` hand their partial sums to the warp's node tile in lane
-// order (rounds of at most kStageLanes lanes); their accumulators are zeroed.
-template <int ORDER, int LPP, bool STAG>
-__device__ __forceinline__ void merge_partials(unsigned mask, P2GAcc<ORDER, LPP, STAG>& acc,
-                                               int cur_base,
-                                               const MergePlan<ORDER, LPP, STAG>& plan,
-                                               TileVal* tile, float* stage, int* stage_base,
-                                               int lane)
-{
-    using C = P2GCfg<ORDER, LPP, false, STAG>;
-    while (mask) {
-        unsigned batch = mask;
-        if (__popc(mask) > kStageLanes) {  // the lowest kStageLanes lanes
-            batch = 0;
-            unsigned mm = mask;
-#pragma unroll
-            for (int q = 0; q < kStageLanes; ++q) {
-                batch |= mm & (~mm + 1u);
-                mm &= mm - 1u;
-            }
-        }
-        mask &= ~batch;
-        if ((batch >> lane) & 1u) {
-            const int slot = __popc(batch & ((1u << lane) - 1u));
-            acc.stage(stage + slot * C::SS);
-            stage_base[slot] = cur_base | ((lane % LPP) << 28);
-            acc.zero();
-        }
-        __syncwarp();
-        add_staged<C::R, C::SS, LPP, false>(__popc(batch), stage, stage_base, plan.moff,
-                                            plan.valid, plan.fstride, tile, lane);
-    }
-}
-
-// Lanes in `mask` (whose bin moved one step along k) hand the first k-plane
-// of their sums to the node tile and shift the rest down: every lane of the
-// mask stages its plane in its own slot and shifts (one pass for the warp),
-// then the warp adds the planes in lane order.
-template <int ORDER, int LPP, bool STAG>
-__device__ __forceinline__ void merge_plane(unsigned mask, P2GAcc<ORDER, LPP, STAG>& acc,
-                                            int cur_base, const MergePlan<ORDER, LPP, STAG>& plan,
-                                            TileVal* tile, float* stage, int* stage_base, int lane)
-{
-    using C = P2GCfg<ORDER, LPP, false, STAG>;
-    if ((mask >> lane) & 1u) {
-        acc.stage_plane(stage + lane * C::PS);
-        acc.shift_k();
-    }
-    stage_base[lane] = cur_base | ((lane % LPP) << 28);
-    __syncwarp();
-    add_staged<C::RP, C::PS, LPP, true>(mask, stage, stage_base, plan.poff, plan.pvalid,
-                                        plan.fstride, tile, lane);
 }
 
 // Bin inside tile t of a particle from its sort key; false if the key is
@@ -707,7 +336,7 @@ __device__ __forceinline__ bool locate_record(const MeshP& mp, const TileP& tp, 
 // past a non-periodic mesh end are left out -- no stencil reaches them).
 // The integer sums do not depend on the order of the reductions.
 template <int ORDER>
-__device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, const TileVal* tile, int i_lo,
+__device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, const float* tile, int i_lo,
                                                 int i_hi, const int ob[3], float* buf_f,
                                                 int buf_nodes, int lane)
 {
@@ -735,15 +364,14 @@ __device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, const TileVal*
             const int row = r0 + q;
             const int i = i_lo + row / e1, j = row - (row / e1) * e1;
             const int idx = i * tp.SI + j * tp.SJ + k;
+            const float4 v = reinterpret_cast<const float4*>(tile)[idx];
+            const float x[4] = {v.x, v.y, v.z, v.w};
             long long w[4];
 #pragma unroll
-            for (int f = 0; f < 4; ++f) {
-                const TileVal x = tile[f * tp.P + idx];
-                w[f] = x != TileVal(0)
-                           ? to_fixed(f == 0 ? A.gm : A.gmu,
-                                      x * (TileVal)(f == 0 ? A.scale_m : A.scale_mu))
-                           : 0LL;
-            }
+            for (int f = 0; f < 4; ++f)
+                w[f] = x[f] != 0.f ? to_fixed(f == 0 ? A.gm : A.gmu,
+                                              x[f] * (f == 0 ? A.scale_m : A.scale_mu))
+                                   : 0LL;
             longlong2* d = reinterpret_cast<longlong2*>(buf + 4 * node);
             d[0] = make_longlong2(w[0], w[1]);
             d[1] = make_longlong2(w[2], w[3]);
@@ -764,36 +392,40 @@ __device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, const TileVal*
         }
         bulk_commit();
     }
-    bulk_wait_read();  // the buffer is the next item's ring
+    bulk_wait_read();  // the buffer is the next item's table
     __syncwarp();
 }
 
 // One P2G work item (tile t, particles [a, b)) by the calling warp.  `warp_smem`
-// holds p2g_warp_floats<ORDER, LPP, REC>(P) floats (16-byte aligned),
-// `stage_base` kStageLanes ints of shared memory.
-template <int ORDER, int LPP, bool REC = false, bool STAG = false>
-__device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, float* warp_smem,
-                         int* stage_base)
+// holds p2g_warp_floats<ORDER, STAG>(P) floats (16-byte aligned).  REC: the
+// particles' positions arrive as spline records (in-cell fraction of the
+// logical position along each dimension in FP32, and the sort key of the bin)
+// instead of the FP64 positions.
+//
+// Bound: issue slots and shared-memory wavefronts together (quadratic 128^3
+// clustered: 28 warp instructions per particle, 60 % of the issue slots and of
+// the shared-memory pipe at 14 warps per SM; 20 warps, tile (4, 4, 8), are no
+// faster).  Measured against one lane (cubic: 4) per particle and stream, with
+// up to 108 sums per lane: cubic 128^3 8 per cell 1.52 -> 0.85 ms, quadratic 256^3
+// 8 per cell clustered 5.53 -> 5.24 ms, a batch of 24 small problems 2.16 -> 1.07
+// ms.  The next step's entry is read before the current one is used (quadratic
+// 5.80 -> 5.35 ms, cubic 0.95 -> 0.85 ms).  Not kept: the streams that move found
+// one by one (5.50 ms instead of testing each); packed FP32 pairs, whose
+// coefficients need more shared-memory reads than they save instructions.
+template <int ORDER, bool REC = false, bool STAG = false>
+__device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, float* warp_smem)
 {
-    using C = P2GCfg<ORDER, LPP, REC, STAG>;
-    using Acc = P2GAcc<ORDER, LPP, STAG>;
-    static_assert(C::SV == P2GCfg<ORDER, LPP, false, STAG>::SV &&
-                      C::SS == P2GCfg<ORDER, LPP, false, STAG>::SS,
-                  "the record form changes only the ring");
-    constexpr int K = C::K;
+    using C = P2GCfg<ORDER, STAG>;
+    constexpr int K = C::K, KK = C::KK, NV = C::NV, NF = C::NF, S = C::S, B = C::B;
     const MeshP& mp = A.mp;
     const TileP& tp = A.tp;
     const int lane = threadIdx.x & 31;
-    const int run = lane / LPP, h = lane % LPP;
-    float* ring = warp_smem;
-    float* stage = warp_smem + C::STAGE_OFF;
-    TileVal* tile = reinterpret_cast<TileVal*>(warp_smem + C::TILE_OFF);
+    float* table = warp_smem;
+    float* wrow = warp_smem + 32 * C::ENTRY;
+    float* tile = warp_smem + C::TILE_OFF;
 
     int ob[3];
     tile_origin(tp, t, ob);
-    const int U = (int)((b - a + C::RUNS - 1) / C::RUNS);
-    const int64_t my0 = a + (int64_t)run * U;
-    const int cnt = (int)max((int64_t)0, min(my0 + U, b) - my0);
     // bin rows spanned by the item (keys are i-major within a tile): the
     // first and last particle bound them; the item's node box is these rows
     // plus the halo, over the whole tile along j and k
@@ -817,255 +449,235 @@ __device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, floa
         }
     }
 
-    for (int i = lane; i < C::NF * tp.P; i += 32) tile[i] = TileVal(0);
-    MergePlan<ORDER, LPP, STAG> plan;
-    plan.init(tp, lane);
+    for (int i = lane; i < NF * tp.P / 2; i += 32)
+        reinterpret_cast<float2*>(tile)[i] = make_float2(0.f, 0.f);
     const float D = (ORDER >= 2) ? inertial_scaling<ORDER, float>(mp.dx[0]) : 1.f;
     const float Dh = D * (float)mp.dx[0];
 
-    auto slot = [&](int q) { return ring + (q % C::DEPTH) * C::RING; };
-    // the copies of a particle record are spread over the run's lanes: copy
-    // j is issued by lane h == j % LPP (position: 3 x 8 bytes or one 16-byte
-    // record, c: 3 x 16 bytes, m: 4 bytes)
-    constexpr int NX = REC ? 1 : 3;
-    auto issue = [&](int q) {
-        if (q < cnt) {
-            const int64_t p = my0 + q;
-            float* s = slot(q);
-            float* sx = s + C::RING_X + run * C::XS;
-            float* sc = s + C::RING_C + run * 12;
-#pragma unroll
-            for (int j = 0; j < NX + 4; ++j) {
-                if (j % LPP != h) continue;
-                if (j < NX) {
-                    if constexpr (REC) cp_async<16>(sx, A.rec + 4 * p);
-                    else cp_async<8>(sx + 2 * j, A.x + 3 * p + j);
-                } else if (j < NX + 3) {
-                    cp_async<16>(sc + 4 * (j - NX), A.c + 12 * p + 4 * (j - NX));
-                } else {
-                    cp_async<4>(s + C::RING_M + run, A.m + p);
-                }
-            }
-        }
-        cp_async_commit();
-    };
-#pragma unroll
-    for (int q = 0; q < C::DEPTH - 1; ++q) issue(q);
-
-    // Spline and bin of one particle, and its mass and coefficients, read
-    // from its ring slot.
-    struct Part {
-        Spline1D<ORDER, float> sp[3];
-        int lb[3];
-        bool ok;
-    };
-    auto locate_slot = [&](int q, Part& P) {
-        P.ok = false;
-        P.lb[0] = P.lb[1] = P.lb[2] = 0;
-        if (q >= cnt) return;
-        if constexpr (REC) {
-            const float4 r = *reinterpret_cast<const float4*>(slot(q) + C::RING_X + run * 4);
-            P.ok = locate_record<ORDER>(mp, tp, t, r, P.sp, P.lb);
-        } else {
-            const double* sx = reinterpret_cast<const double*>(slot(q) + C::RING_X + run * 6);
-            const double xp[3] = {sx[0], sx[1], sx[2]};
-            P.ok = locate<ORDER>(mp, tp, xp, ob, P.sp, P.lb);
-        }
-        // a particle out of the item's rows (the particles are not sorted)
-        // is skipped like one of another tile
-        P.ok = P.ok && P.lb[0] >= i_lo && P.lb[0] <= i_hi;
-        if (!P.ok && A.err && h == 0) atomicAdd(A.err, 1);
-    };
-    auto read_c = [&](int q, float cp[12], float& mass) {
-        const float* sl = slot(q);
-        const float* sc = sl + C::RING_C + run * 12;
-#pragma unroll
-        for (int v = 0; v < 3; ++v) {
-            const float4 w = *reinterpret_cast<const float4*>(sc + 4 * v);
-            cp[4 * v] = w.x;
-            cp[4 * v + 1] = w.y;
-            cp[4 * v + 2] = w.z;
-            cp[4 * v + 3] = w.w;
-        }
-        mass = sl[C::RING_M + run];
-    };
-    // cp[r * 3 + d] = c_p(r, d); field g of the lane: mass (g = 0) or
-    // momentum d = g - 1 (staggered: d = the entity's dimension)
-    auto centre_form = [&](const float cp[12], const Spline1D<ORDER, float> sp[3],
-                           float E[C::F], float G[C::F][3]) {
-#pragma unroll
-        for (int f = 0; f < C::F; ++f) {
-            const int g = C::ISPLIT ? f : h * C::F + f;
-            if (g == 0) {
-                E[f] = 1.f;
-                G[f][0] = G[f][1] = G[f][2] = 0.f;
+    // the lane as evaluator: slot es of stream eg
+    const int U = (int)((b - a + S - 1) / S);  // particles per stream
+    const int eg = lane / B, es = lane - eg * B;
+    const int64_t p_first = a + (int64_t)eg * U;
+    const int ecnt = eg < S ? (int)max((int64_t)0, min(p_first + U, b) - p_first) : 0;
+    // its next particle, read one table ahead
+    float4 nc[3], nrec = make_float4(0.f, 0.f, 0.f, 0.f);
+    double nx[3] = {0.0, 0.0, 0.0};
+    float nm = 0.f;
+    auto fetch = [&](int s0) {
+        if (s0 + es < ecnt) {
+            const int64_t p = p_first + s0 + es;
+            if constexpr (REC) {
+                nrec = __ldg(reinterpret_cast<const float4*>(A.rec) + p);
             } else {
-                const int d = STAG ? A.stag : g - 1;
-                const float bx = d == 0 ? cp[3] : (d == 1 ? cp[4] : cp[5]);
-                const float by = d == 0 ? cp[6] : (d == 1 ? cp[7] : cp[8]);
-                const float bz = d == 0 ? cp[9] : (d == 1 ? cp[10] : cp[11]);
-                const float v = d == 0 ? cp[0] : (d == 1 ? cp[1] : cp[2]);
-                const float bd = fmaf(bz, sp[2].d[C::N0],
-                                      fmaf(by, sp[1].d[C::N0], bx * sp[0].d[C::N0]));
-                E[f] = fmaf(D, bd, v);
-                G[f][0] = Dh * bx;
-                G[f][1] = Dh * by;
-                G[f][2] = Dh * bz;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) nx[d] = __ldg(A.x + 3 * p + d);
             }
+#pragma unroll
+            for (int v = 0; v < 3; ++v) nc[v] = __ldg(reinterpret_cast<const float4*>(A.c) + 3 * p + v);
+            nm = __ldg(A.m + p);
         }
     };
-    auto linear_form = [&](const float cp[12], float co[C::F][4]) {
+    auto evaluate = [&](int s0) {
+        float* e = table + lane * C::ENTRY;
+        float out[C::ENTRY], wxy[C::WROWS];
 #pragma unroll
-        for (int f = 0; f < C::F; ++f) {
-            const int g = h * C::F + f;
-            if (g == 0) {
-                co[f][0] = 1.f;
-                co[f][1] = co[f][2] = co[f][3] = 0.f;
+        for (int v = 0; v < C::ENTRY; ++v) out[v] = 0.f;
+#pragma unroll
+        for (int v = 0; v < C::WROWS; ++v) wxy[v] = 0.f;
+        int at = -1;
+        if (s0 + es < ecnt) {
+            Spline1D<ORDER, float> sp[3];
+            int lb[3];
+            bool ok;
+            if constexpr (REC) {
+                ok = locate_record<ORDER>(mp, tp, t, nrec, sp, lb);
             } else {
-                const int d = STAG ? A.stag : g - 1;
-                co[f][0] = d == 0 ? cp[0] : (d == 1 ? cp[1] : cp[2]);
-                co[f][1] = d == 0 ? cp[3] : (d == 1 ? cp[4] : cp[5]);
-                co[f][2] = d == 0 ? cp[6] : (d == 1 ? cp[7] : cp[8]);
-                co[f][3] = d == 0 ? cp[9] : (d == 1 ? cp[10] : cp[11]);
+                ok = locate<ORDER>(mp, tp, nx, ob, sp, lb);
             }
-        }
-    };
-
-    Acc acc;
-    acc.zero();
-    int cur = -1, cur_base = 0;
-    if constexpr (C::SHARE) {
-        // Groups of LPP steps: lane h of a run evaluates particle s0 + h of
-        // the run (record, splines, bin, affine form) and writes it to the
-        // table; in sub-step q the run's lanes read entry (q, run).  Entries
-        // are sub-step-major so that the 8 runs' entries of one sub-step fall
-        // on different banks, and the entries of sub-step q are shifted by 8 q
-        // floats so that the 8 lanes of a quarter warp (2 runs x 4 sub-steps)
-        // write to different banks too (ENTRY * 8 is a multiple of 32).  The
-        // ring holds one group (DEPTH == LPP): the
-        // next group's records are issued once the entries are written and
-        // arrive during the sub-steps.  Same arithmetic as the loop below.
-        static_assert(C::DEPTH == LPP, "one group in the ring");
-        float* table = warp_smem + C::TILE_OFF + C::NF * tp.P * kTileWords;
-        issue(C::DEPTH - 1);  // steps 0 .. DEPTH - 2 are in flight
-        for (int s0 = 0; s0 < U; s0 += LPP) {
-            cp_async_wait<0>();  // the group's records have landed
-            __syncwarp();        // ... for every lane of each run
-            {
-                const int q = s0 + h;
-                Spline1D<ORDER, float> sp[3];
-                int lb[3] = {0, 0, 0};
-                bool ok = false;
-                float cp[12], mass = 0.f;
+            // a particle out of the item's rows (the particles are not sorted)
+            // is skipped like one of another tile
+            ok = ok && lb[0] >= i_lo && lb[0] <= i_hi;
+            if (!ok) {
+                if (A.err) atomicAdd(A.err, 1);
+            } else {
+                at = lb[0] * tp.SI + lb[1] * tp.SJ + lb[2];
+                // c_p(r, d) is element 3 r + d
+                const float cp[12] = {nc[0].x, nc[0].y, nc[0].z, nc[0].w, nc[1].x, nc[1].y,
+                                      nc[1].z, nc[1].w, nc[2].x, nc[2].y, nc[2].z, nc[2].w};
 #pragma unroll
-                for (int v = 0; v < 12; ++v) cp[v] = 0.f;
+                for (int f = 0; f < NV; ++f) {
+                    const int d = STAG ? A.stag : f;
+                    float v[4];
 #pragma unroll
-                for (int d = 0; d < 3; ++d)
+                    for (int r = 0; r < 4; ++r)
+                        v[r] = d == 0 ? cp[3 * r] : (d == 1 ? cp[3 * r + 1] : cp[3 * r + 2]);
+                    if constexpr (ORDER >= 2) {
+                        const float bd =
+                            fmaf(v[3], sp[2].d[1], fmaf(v[2], sp[1].d[1], v[1] * sp[0].d[1]));
+                        out[4 * f] = fmaf(D, bd, v[0]);
 #pragma unroll
-                    for (int n = 0; n < K; ++n) sp[d].w[n] = sp[d].d[n] = 0.f;
-                if (q < cnt) {
-                    const float4 r = *reinterpret_cast<const float4*>(slot(q) + C::RING_X + run * 4);
-                    ok = locate_record<ORDER>(mp, tp, t, r, sp, lb);
-                    // a particle out of the item's rows is skipped like one of
-                    // another tile
-                    ok = ok && lb[0] >= i_lo && lb[0] <= i_hi;
-                    if (!ok && A.err) atomicAdd(A.err, 1);
-                    read_c(q, cp, mass);
-                }
-                float E[C::F], G[C::F][3];
-                centre_form(cp, sp, E, G);
-                float4* e =
-                    reinterpret_cast<float4*>(table + (h * C::RUNS + run) * C::ENTRY + 8 * h);
-                e[0] = make_float4(sp[0].w[0], sp[0].w[1], sp[0].w[2], sp[0].w[3]);
-                e[1] = make_float4(sp[1].w[0], sp[1].w[1], sp[1].w[2], sp[1].w[3]);
-                e[2] = make_float4(sp[2].w[0], sp[2].w[1], sp[2].w[2], sp[2].w[3]);
-                e[3] = make_float4(mass, E[1], E[2], E[3]);
-                e[4] = make_float4(G[1][0], G[1][1], G[1][2], G[2][0]);
-                e[5] = make_float4(G[2][1], G[2][2], G[3][0], G[3][1]);
-                const int lbin = ok ? (lb[0] * tp.T[1] + lb[1]) * tp.T[2] + lb[2] : -1;
-                e[6] = make_float4(G[3][2], __int_as_float(lbin),
-                                   __int_as_float(lb[0] * tp.SI + lb[1] * tp.SJ + lb[2]),
-                                   __int_as_float(lb[2]));
-            }
-            __syncwarp();  // entries written, the group's ring slots read
+                        for (int r = 1; r < 4; ++r) out[4 * f + r] = Dh * v[r];
+                    } else {
+                        out[4 * f] = v[0] * nm;
 #pragma unroll
-            for (int q = 0; q < LPP; ++q) issue(s0 + LPP + q);
-            for (int q = 0; q < LPP; ++q) {
-                const float* ef = table + (q * C::RUNS + run) * C::ENTRY + 8 * q;
-                const float4* e = reinterpret_cast<const float4*>(ef);
-                const float wx = ef[h];
-                const float4 wy4 = e[1], wz4 = e[2], me = e[3], g0 = e[4], g1 = e[5], g2 = e[6];
-                const int lbin = __float_as_int(g2.y);
-                const bool ok = lbin >= 0;
-                const bool chg = ok && cur >= 0 && lbin != cur;
-                const bool kstep = chg && lbin == cur + 1 && __float_as_int(g2.w) != 0;
-                const unsigned pm = __ballot_sync(kFull, kstep);
-                const unsigned fm = __ballot_sync(kFull, chg && !kstep);
-                if (pm) merge_plane(pm, acc, cur_base, plan, tile, stage, stage_base, lane);
-                if (fm) merge_partials(fm, acc, cur_base, plan, tile, stage, stage_base, lane);
-                if (ok) {
-                    if (lbin != cur) {
-                        cur = lbin;
-                        cur_base = __float_as_int(g2.z);
+                        for (int r = 1; r < 4; ++r) out[4 * f + r] = v[r] * nm * (float)mp.rdx[r - 1];
                     }
-                    const float wy[4] = {wy4.x, wy4.y, wy4.z, wy4.w};
-                    const float wz[4] = {wz4.x, wz4.y, wz4.z, wz4.w};
-                    const float E[C::F] = {1.f, me.y, me.z, me.w};
-                    const float G[C::F][3] = {{0.f, 0.f, 0.f},
-                                              {g0.x, g0.y, g0.z},
-                                              {g0.w, g1.x, g1.y},
-                                              {g1.z, g1.w, g2.x}};
-                    acc.add_isplit(wx, wy, wz, me.x, E, G, h);
+                }
+#pragma unroll
+                for (int k = 0; k < K; ++k) out[C::WZ + k] = sp[2].w[k];
+                if constexpr (ORDER == 1) {
+                    out[C::WZ + K] = nm;
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        wxy[k] = sp[0].w[k];
+                        wxy[K + k] = sp[1].w[k];
+                    }
+                } else {
+#pragma unroll
+                    for (int i = 0; i < K; ++i) {
+                        const float wx = sp[0].w[i] * nm;
+#pragma unroll
+                        for (int j = 0; j < K; ++j) wxy[i * K + j] = wx * sp[1].w[j];
+                    }
                 }
             }
         }
-    } else
-    for (int s = 0; s < U; ++s) {
-        __syncwarp();  // no lane still reads the slot refilled next
-        issue(s + C::DEPTH - 1);
-        cp_async_wait<C::DEPTH - 1>();  // record s has landed
-        __syncwarp();                   // ... for every lane of its run
-        Part P;
-        locate_slot(s, P);
-        const bool ok = P.ok;
-        const int* lb = P.lb;
-        const int lbin = ok ? (lb[0] * tp.T[1] + lb[1]) * tp.T[2] + lb[2] : -1;
-        // a bin change to the next bin along k (same i, j) keeps two thirds
-        // of the stencil: only the finished k-plane is merged
-        const bool chg = ok && cur >= 0 && lbin != cur;
-        const bool kstep = chg && lbin == cur + 1 && lb[2] != 0;
-        const unsigned pm = __ballot_sync(kFull, kstep);
-        const unsigned fm = __ballot_sync(kFull, chg && !kstep);
-        if (pm) merge_plane(pm, acc, cur_base, plan, tile, stage, stage_base, lane);
-        if (fm) merge_partials(fm, acc, cur_base, plan, tile, stage, stage_base, lane);
-        if (ok) {
-            if (lbin != cur) {
-                cur = lbin;
-                cur_base = lb[0] * tp.SI + lb[1] * tp.SJ + lb[2];
+        out[C::AT] = __int_as_float(at);
+#pragma unroll
+        for (int v = 0; v < (C::AT + 4) / 4; ++v)
+            reinterpret_cast<float4*>(e)[v] =
+                make_float4(out[4 * v], out[4 * v + 1], out[4 * v + 2], out[4 * v + 3]);
+#pragma unroll
+        for (int v = 0; v < C::WROWS; ++v) wrow[v * C::WROW + lane] = wxy[v];
+    };
+
+    // the lane as k-row (ri, rj) of stream g
+    const bool act = lane < S * KK;
+    const int g = act ? lane / KK : 0, row = act ? lane - g * KK : 0;
+    const int ri = row / K, rj = row - ri * K;
+    const float oi = (float)(ri - 1), oj = (float)(rj - 1);
+    float* trow = tile + NF * (ri * tp.SI + rj * tp.SJ);
+    float acc[NF][K];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[f][k] = 0.f;
+    int cur = -1;  // tile offset of the sums' stencil
+    auto add_node = [&](int k) {
+        if constexpr (NF == 4) {
+            float4* d = reinterpret_cast<float4*>(trow + 4 * (cur + k));
+            const float4 v = *d;
+            *d = make_float4(v.x + acc[0][k], v.y + acc[1][k], v.z + acc[NF - 2][k], v.w + acc[NF - 1][k]);
+        } else {
+            float2* d = reinterpret_cast<float2*>(trow + 2 * (cur + k));
+            const float2 v = *d;
+            *d = make_float2(v.x + acc[0][k], v.y + acc[1][k]);
+        }
+    };
+    // The lanes whose stream moves (mine; step: by one node along k) add their
+    // finished nodes to the tile, stream after stream; `moved`: ballot of mine.
+    auto merge = [&](unsigned moved, bool mine, bool step) {
+#pragma unroll
+        for (int q = 0; q < S; ++q) {
+            if (!((moved >> (q * KK)) & 1u)) continue;
+            if (mine && g == q) {
+                add_node(0);
+                if (!step) {
+#pragma unroll
+                    for (int k = 1; k < K; ++k) add_node(k);
+                }
             }
-            float cp[12], mass;
-            read_c(s, cp, mass);
-            if constexpr (ORDER >= 2) {
-                float E[C::F], G[C::F][3];
-                centre_form(cp, P.sp, E, G);
-                acc.add(P.sp, mass, E, G, h);
+            __syncwarp();
+        }
+        if (mine) {
+#pragma unroll
+            for (int f = 0; f < NF; ++f)
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+                    acc[f][k] = step && k + 1 < K ? acc[f][k + 1 < K ? k + 1 : k] : 0.f;
+        }
+    };
+
+    fetch(0);
+    for (int s0 = 0; s0 < U; s0 += B) {
+        __syncwarp();  // the table has been read
+        evaluate(s0);
+        __syncwarp();
+        fetch(s0 + B);
+        const int steps = min(B, U - s0);
+        const float* e = table + g * B * C::ENTRY;
+        const float* w = wrow + g * B;
+        // a particle's entry as the lane reads it, one step ahead of its use
+        // (past the last step: the words after the entries, not used)
+        struct Entry {
+            float4 v[NV];
+            float wz[K], wa, wb;  // wa: w_x w_y m of the k-row (linear: w_x; wb: w_y), m
+            float m;
+            int at;
+        };
+        auto read = [&](int q) {
+            Entry r;
+            const float* p = e + q * C::ENTRY;
+#pragma unroll
+            for (int f = 0; f < NV; ++f) r.v[f] = *reinterpret_cast<const float4*>(p + 4 * f);
+            const float4 z = *reinterpret_cast<const float4*>(p + C::WZ);
+            const float zz[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+            for (int k = 0; k < K; ++k) r.wz[k] = zz[k];
+            const int at = __float_as_int(K < 4 ? z.w : p[C::AT]);
+            r.at = act ? at : -1;
+            r.m = ORDER == 1 ? z.z : 0.f;
+            r.wa = ORDER == 1 ? w[ri * C::WROW + q] : w[row * C::WROW + q];
+            r.wb = ORDER == 1 ? w[(K + rj) * C::WROW + q] : 0.f;
+            return r;
+        };
+        Entry next = read(0);
+#pragma unroll 2
+        for (int q = 0; q < steps; ++q) {
+            const Entry r = next;
+            next = read(q + 1);
+            const bool mine = r.at >= 0 && cur >= 0 && r.at != cur;
+            const unsigned moved = __ballot_sync(kFull, mine);
+            if (moved) merge(moved, mine, r.at == cur + 1);
+            if (r.at >= 0) cur = r.at;
+            if constexpr (ORDER == 1) {
+                const float wx = r.wa, wy = r.wb;
+                const float wab = wx * wy, mab = r.m * wab;
+                const float sx = ri ? wy : -wy, sy = rj ? wx : -wx;
+                acc[0][0] = fmaf(mab, r.wz[0], acc[0][0]);
+                acc[0][1] = fmaf(mab, r.wz[1], acc[0][1]);
+#pragma unroll
+                for (int f = 0; f < NV; ++f) {
+                    const float p = fmaf(r.v[f].z, sy, fmaf(r.v[f].y, sx, r.v[f].x * wab));
+                    const float c = r.v[f].w * wab;
+                    acc[1 + f][0] += fmaf(p, r.wz[0], -c);
+                    acc[1 + f][1] += fmaf(p, r.wz[1], c);
+                }
             } else {
-                float co[C::F][4];
-                linear_form(cp, co);
-                acc.add_linear(P.sp, mass, co);
+                float wn[K];
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    wn[k] = r.wa * r.wz[k];
+                    acc[0][k] += wn[k];
+                }
+#pragma unroll
+                for (int f = 0; f < NV; ++f) {
+                    const float p = fmaf(oj, r.v[f].z, fmaf(oi, r.v[f].y, r.v[f].x));
+#pragma unroll
+                    for (int k = 0; k < K; ++k)
+                        acc[1 + f][k] = fmaf(wn[k], add_steps(k - 1, p, r.v[f].w), acc[1 + f][k]);
+                }
             }
         }
     }
-    cp_async_wait<0>();
-    const unsigned fm = __ballot_sync(kFull, cur >= 0);
-    if (fm) merge_partials(fm, acc, cur_base, plan, tile, stage, stage_base, lane);
+    const unsigned last = __ballot_sync(kFull, cur >= 0);
+    if (last) merge(last, cur >= 0, false);
     // the item's node box, rounded to fixed point and added to HBM: by bulk
-    // reductions of whole k-rows into a packed accumulator (the ring and the
-    // staging area hold the rounded rows), else node by node (nodes that
-    // received nothing are skipped)
-    if (!STAG && A.bulk_flush && __any_sync(kFull, cur >= 0)) {
+    // reductions of whole k-rows into a packed accumulator (the table holds the
+    // rounded rows), else node by node (nodes that received nothing are skipped)
+    if (!STAG && A.bulk_flush && last) {
         flush_rows_bulk<ORDER>(A, tile, i_lo, i_hi, ob, warp_smem, C::TILE_OFF / 8, lane);
-    } else if (__any_sync(kFull, cur >= 0)) {
+    } else if (last) {
         const int e1 = tp.NT[1], e2 = tp.NT[2];
         const int total = (i_hi - i_lo + K) * e1 * e2;
         for (int e = lane; e < total; e += 32) {
@@ -1081,11 +693,11 @@ __device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, floa
             char* bm = halo_route(A.hp, 0, A.gm.data, gi, gx_m);
             char* bmu = halo_route(A.hp, 1, A.gmu.data, gi, gx_mu);
 #pragma unroll
-            for (int f = 0; f < C::NF; ++f) {
-                const TileVal v = tile[f * tp.P + idx];
-                if (v != TileVal(0)) {
-                    const long long q = to_fixed(
-                        f == 0 ? A.gm : A.gmu, v * (TileVal)(f == 0 ? A.scale_m : A.scale_mu));
+            for (int f = 0; f < NF; ++f) {
+                const float v = tile[NF * idx + f];
+                if (v != 0.f) {
+                    const long long q =
+                        to_fixed(f == 0 ? A.gm : A.gmu, v * (f == 0 ? A.scale_m : A.scale_mu));
                     unsigned long long* dst =
                         f == 0 ? reinterpret_cast<unsigned long long*>(bm) +
                                      A.gm.index(gx_m, gj, gk, 0)
@@ -1137,7 +749,7 @@ __device__ __forceinline__ void region_range(const MeshP& mp, const TileP& tp, i
 
 __device__ __forceinline__ uint32_t tile_items_of(const TileP& tp, int64_t s)
 {
-    return __ldg(tp.items + s + 1) - __ldg(tp.items + s);
+    return (__ldg(tp.items + s + 1) - __ldg(tp.items + s)) * (uint32_t)tp.split;
 }
 
 // Items of the tiles that touch region `reg` of tile (q0, q1, q2).
@@ -1452,14 +1064,14 @@ __device__ void g2p_item(const G2PArgs& A, int64_t t, int64_t a, int64_t b, floa
 
 // host helpers (tiled.cu)
 bool fused_update_fits(const TileP& tp, int order);
-bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, TileP* tp, int lpp = 0,
-                int nf = 4);
+bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n, TileP* tp,
+                bool p2g_strides = false);
+int64_t item_bound(const TileP& tp, int64_t n);  // items (parts) of n particles, at most
 int device_smem_optin();
 bool packed_x(const PField& x);
 bool packed_m(const PField& m);
 bool packed_c(const PField& c);
-int default_lpp(int order);
-bool valid_lpp(int order, int lpp, bool stag = false);
-size_t p2g_warp_bytes(int order, int lpp, int P, bool rec = false, bool stag = false);
+bool valid_lanes(int order, int lanes, bool stag = false);
+size_t p2g_warp_bytes(int order, int P, bool stag = false);
 
 }  // namespace pb
