@@ -403,8 +403,8 @@ class PolyPIC:
     def p2g(m_p, u_p, c_p, mu_i, m_i, dt, sd, stream=None, error_count=None, bins=None,
             overflow_count=None):
         """PolyPIC::p2g(m_p, u_p, c_p, mu_i, m_i, dt, sd) -- field before mass.
-        With bins (cell-sorted particles) the FP32 form runs the tiled kernel
-        (bit-identical grid)."""
+        With bins (cell-sorted particles) the FP32 form counts particles that
+        have left the tile they were sorted into instead of adding them."""
         ncomp = c_p.shape[2]
         _check_grid_extent(m_i, sd.desc.mesh)
         _check_grid_extent(mu_i, sd.desc.mesh)

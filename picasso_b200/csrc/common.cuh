@@ -342,16 +342,9 @@ __device__ __forceinline__ bool resolve_stencil(const MeshP& mp, int d, int s0, 
 // ---------------------------------------------------------------------------
 // accumulation into grid arrays
 // ---------------------------------------------------------------------------
-// FP64 grid: hardware FP64 atomic add.  I64 fixed-point grid: the value is
-// rounded to the nearest multiple of 2^-bits and added as a 64-bit integer,
-// which makes the sum independent of the order of contributions.
-struct AccF64 {
-    __device__ __forceinline__ static void add(const GField& g, int i, int j, int k, int c,
-                                               double v, double /*scale*/)
-    {
-        atomicAdd(g.ptr<double>(i, j, k, c), v);
-    }
-};
+// I64 fixed-point grid: the value is rounded to the nearest multiple of 2^-bits
+// and added as a 64-bit integer, which makes the sum independent of the order of
+// contributions.
 struct AccFixed {
     __device__ __forceinline__ static void add(const GField& g, int i, int j, int k, int c,
                                                double v, double scale)

@@ -1,8 +1,9 @@
-// PolyPIC particle-to-grid and grid-to-particle transfers, one thread per
-// particle.  Linear (8 modes) follows Picasso_PolyPIC.hpp; quadratic (27
-// modes) has no reference implementation and is the 3-D tensor-product
-// extension of the reference's 2-D derivation (doc/polypic/
-// polypic_2d_quadratic.nb): per dimension the weight-orthogonal modes
+// PolyPIC particle-to-grid (streams of particles, a lane per k-row of the stencil)
+// and grid-to-particle transfers (one thread per particle).  Linear (8 modes)
+// follows Picasso_PolyPIC.hpp; quadratic (27 modes) has no reference
+// implementation and is the 3-D tensor-product extension of the reference's 2-D
+// derivation (doc/polypic/polypic_2d_quadratic.nb): per dimension the
+// weight-orthogonal modes
 //   s0 = 1, s1 = r, s2 = r^2 - h^2/4 - alpha r,
 //   alpha = p (h^2 - 4 p^2) / h^2, p = particle offset from the centre knot,
 // and the G2P coefficients are the weighted least-squares projections
@@ -26,26 +27,10 @@ __host__ __device__ __forceinline__ constexpr int mode_deg(int r, int d)
                   (2 * r)) & 3ull);
 }
 
-// a[i] for a register array and a run-time i (a select chain, no local memory).
-template <int K, class T>
-__device__ __forceinline__ T pick(const T (&a)[K], int i)
-{
-    T v = a[0];
-#pragma unroll
-    for (int q = 1; q < K; ++q) v = (i == q) ? a[q] : v;
-    return v;
-}
-
 template <class R>
 __device__ __forceinline__ R quad_alpha(R p, R h)
 {
     return p * (h * h - R(4) * p * p) / (h * h);
-}
-
-template <class R>
-__device__ __forceinline__ R mode1d(int deg, R r, R h, R alpha)
-{
-    return deg == 0 ? R(1) : (deg == 1 ? r : r * r - R(0.25) * h * h - alpha * r);
 }
 
 // 3x3 inverse by cofactors times 1/det (BatchedLinearAlgebra.hpp:4337-4350,
@@ -70,133 +55,389 @@ __device__ __forceinline__ void inverse3(const R a[9], R inv[9])
 // ---------------------------------------------------------------------------
 // P2G: PolyPIC.hpp:41-130 (collocated) and :140-229 (staggered)
 // ---------------------------------------------------------------------------
-// Spline and stencil indices of a particle on the whole local mesh (periodic
-// wrap, bounds check): the placement of the plain kernels.
-template <int ORDER, class R>
-struct MeshPlace {
-    const MeshP& mp;
-    __device__ __forceinline__ bool operator()(const double xp[3], Spline1D<ORDER, R> sp[3],
-                                               int idx[3][SplineTraits<ORDER>::K]) const
-    {
-        bool ok = true;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            eval_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
-            ok = ok && resolve_stencil<SplineTraits<ORDER>::K>(mp, d, sp[d].s0, idx[d]);
-        }
-        return ok;
-    }
+// A warp takes a contiguous segment of the particles, cut into S streams (3 for
+// quadratic, 8 for linear splines) that it sweeps side by side.  Its lanes first
+// stage the next particles of every stream in shared memory -- one lane per
+// particle evaluates the spline, the backtracking matrix A^-1 and the mode shifts;
+// the mode coefficients are copied in the order of their degrees (a, b, c) -- and
+// then, step by step, K^2 lanes per stream, one for every k-row of the stencil,
+// evaluate the stream's next particle at the row's K nodes,
+//   w m sum_abc f0_a(xi_0) f1_b(xi_1) f2_c(xi_2) c_abc,  xi = A^-1 d,
+// one dimension after the other, and add it to sums in registers: FP64, or 64-bit
+// fixed point with every contribution rounded.  Only when the stream's stencil
+// moves are the finished nodes (one k-plane for a move along k, else all) added
+// to the grid.  The particles may come in any order; sorted ones move rarely.
+// The fixed-point sums are integers: the grid does not depend on the particles'
+// order, nor on how they are cut into segments and streams.
+//
+// With the bins of cell-sorted particles, one that is not in the tile it was sorted
+// into is counted instead, as the G2P does.
+//
+// Bound: quadratic, the shared-memory wavefronts of the coefficients (81 values are
+// read once per lane group and particle: 64 % of the pipe in FP32, 70 % in FP64)
+// next to the FMAs of the sums (about 100 per node with 3 components) and, in fixed
+// point, 16 instructions per node for the four roundings (57 % of the issue slots);
+// linear, the instructions around the few FMAs: 83 per particle, a third of them for
+// the table, the copies and the moved stencils.  Against one thread per particle
+// with a shared integer tile (FP32) or grid atomics per node (FP64), cell-sorted
+// particles: quadratic FP32 96^3 cells 5 per cell 2.50 -> 1.89 ms, FP64 48^3 0.73 ->
+// 0.44 ms, linear FP32 101 x 67 x 83 0.278 -> 0.276 ms.  Quadratic warps hold 10
+// (FP64: 6) particles per stream in the table and half of them in each of the two
+// coefficient chunks; other splits of the shared memory between table and chunks
+// took 1 to 9 % longer.
+template <int ORDER, int NCU, class R>
+struct PPStreams {
+    static constexpr int K = SplineTraits<ORDER>::K;
+    static constexpr int KK = K * K;
+    static constexpr int D = ORDER + 1;                    // modes per dimension
+    static constexpr int S = 32 / KK;                      // streams
+    // Evaluated particles per stream (table slots), and of those the ones whose
+    // coefficients are in shared memory at a time (two chunks, the next one on its
+    // way while one is used).
+    static constexpr int B = ORDER == 2 ? (sizeof(R) == 8 ? 6 : 10) : 32 / S;
+    static constexpr int H = ORDER == 2 ? B / 2 : B;
+    static_assert(B % H == 0, "whole chunks");
+    static constexpr int P = S * B;
+    static constexpr int AB = (D * D * NCU + 3) & ~3;      // coefficients of degree a, padded
+    static constexpr int CN = D * AB;
+    // Entry of a particle: A^-1, alpha, d_z, (pad), w_z, (pad), d_x, d_y, w_x w_y m.
+    // 36 values: the 16-byte accesses of 8 lanes fall on distinct banks.
+    static constexpr int E_ALPHA = 9, E_DZ = 12, E_WZ = 16, E_DX = 20, E_DY = 20 + K, E_W = 20 + 2 * K;
+    static constexpr int ENTRY = 36;
+    static_assert(E_W + KK <= ENTRY, "a particle's entry");
+    static constexpr int CHUNK = S * H * CN;  // coefficients of a chunk
+    static constexpr size_t kBytes = sizeof(R) * (2 * CHUNK + P * ENTRY) + sizeof(int4) * P;  // per warp
 };
 
-// One particle.  place(xp, sp, idx) evaluates the spline and the stencil's
-// grid indices (false: skip the particle); acc(f, i, j, k, v) adds v to grid
-// field f (0 mass, 1 + d momentum component d); mode(v) returns c_p value v
-// (element v of the particle's record).
-template <int ORDER, int NC, bool STAG, class PT, class R, class Place, class Acc, class Mode>
-__device__ __forceinline__ void polypic_p2g_particle(const MeshP& mp, int64_t p, const PField& x,
-                                                     const PField& m, const PField& u, R dt,
-                                                     int col, int* err, Place&& place, Acc&& acc,
-                                                     Mode&& mode)
+// Consecutive values of shared memory from a 16-byte aligned address.
+template <int N, class R>
+__device__ __forceinline__ void read_shared(const R* p, R (&v)[N])
 {
-    constexpr int K = SplineTraits<ORDER>::K;
-    {
-        Spline1D<ORDER, R> sp[3];
-        int idx[3][K];
-        const double xp[3] = {x.get<double>(p, 0), x.get<double>(p, 1), x.get<double>(p, 2)};
-        if (!place(xp, sp, idx)) {
-            if (err) atomicAdd(err, 1);
-            return;
-        }
-        const R mass = (R)m.get<PT>(p, 0);
-        // affine material motion operator and its inverse (PolyPIC.hpp:81-87)
-        R am[9], ai[9];
+    constexpr int W = 16 / sizeof(R);
+    static_assert(N % W == 0, "whole 16-byte words");
 #pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const R v = dt * (R)u.get<PT>(p, (1 + a) * 3 + b);
-                am[3 * a + b] = (a == b) ? R(1) + v : v;
-            }
-        inverse3(am, ai);
-        R alpha[3] = {R(0), R(0), R(0)};
-        R h[3];
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            h[d] = (R)mp.dx[d];
-            if (ORDER == 2) alpha[d] = quad_alpha(-sp[d].d[1], h[d]);
-        }
-        // modes of the transferred field: all NC columns, or column `col`
-        constexpr int NCU = STAG ? 1 : NC;
-        constexpr int D = ORDER + 1;  // modes per dimension: degrees 0 .. ORDER
-        const int ncp = STAG ? (col >= 0 ? NC : 1) : NC;
-        // The components are transferred in passes of CB (27 FP64 modes: one
-        // at a time, so that a pass holds 27 mode values rather than 81 in
-        // registers).
-        // The basis sum sum_r c_r b_r(xi) is contracted one dimension at a
-        // time: sum_a f0_a sum_b f1_b sum_c f2_c c_(abc).
-        constexpr int CB = (sizeof(R) == 8 && ORDER == 2) ? 1 : NCU;
-#pragma unroll 1
-        for (int d0 = 0; d0 < NCU; d0 += CB) {
-            R cp[D][D][D][CB];
-            // loop over the modes: their degrees fold to constants
-#pragma unroll
-            for (int r = 0; r < D * D * D; ++r)
-#pragma unroll
-                for (int e = 0; e < CB; ++e)
-                    cp[mode_deg(r, 0)][mode_deg(r, 1)][mode_deg(r, 2)][e] =
-                        (R)mode(r * ncp + (STAG ? col : d0 + e));
-            // quadratic: i-planes one after the other, not unrolled (bounds the
-            // live range of the 9-node plane bodies, which spill in FP64, and
-            // the code size, whose instruction-cache misses stalled the FP32
-            // kernel: 6.55 -> 5.50 ms at 128^3 8 ppc)
-#pragma unroll(ORDER == 2 ? 1 : K)
-            for (int i = 0; i < K; ++i) {
-                const R wxi = pick<K>(sp[0].w, i), dxi = pick<K>(sp[0].d, i);
-                const int gi = pick<K>(idx[0], i);
-#pragma unroll
-                for (int j = 0; j < K; ++j)
-#pragma unroll
-                    for (int k = 0; k < K; ++k) {
-                        const R wm = mass * wxi * sp[1].w[j] * sp[2].w[k];
-                        const R dist[3] = {dxi, sp[1].d[j], sp[2].d[k]};
-                        // backtracked distance xi = A^-1 d (PolyPIC.hpp:90-106)
-                        R map[3];
-#pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            R t = R(0);
-#pragma unroll
-                            for (int v = 0; v < 3; ++v) t += ai[3 * q + v] * dist[v];
-                            map[q] = t;
-                        }
-                        R f[3][D];
-#pragma unroll
-                        for (int q = 0; q < 3; ++q)
-#pragma unroll
-                            for (int g = 0; g < D; ++g)
-                                f[q][g] = (ORDER == 1) ? (g == 0 ? R(1) : map[q])
-                                                       : mode1d(g, map[q], h[q], alpha[q]);
-#pragma unroll
-                        for (int e = 0; e < CB; ++e) {
-                            R sa = R(0);
-#pragma unroll
-                            for (int a = 0; a < D; ++a) {
-                                R sb = R(0);
-#pragma unroll
-                                for (int b = 0; b < D; ++b) {
-                                    R sc = R(0);
-#pragma unroll
-                                    for (int cc = 0; cc < D; ++cc) sc += f[2][cc] * cp[a][b][cc][e];
-                                    sb += f[1][b] * sc;
-                                }
-                                sa += f[0][a] * sb;
-                            }
-                            acc(1 + d0 + e, gi, idx[1][j], idx[2][k], wm * sa);
-                        }
-                        if (d0 == 0) acc(0, gi, idx[1][j], idx[2][k], wm);
-                    }
-            }
+    for (int q = 0; q < N / W; ++q) {
+        if constexpr (sizeof(R) == 4) {
+            const float4 w = reinterpret_cast<const float4*>(p)[q];
+            v[4 * q] = w.x, v[4 * q + 1] = w.y, v[4 * q + 2] = w.z, v[4 * q + 3] = w.w;
+        } else {
+            const double2 w = reinterpret_cast<const double2*>(p)[q];
+            v[2 * q] = w.x, v[2 * q + 1] = w.y;
         }
     }
+}
+
+// NC: components of u_p and c_p; STAG: a staggered location, column col of a
+// 3-component field (col >= 0, PolyPIC.hpp:181) transferred.  PT: particle storage;
+// R: arithmetic; FIXED: 64-bit fixed-point grids (else FP64).
+constexpr int kPPWarps = 4;
+
+template <int ORDER, int NC, bool STAG, class PT, class R, bool FIXED>
+__global__ void __launch_bounds__(32 * kPPWarps, sizeof(R) == 8 ? 2 : 3)
+polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField m, PField u, PField c,
+                   GField gmu, GField gm, R dt, int col, R scale_mu, R scale_m, int* err)
+{
+    constexpr int NCU = STAG ? 1 : NC;
+    using C = PPStreams<ORDER, NCU, R>;
+    using A = typename std::conditional<FIXED, unsigned long long, double>::type;
+    constexpr int K = C::K, KK = C::KK, D = C::D, S = C::S, B = C::B, NF = 1 + NCU;
+    extern __shared__ __align__(16) unsigned char pp_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    R* cs = reinterpret_cast<R*>(pp_smem + warp * C::kBytes);
+    R* table = cs + 2 * C::CHUNK;
+    int4* meta = reinterpret_cast<int4*>(table + C::P * C::ENTRY);
+    const int64_t a = ((int64_t)blockIdx.x * kPPWarps + warp) * seg;
+    if (a >= n) return;
+    const int64_t b = min(a + seg, n);
+    const int len = (int)(b - a), U = (len + S - 1) / S;  // particles, per stream
+    const int ncp = STAG ? (col >= 0 ? NC : 1) : NC;
+
+    // the lane as evaluator: slot es of stream eg
+    const int eg = lane / B, es = lane - eg * B;
+    const int64_t p_first = a + (int64_t)eg * U;
+    const int ecnt = eg < S ? (int)max((int64_t)0, min(p_first + U, b) - p_first) : 0;
+    // the lane as k-row (ri, rj) of stream g
+    const bool act = lane < S * KK;
+    const int g = act ? lane / KK : 0, row = act ? lane - g * KK : 0;
+    const int ri = row / K, rj = row - ri * K;
+
+    // where the lane's values of a particle's record go among the coefficients by
+    // degree (bytes)
+    constexpr int NVAL = D * D * D * NCU, VPL = (NVAL + 31) / 32;
+    unsigned to[VPL];
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+        const int e = lane + 32 * v, r = e / NCU, comp = e - r * NCU;
+        to[v] = (unsigned)sizeof(R) *
+                (mode_deg(r, 0) * C::AB + (mode_deg(r, 1) * D + mode_deg(r, 2)) * NCU + comp);
+    }
+    const bool packed = !STAG && c.shift == 0 && c.tile_stride == NVAL && c.comp_stride == 1;
+
+    int lim[3], off[3];  // wrap of a stencil index: [0, lim) then + off
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        lim[d] = mp.periodic[d] ? mp.own_n[d] : 0x7FFFFFFF;
+        off[d] = mp.periodic[d] ? mp.own_lo[d] : 0;
+    }
+    A acc[NF][K];
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+        for (int k = 0; k < K; ++k) acc[f][k] = A(0);
+    int cur[3] = {-1, -1, -1};  // stencil start of the sums
+    // the sums of the first `count` nodes of the lane's row to the grid
+    auto add_nodes = [&](int count) {
+        const bool inside = cur[0] + K <= lim[0] && cur[1] + K <= lim[1] && cur[2] + K <= lim[2];
+        int q[3] = {cur[0] + ri, cur[1] + rj, cur[2]};
+        if (!inside) {
+#pragma unroll
+            for (int d = 0; d < 2; ++d)
+                while (q[d] >= lim[d]) q[d] -= lim[d];
+        }
+        A* pm = gm.ptr<A>(q[0] + off[0], q[1] + off[1], off[2], 0);
+        A* pmu = gmu.ptr<A>(q[0] + off[0], q[1] + off[1], off[2], 0);
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            if (k >= count) break;
+            int qk = q[2] + k;
+            while (qk >= lim[2]) qk -= lim[2];
+            atomicAdd(pm + (int64_t)qk * gm.s[2], acc[0][k]);
+#pragma unroll
+            for (int f = 1; f < NF; ++f)
+                atomicAdd(pmu + (int64_t)qk * gmu.s[2] + (f - 1) * gmu.s[3], acc[f][k]);
+        }
+    };
+    bool in_range = true;  // of fixed point, the step's contributions
+    auto add_to = [&](A& sum, R q) {  // q: scaled to the fixed point
+        if constexpr (FIXED) {
+            if constexpr (sizeof(R) == 4) {
+                in_range = in_range && fabsf(q) < kFixedLimitF;
+                sum += (unsigned long long)__float2ll_rn(q);
+            } else {
+                in_range = in_range && fabs(q) < kFixedLimitD;
+                sum += (unsigned long long)__double2ll_rn(q);
+            }
+        } else {
+            sum += q;
+        }
+    };
+
+    // Copies of the mode coefficients of chunk `ci` (particles ci H .. of every
+    // stream) into its buffer, by degree.
+    auto fetch = [&](int ci) {
+        const int s0 = ci * C::H;
+        R* buf = cs + (ci & 1) * C::CHUNK;
+        unsigned dst = smem_addr(buf);
+        const int here = min(C::H, U - s0);
+        auto copy = [](unsigned at, const PT* from) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(at), "l"(from),
+                         "n"(sizeof(R)));
+        };
+        if (packed) {  // a record's values are consecutive, as are the records
+            const PT* src = reinterpret_cast<const PT*>(c.data) + (a + s0) * NVAL + lane;
+            int left = len - s0;  // particles from the stream's next one on
+#pragma unroll 1
+            for (int q = 0; q < S; ++q, left -= U, src += (int64_t)U * NVAL,
+                     dst += (unsigned)sizeof(R) * C::H * C::CN) {
+#pragma unroll
+                for (int pl = 0; pl < C::H; ++pl) {
+                    if (pl >= here || pl >= left) break;
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v)
+                        if (lane + 32 * v < NVAL)
+                            copy(dst + (unsigned)sizeof(R) * pl * C::CN + to[v],
+                                 src + pl * NVAL + 32 * v);
+                }
+            }
+        } else {
+#pragma unroll 1
+            for (int q = 0; q < S; ++q) {
+                const int64_t first = a + (int64_t)q * U + s0;
+#pragma unroll 1
+                for (int pl = 0; pl < here && first + pl < b; ++pl) {
+                    const PT* src = reinterpret_cast<const PT*>(c.data) + c.index(first + pl, 0);
+#pragma unroll
+                    for (int v = 0; v < VPL; ++v) {
+                        const int e = lane + 32 * v, r = e / NCU, comp = e - r * NCU;
+                        if (e < NVAL)
+                            copy(dst + (unsigned)sizeof(R) * (q * C::H + pl) * C::CN + to[v],
+                                 src + (int64_t)(r * ncp + (STAG ? max(col, 0) : comp)) * c.comp_stride);
+                    }
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;\n");
+    };
+    static_assert(sizeof(PT) == sizeof(R), "copied as they are");
+
+    fetch(0);
+    for (int s0 = 0; s0 < U; s0 += B) {
+        // (the table's readers have passed the syncwarp after their last chunk)
+        if (s0 + B + es < ecnt) {  // the next table's particles, into L2
+            asm volatile("prefetch.global.L2 [%0];\n" ::"l"(reinterpret_cast<const double*>(x.data) +
+                                                            x.index(p_first + s0 + B + es, 0)));
+        }
+        if (lane < C::P) {
+            int4 at = make_int4(-1, -1, -1, 0);
+            R* e = table + lane * C::ENTRY;
+            if (s0 + es < ecnt) {
+                const int64_t p = p_first + s0 + es;
+                Spline1D<ORDER, R> sp[3];
+                int st[3];
+                bool ok = true;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    eval_spline<ORDER>(x.get<double>(p, d), mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
+                    ok = stencil_start<K>(mp, d, sp[d].s0, st[d]) && ok;
+                }
+                int64_t t_lo = 0, t_hi = n;  // particles sorted into its tile
+                if (tp.off && ok) {
+                    int64_t t = 0;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const int bin = bin_of(mp, tp, d, sp[d].s0);
+                        t = t * tp.nt[d] + (tp.tsh[d] >= 0 ? bin >> tp.tsh[d] : bin / tp.T[d]);
+                    }
+                    t_lo = __ldg(tp.off + t);
+                    t_hi = __ldg(tp.off + t + 1);
+                }
+                if (ok) {
+                    const R mass = (R)m.get<PT>(p, 0);
+                    // affine material motion operator and its inverse
+                    // (PolyPIC.hpp:81-87)
+                    R am[9], ai[9];
+#pragma unroll
+                    for (int q = 0; q < 3; ++q)
+#pragma unroll
+                        for (int r = 0; r < 3; ++r) {
+                            const R v = dt * (R)u.get<PT>(p, (1 + q) * 3 + r);
+                            am[3 * q + r] = (q == r) ? R(1) + v : v;
+                        }
+                    inverse3(am, ai);
+#pragma unroll
+                    for (int q = 0; q < 9; ++q) e[q] = ai[q];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+                        e[C::E_ALPHA + d] = ORDER == 2 ? quad_alpha(-sp[d].d[1], (R)mp.dx[d]) : R(0);
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        e[C::E_DZ + k] = sp[2].d[k];
+                        e[C::E_WZ + k] = sp[2].w[k];
+                        e[C::E_DX + k] = sp[0].d[k];
+                        e[C::E_DY + k] = sp[1].d[k];
+                    }
+#pragma unroll
+                    for (int i = 0; i < K; ++i)
+#pragma unroll
+                        for (int j = 0; j < K; ++j)
+                            e[C::E_W + i * K + j] = mass * sp[0].w[i] * sp[1].w[j];
+                }
+                if (ok && p >= t_lo && p < t_hi) at = make_int4(st[0], st[1], st[2], 0);
+                else if (err) atomicAdd(err, 1);
+            }
+            if (at.x < 0) {  // adds nothing, moves nothing
+#pragma unroll
+                for (int q = 0; q < C::ENTRY; ++q) e[q] = R(0);
+            }
+            meta[lane] = at;
+        }
+        for (int h = 0; h < B / C::H && s0 + h * C::H < U; ++h) {
+        const int ci = s0 / C::H + h;
+        fetch(ci + 1);
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this chunk has landed
+        __syncwarp();  // ... for every lane, and the table is written
+        const int steps = min(C::H, U - (s0 + h * C::H));
+        const R* chunk = cs + (ci & 1) * C::CHUNK + g * C::H * C::CN;
+#pragma unroll 1
+        for (int q = 0; q < steps; ++q) {
+            const int slot = g * B + h * C::H + q;
+            int4 at = meta[slot];
+            if (!act) at.x = -1;
+            const bool live = at.x >= 0;
+            const bool same2 = at.x == cur[0] && at.y == cur[1];
+            if (live && !(same2 && at.z == cur[2])) {
+                const bool step = same2 && at.z == cur[2] + 1;
+                if (cur[0] >= 0) {
+                    add_nodes(step ? 1 : K);
+#pragma unroll
+                    for (int f = 0; f < NF; ++f)
+#pragma unroll
+                        for (int k = 0; k < K; ++k)
+                            acc[f][k] = step && k + 1 < K ? acc[f][k + 1 < K ? k + 1 : k] : A(0);
+                }
+                cur[0] = at.x;
+                cur[1] = at.y;
+                cur[2] = at.z;
+            }
+            __syncwarp();
+            if (!live) continue;
+            const R* e = table + slot * C::ENTRY;
+            R ia[12], dz[4], wz[4];  // A^-1 and alpha, d_z, w_z
+            read_shared(e, ia);
+            read_shared(e + C::E_DZ, dz);
+            read_shared(e + C::E_WZ, wz);
+            const R di = e[C::E_DX + ri], dj = e[C::E_DY + rj], wab = e[C::E_W + row];
+            // modes of the row's nodes (f[.][.][0] is 1): xi = A^-1 d (the
+            // backtracked distance, PolyPIC.hpp:90-106), and for degree 2
+            // xi^2 - h^2/4 - alpha xi
+            R f1[3][K], f2[3][K];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const R base = fma(ia[3 * d + 1], dj, ia[3 * d] * di);
+                const R h2 = R(0.25) * (R)mp.dx[d] * (R)mp.dx[d];
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    f1[d][k] = fma(ia[3 * d + 2], dz[k], base);
+                    f2[d][k] = ORDER == 2 ? fma(f1[d][k], f1[d][k] - ia[C::E_ALPHA + d], -h2) : R(0);
+                }
+            }
+            // sum_a f0_a sum_b f1_b sum_c f2_c c_abc of every component and node
+            R sa[NCU][K];
+            const R* cp = chunk + q * C::CN;
+#pragma unroll
+            for (int da = 0; da < D; ++da) {
+                R cc[C::AB];
+                read_shared(cp + da * C::AB, cc);
+#pragma unroll
+                for (int n_ = 0; n_ < NCU; ++n_)
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        R sb = R(0);
+#pragma unroll
+                        for (int db = 0; db < D; ++db) {
+                            R sc = fma(f1[2][k], cc[(db * D + 1) * NCU + n_], cc[db * D * NCU + n_]);
+                            if (ORDER == 2) sc = fma(f2[2][k], cc[(db * D + D - 1) * NCU + n_], sc);
+                            sb = db == 0 ? sc : fma(db == 1 ? f1[1][k] : f2[1][k], sc, sb);
+                        }
+                        sa[n_][k] = da == 0 ? sb : fma(da == 1 ? f1[0][k] : f2[0][k], sb, sa[n_][k]);
+                    }
+            }
+            // (the scales are powers of two: the weights take them exactly)
+            const R wm = FIXED ? wab * scale_m : wab, wmu = FIXED ? wab * scale_mu : wab;
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const R w = wmu * wz[k];
+                add_to(acc[0][k], wm * wz[k]);
+#pragma unroll
+                for (int n_ = 0; n_ < NCU; ++n_) add_to(acc[1 + n_][k], w * sa[n_][k]);
+            }
+            if (FIXED && !in_range) {  // count the contributions out of range
+                in_range = true;
+                if (gm.overflow) {
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        to_fixed(gm, wm * wz[k]);
+#pragma unroll
+                        for (int n_ = 0; n_ < NCU; ++n_) to_fixed(gmu, wmu * wz[k] * sa[n_][k]);
+                    }
+                }
+            }
+        }
+        __syncwarp();  // the chunk's buffer may be refilled
+        }
+    }
+    asm volatile("cp.async.wait_group 0;\n");
+    if (act && cur[0] >= 0) add_nodes(K);
 }
 
 // Modes per particle record (c_p rows): 8 linear, 27 quadratic.
@@ -228,31 +469,32 @@ struct WarpRecords {
     }
 };
 
-template <int ORDER, int NC, bool STAG, class PT, class R, class ACC>
-__global__ void __launch_bounds__(128)
-polypic_p2g_kernel(MeshP mp, int64_t n, PField x, PField m, PField u, PField c, GField gmu,
-                   GField gm, R dt, int col, R scale_mu, R scale_m, int* err)
-{
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const MeshPlace<ORDER, R> place{mp};
-    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
-        polypic_p2g_particle<ORDER, NC, STAG, PT, R>(
-            mp, p, x, m, u, dt, col, err, place,
-            [&](int f, int i, int j, int k, R v) {
-                if (f == 0) ACC::add(gm, i, j, k, 0, v, scale_m);
-                else ACC::add(gmu, i, j, k, f - 1, v, scale_mu);
-            },
-            [&](int v) { return c.get<PT>(p, v); });
-}
-
 // ---------------------------------------------------------------------------
 // G2P: PolyPIC.hpp:236-293 (collocated) and :300-358 (staggered)
 // ---------------------------------------------------------------------------
+// Spline and stencil indices of a particle on the whole local mesh (periodic
+// wrap, bounds check): the placement of the plain kernels.
+template <int ORDER, class R>
+struct MeshPlace {
+    const MeshP& mp;
+    __device__ __forceinline__ bool operator()(const double xp[3], Spline1D<ORDER, R> sp[3],
+                                               int idx[3][SplineTraits<ORDER>::K]) const
+    {
+        bool ok = true;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            eval_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
+            ok = ok && resolve_stencil<SplineTraits<ORDER>::K>(mp, d, sp[d].s0, idx[d]);
+        }
+        return ok;
+    }
+};
+
 // One particle; emit(v, value) receives c_p value v (element v of the
 // particle's record).  False if the particle was skipped (stencil outside a
 // non-periodic mesh): then nothing is emitted.
-// place: as for polypic_p2g_particle; grid(i, j, k, c) returns component c
-// of u at stencil indices (i, j, k).
+// place(x, splines, indices) locates the particle; grid(i, j, k, c) returns
+// component c of u at stencil indices (i, j, k).
 template <int ORDER, int NC, bool STAG, class PT, class R, class Place, class Grid, class Emit>
 __device__ __forceinline__ bool polypic_g2p_particle(const MeshP& mp, int64_t p, const PField& x,
                                                      int col, int* err, Place&& place,
@@ -434,91 +676,6 @@ __device__ __forceinline__ void count_unsorted(const TileP& tp, int64_t n, int* 
     }
 }
 
-// P2G: the item's contributions are rounded to 64-bit fixed point exactly as
-// the plain kernel rounds them and summed in a shared-memory node tile with
-// 32-bit integer atomics, either on three slices of each value (q = hi 2^32 +
-// mid 2^16 + lo with mid, lo in [0, 2^16): the lo and mid sums of at most
-// 65536 contributions are exact, the hi sum is exact modulo 2^32) or on two
-// words (the low word's carries, read from the atomics' old values, added to
-// the high word), so the recombined 64-bit total equals the sum of the q
-// modulo 2^64; then the tile is added to the grid.  Integer sums do not
-// depend on their order: the grid is bit-identical to the plain kernel's
-// (which adds every contribution to the grid), with one grid atomic per
-// touched node and field per item instead of per particle and node.
-// Quadratic: 3 CTAs per SM (168 registers, 44 bytes of spills) instead of 2 at
-// 255 registers: 27 modes at 128^3 8 ppc 6.24 -> 5.85 ms.
-template <int ORDER, int NC>
-__global__ void __launch_bounds__(128, ORDER == 2 ? 3 : 1)
-polypic_p2g_tiled_kernel(MeshP mp, TileP tp, int64_t n, PField x, PField m, PField u, PField c,
-                         GField gmu, GField gm, float dt, float scale_mu, float scale_m, int* err)
-{
-    extern __shared__ __align__(16) unsigned int pp_tacc[];  // 3 slices x (1 + NC) x nodes
-    count_unsorted(tp, n, err);
-    int64_t t, a, b;
-    if (!item_range(tp, blockIdx.x, t, a, b)) return;  // CTA-uniform
-    // linear stencils (consecutive particles per warp): two words per value,
-    // the low word's carry found from the atomic's old value and added to
-    // the high word (2.11 -> 1.52 ms at 128^3 8 ppc); quadratic stencils (a
-    // run per thread): three slices without returned values (the returning
-    // atomic measured 6.20 -> 7.27 ms there)
-    constexpr bool TWO = ORDER == 1;
-    const int nodes = tp.nodes, slice = (1 + NC) * nodes;
-    for (int e = threadIdx.x; e < (TWO ? 2 : 3) * slice; e += blockDim.x) pp_tacc[e] = 0u;
-    __syncthreads();
-    int ob[3];
-    tile_origin(tp, t, ob);
-    const TilePlace<ORDER> place{mp, tp, ob};
-    // Quadratic: each thread sweeps its own contiguous run of the item, so
-    // that the lanes of a warp sit in different cells and their tile atomics
-    // rarely hit the same node (128^3 8 ppc: 6.5 ms instead of 9.1 ms with
-    // consecutive particles per warp).  Linear (8 nodes, little arithmetic)
-    // keeps consecutive particles per warp for coalesced loads (2.1 vs 2.5 ms).
-    const int64_t U = ORDER == 2 ? (b - a + blockDim.x - 1) / blockDim.x : 1;
-    const int64_t r0 = ORDER == 2 ? a + (int64_t)threadIdx.x * U : a + threadIdx.x;
-    const int64_t r1 = ORDER == 2 ? min(r0 + U, b) : b;
-    const int64_t step = ORDER == 2 ? 1 : blockDim.x;
-    for (int64_t p = r0; p < r1; p += step)
-        polypic_p2g_particle<ORDER, NC, false, float, float>(
-            mp, p, x, m, u, dt, -1, err, place,
-            [&](int f, int i, int j, int k, float v) {
-                const long long q = to_fixed(f == 0 ? gm : gmu, v * (f == 0 ? scale_m : scale_mu));
-                const int e = f * nodes + (i * tp.NT[1] + j) * tp.NT[2] + k;
-                if constexpr (TWO) {
-                    const unsigned long long uq = (unsigned long long)q;
-                    const unsigned lo = (unsigned)uq;
-                    const unsigned old = atomicAdd(&pp_tacc[e], lo);
-                    const unsigned hi = (unsigned)(uq >> 32) + (old + lo < old ? 1u : 0u);
-                    if (hi) atomicAdd(&pp_tacc[slice + e], hi);
-                } else {
-                    atomicAdd(&pp_tacc[e], (unsigned int)(q & 0xFFFF));
-                    atomicAdd(&pp_tacc[slice + e], (unsigned int)((q >> 16) & 0xFFFF));
-                    atomicAdd(&pp_tacc[2 * slice + e], (unsigned int)(q >> 32));
-                }
-            },
-            [&](int v) { return c.get<float>(p, v); });
-    __syncthreads();
-    for (int e = threadIdx.x; e < nodes; e += blockDim.x) {
-        const int k = e % tp.NT[2], j = (e / tp.NT[2]) % tp.NT[1], i = e / (tp.NT[1] * tp.NT[2]);
-        const int gi = node_global(mp, tp, 0, ob[0], i);
-        const int gj = node_global(mp, tp, 1, ob[1], j);
-        const int gk = node_global(mp, tp, 2, ob[2], k);
-#pragma unroll
-        for (int f = 0; f <= NC; ++f) {
-            const int q = f * nodes + e;
-            const unsigned long long v =
-                TWO ? ((unsigned long long)pp_tacc[slice + q] << 32) + (unsigned long long)pp_tacc[q]
-                    : ((unsigned long long)pp_tacc[2 * slice + q] << 32) +
-                          ((unsigned long long)pp_tacc[slice + q] << 16) +
-                          (unsigned long long)pp_tacc[q];
-            if (v)
-                atomicAdd(reinterpret_cast<unsigned long long*>(
-                              f == 0 ? gm.ptr<long long>(gi, gj, gk, 0)
-                                     : gmu.ptr<long long>(gi, gj, gk, f - 1)),
-                          v);
-        }
-    }
-}
-
 // G2P: the tile's node velocities are staged once per item in shared memory;
 // packed c_p records leave through WarpRecords.
 template <int ORDER, int NC, bool WS>
@@ -578,22 +735,6 @@ polypic_g2p_tiled_kernel(MeshP mp, TileP tp, int64_t n, PField x, GField u, PFie
 }
 
 template <int ORDER, int NC>
-static picasso_status launch_pp_p2g_tiled(const MeshP& mp, const TileP& tp, int64_t n,
-                                          const PField& x, const PField& m, const PField& u,
-                                          const PField& c, const GField& gmu, const GField& gm,
-                                          double dt, int* err, cudaStream_t st)
-{
-    const size_t smem = 3 * sizeof(unsigned int) * (1 + NC) * (size_t)tp.nodes;
-    auto kern = polypic_p2g_tiled_kernel<ORDER, NC>;
-    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    const int64_t items = item_bound(tp, n);
-    kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, m, u, c, gmu, gm, (float)dt,
-                                             ldexpf(1.f, gmu.fixed_bits), ldexpf(1.f, gm.fixed_bits),
-                                             err);
-    return check_launch();
-}
-
-template <int ORDER, int NC>
 static picasso_status launch_pp_g2p_tiled(const MeshP& mp, const TileP& tp, int64_t n,
                                           const PField& x, const GField& u, const PField& c,
                                           int* err, cudaStream_t st)
@@ -628,33 +769,44 @@ static void launch_staged(Kern kernel, bool ws, unsigned blocks, cudaStream_t st
     kernel<<<blocks, 128, smem, st>>>(args...);
 }
 
-template <int ORDER, int NC, bool STAG, class PT, class R, class ACC>
-static void launch_pp_p2g_form(const MeshP& mp, int64_t n, const PField& x, const PField& m,
-                               const PField& u, const PField& c, const GField& gmu,
-                               const GField& gm, R dt, int col, R smu, R sm, int* err,
-                               cudaStream_t st)
+// Particles per warp: up to 8 tables (a run's end at a segment's costs as much as
+// a stencil), less when that would not give every SM 16 warps.
+template <int ORDER, int NC, bool STAG, class PT, class R, bool FIXED>
+static picasso_status launch_pp_p2g_form(const MeshP& mp, const TileP& tp, int64_t n, const PField& x,
+                                         const PField& m, const PField& u, const PField& c,
+                                         const GField& gmu, const GField& gm, R dt, int col, R smu,
+                                         R sm, int* err, cudaStream_t st)
 {
-    const unsigned blocks = grid_for(n, 128, 148LL * 128);
-    polypic_p2g_kernel<ORDER, NC, STAG, PT, R, ACC><<<blocks, 128, 0, st>>>(
-        mp, n, x, m, u, c, gmu, gm, dt, col, smu, sm, err);
+    using C = PPStreams<ORDER, STAG ? 1 : NC, R>;
+    auto kern = polypic_p2g_kernel<ORDER, NC, STAG, PT, R, FIXED>;
+    const size_t smem = kPPWarps * C::kBytes;
+    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int64_t tables = n / (148 * 16) / C::P;
+    if (tables < 1) tables = 1;
+    if (tables > 8) tables = 8;
+    const int64_t seg = tables * C::P;
+    const int64_t ctas = (n + seg * kPPWarps - 1) / (seg * kPPWarps);
+    kern<<<(unsigned)ctas, 32 * kPPWarps, smem, st>>>(mp, tp, n, seg, x, m, u, c, gmu, gm, dt, col, smu, sm,
+                                                      err);
+    return check_launch();
 }
 
 template <int ORDER, int NC, bool STAG>
-static void launch_pp_p2g(int form, const MeshP& mp, int64_t n, const PField& x, const PField& m,
-                          const PField& u, const PField& c, const GField& gmu, const GField& gm,
-                          double dt, int col, int* err, cudaStream_t st)
+static picasso_status launch_pp_p2g(int form, const MeshP& mp, const TileP& tp, int64_t n, const PField& x,
+                                    const PField& m, const PField& u, const PField& c,
+                                    const GField& gmu, const GField& gm, double dt, int col, int* err,
+                                    cudaStream_t st)
 {
     if (form == 0)
-        launch_pp_p2g_form<ORDER, NC, STAG, double, double, AccF64>(
-            mp, n, x, m, u, c, gmu, gm, dt, col, 0.0, 0.0, err, st);
-    else if (form == 1)
-        launch_pp_p2g_form<ORDER, NC, STAG, float, float, AccFixed>(
-            mp, n, x, m, u, c, gmu, gm, (float)dt, col, ldexpf(1.0f, gmu.fixed_bits),
+        return launch_pp_p2g_form<ORDER, NC, STAG, double, double, false>(
+            mp, tp, n, x, m, u, c, gmu, gm, dt, col, 0.0, 0.0, err, st);
+    if (form == 1)
+        return launch_pp_p2g_form<ORDER, NC, STAG, float, float, true>(
+            mp, tp, n, x, m, u, c, gmu, gm, (float)dt, col, ldexpf(1.0f, gmu.fixed_bits),
             ldexpf(1.0f, gm.fixed_bits), err, st);
-    else
-        launch_pp_p2g_form<ORDER, NC, STAG, double, double, AccFixed>(
-            mp, n, x, m, u, c, gmu, gm, dt, col, ldexp(1.0, gmu.fixed_bits),
-            ldexp(1.0, gm.fixed_bits), err, st);
+    return launch_pp_p2g_form<ORDER, NC, STAG, double, double, true>(
+        mp, tp, n, x, m, u, c, gmu, gm, dt, col, ldexp(1.0, gmu.fixed_bits), ldexp(1.0, gm.fixed_bits),
+        err, st);
 }
 
 template <int ORDER, int NC, bool STAG, class T>
@@ -757,32 +909,21 @@ extern "C" picasso_status picasso_polypic_p2g(const picasso_spline* sd, int64_t 
     gmu.overflow = gm.overflow = exec ? exec->overflow_count : nullptr;
     bool tiled = false;
     TileP tp;
-    // (the tile's 32-bit slice sums are exact for work items of at most
-    // 65536 particles)
     const bool p2g_ok = form == 1 && stag < 0 && exec && exec->bins && exec->bins->chunk <= 65536;
     if ((st = polypic_tiles(sd, exec, num_particles, p2g_ok, mp, 12 * (1 + ncomp), &tiled, &tp))) return st;
-    if (tiled) {
-        if (sd->order == 1) {
-            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g_tiled<1, NC_>(mp, tp, num_particles, x, m,
-                                                                      u, c, gmu, gm, dt, err, s));
-        } else {
-            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g_tiled<2, NC_>(mp, tp, num_particles, x, m,
-                                                                      u, c, gmu, gm, dt, err, s));
-        }
-    }
+    if (!tiled) tp.off = nullptr;
     if (sd->order == 1) {
         if (stag >= 0) {
-            PB_PP_NC_SWITCH(ncomp, launch_pp_p2g<1, NC_, true>(form, mp, num_particles, x, m, u, c,
-                                                                gmu, gm, dt, col, err, s));
+            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, true>(
+                                       form, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
         } else {
-            PB_PP_NC_SWITCH(ncomp, launch_pp_p2g<1, NC_, false>(form, mp, num_particles, x, m, u, c,
-                                                                 gmu, gm, dt, col, err, s));
+            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, false>(
+                                       form, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
         }
-    } else {
-        PB_PP_NC_SWITCH(ncomp, launch_pp_p2g<2, NC_, false>(form, mp, num_particles, x, m, u, c,
-                                                             gmu, gm, dt, col, err, s));
     }
-    return check_launch();
+    PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<2, NC_, false>(form, mp, tp, num_particles, x, m, u, c,
+                                                               gmu, gm, dt, col, err, s));
+    return PICASSO_OK;
 }
 
 extern "C" picasso_status picasso_polypic_g2p(const picasso_spline* sd, int64_t num_particles,
