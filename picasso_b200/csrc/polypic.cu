@@ -80,7 +80,7 @@ __device__ __forceinline__ void inverse3(const R a[9], R inv[9])
 // linear, the instructions around the few FMAs: 83 per particle, a third of them for
 // the table, the copies and the moved stencils.  Against one thread per particle
 // with a shared integer tile (FP32) or grid atomics per node (FP64), cell-sorted
-// particles: quadratic FP32 96^3 cells 5 per cell 2.50 -> 1.89 ms, FP64 48^3 0.73 ->
+// particles: quadratic FP32 96^3 cells 8 per cell 2.50 -> 1.89 ms, FP64 48^3 0.73 ->
 // 0.44 ms, linear FP32 101 x 67 x 83 0.278 -> 0.276 ms.  Quadratic warps hold 10
 // (FP64: 6) particles per stream in the table and half of them in each of the two
 // coefficient chunks; other splits of the shared memory between table and chunks

@@ -875,8 +875,47 @@ __global__ void zero_untouched_regions_kernel(MeshP mp, TileP tp, FusedUpdate F)
 // ---------------------------------------------------------------------------
 // G2P
 // ---------------------------------------------------------------------------
+// Term n of the sum of w_n v_n: the first one sets it.
+__device__ __forceinline__ float add_term(int n, float w, float v, float sum)
+{
+    return n == 0 ? __fmul_rn(w, v) : fmaf(w, v, sum);
+}
+
+// Term n of S0 = sum w_n v_n and S1 = sum (n - n0) w_n v_n, n0 the stencil's centre
+// knot (0 linear, else 1), in the fewest instructions: 2 (linear), 4 (quadratic)
+// and 6 (cubic) for all terms.
+template <int ORDER>
+__device__ __forceinline__ void add_moments(int n, float w, float v, float& S0, float& S1)
+{
+    if constexpr (ORDER == 1) {
+        if (n == 0) {
+            S0 = __fmul_rn(w, v);
+        } else {
+            S1 = __fmul_rn(w, v);
+            S0 = __fadd_rn(S0, S1);
+        }
+    } else {
+        if (n == 0) {
+            S0 = __fmul_rn(w, v);
+            return;
+        }
+        if (n == 2) S1 = fmaf(w, v, -S1);
+        if (n == 1) S1 = S0;  // the first term, to be subtracted
+        if (n == 3) S1 = fmaf(2.f * w, v, S1);
+        S0 = fmaf(w, v, S0);
+    }
+}
+
 // One G2P work item by NTHR threads (a warp or a CTA) sharing `tile`
 // (tp.nodes float4).  Threads are numbered tid in [0, NTHR).
+// Bound by the instructions of the contraction together with its 16-byte reads of
+// shared memory (quadratic, 128^3 cells 8 per cell clustered: 66 % of the issue slots
+// and 73 % of the L1 data pipe of a busy SM, 390 instructions and 78 shared-memory
+// wavefronts per 32 particles; DRAM at 42 %).  Taking the moments in fused
+// multiply-adds (add_moments), walking the rows by one pointer and staging the tile
+// without divisions took 440 instructions to 390: 256^3 2.16 -> 2.06 ms, 128^3 0.326
+// -> 0.301 ms, cubic with advection 128^3 0.66 -> 0.635 ms.  More warps at fewer
+// registers lose more to spills (64 instead of 72: 2.51 ms).
 // ADV: each particle is then moved, x += dt u_p (FP64, as picasso_advect).
 // The positions of the item's first and last particle are read before the
 // tile barrier, so no thread reads a position another thread has moved.
@@ -928,10 +967,10 @@ __device__ void g2p_item(const G2PArgs& A, int64_t t, int64_t a, int64_t b, floa
     const int plane = tp.NT[1] * tp.NT[2];
     const int total = (i_hi - i_lo + K) * plane;
     sync();  // the previous item's threads are done with the tile
+    // node e = tid, tid + NTHR, ...: (i, j, k) by carries, not by divisions
+    const int step_k = NTHR % tp.NT[2], step_j = NTHR / tp.NT[2] % tp.NT[1], step_i = NTHR / plane;
+    int k = tid % tp.NT[2], j = tid / tp.NT[2] % tp.NT[1], i = i_lo + tid / plane;
     for (int e = tid; e < total; e += NTHR) {
-        const int k = e % tp.NT[2];
-        const int j = (e / tp.NT[2]) % tp.NT[1];
-        const int i = i_lo + e / plane;
         const int gi = node_global(mp, tp, 0, ob[0], i);
         const int gj = node_global(mp, tp, 1, ob[1], j);
         const int gk = node_global(mp, tp, 2, ob[2], k);
@@ -949,7 +988,18 @@ __device__ void g2p_item(const G2PArgs& A, int64_t t, int64_t a, int64_t b, floa
                 v.z = __ldcg(ub + A.u.index(gx, gj, gk, 2));
             }
         }
-        tile[(i * tp.NT[1] + j) * tp.NT[2] + k] = v;
+        tile[i_lo * plane + e] = v;
+        k += step_k;
+        j += step_j;
+        i += step_i;
+        if (k >= tp.NT[2]) {
+            k -= tp.NT[2];
+            ++j;
+        }
+        if (j >= tp.NT[1]) {
+            j -= tp.NT[1];
+            ++i;
+        }
     }
     sync();
     // positions (records) are prefetched one particle ahead
@@ -996,41 +1046,34 @@ __device__ void g2p_item(const G2PArgs& A, int64_t t, int64_t a, int64_t b, floa
         //   B_p(:,q) = dx M_q + dist_q(n0) u_p
         float up[3] = {0.f, 0.f, 0.f};
         float M[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        const float4* row = tile + base;
 #pragma unroll
         for (int i = 0; i < K; ++i) {
-            float A0[3] = {0.f, 0.f, 0.f}, A1[3] = {0.f, 0.f, 0.f}, A2[3] = {0.f, 0.f, 0.f};
+            float A0[3], A1[3], A2[3];
 #pragma unroll
             for (int j = 0; j < K; ++j) {
-                const float4* row = tile + base + (i * tp.NT[1] + j) * tp.NT[2];
-                float S0[3] = {0.f, 0.f, 0.f}, S1[3] = {0.f, 0.f, 0.f};
+                float S0[3], S1[3];
 #pragma unroll
                 for (int k = 0; k < K; ++k) {
                     const float4 ue = row[k];
                     const float uk[3] = {ue.x, ue.y, ue.z};
 #pragma unroll
                     for (int d = 0; d < NU; ++d) {
-                        const float wu = sp[2].w[k] * uk[d];
-                        S0[d] += wu;
-                        S1[d] = add_steps(k - N0, S1[d], wu);
+                        add_moments<ORDER>(k, sp[2].w[k], uk[d], S0[d], S1[d]);
                     }
                 }
-                const float wy = sp[1].w[j];
 #pragma unroll
                 for (int d = 0; d < NU; ++d) {
-                    const float wS0 = wy * S0[d];
-                    A0[d] += wS0;
-                    A1[d] = add_steps(j - N0, A1[d], wS0);
-                    A2[d] = fmaf(wy, S1[d], A2[d]);
+                    add_moments<ORDER>(j, sp[1].w[j], S0[d], A0[d], A1[d]);
+                    A2[d] = add_term(j, sp[1].w[j], S1[d], A2[d]);
                 }
+                row += j + 1 < K ? tp.NT[2] : plane - (K - 1) * tp.NT[2];
             }
-            const float wx = sp[0].w[i];
 #pragma unroll
             for (int d = 0; d < NU; ++d) {
-                const float wA0 = wx * A0[d];
-                up[d] += wA0;
-                M[d][0] = add_steps(i - N0, M[d][0], wA0);
-                M[d][1] = fmaf(wx, A1[d], M[d][1]);
-                M[d][2] = fmaf(wx, A2[d], M[d][2]);
+                add_moments<ORDER>(i, sp[0].w[i], A0[d], up[d], M[d][0]);
+                M[d][1] = add_term(i, sp[0].w[i], A1[d], M[d][1]);
+                M[d][2] = add_term(i, sp[0].w[i], A2[d], M[d][2]);
             }
         }
         float B[3][3];
