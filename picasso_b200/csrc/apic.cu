@@ -185,7 +185,7 @@ static picasso_status launch_g2p_tiled_f64(const MeshP& mp, const TileP& tp, int
     const bool packed = packed_rows_f64(x, c, 12, adv != nullptr);
     const int64_t items = item_bound(tp, n);
     auto launch = [&](auto kern) -> picasso_status {
-        PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_CUDA_TRY(allow_smem(kern, smem));
         kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, u, c, err, adv ? *adv : Advect{}, packed);
         return check_launch();
     };

@@ -746,11 +746,11 @@ static picasso_status launch_pp_g2p_tiled(const MeshP& mp, const TileP& tp, int6
     const int64_t items = item_bound(tp, n);
     if (ws) {
         auto kern = polypic_g2p_tiled_kernel<ORDER, NC, true>;
-        PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_CUDA_TRY(allow_smem(kern, smem));
         kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, u, c, err);
     } else {
         auto kern = polypic_g2p_tiled_kernel<ORDER, NC, false>;
-        PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_CUDA_TRY(allow_smem(kern, smem));
         kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, u, c, err);
     }
     return check_launch();
@@ -765,7 +765,7 @@ template <class PT, int NV, class Kern, class... Args>
 static void launch_staged(Kern kernel, bool ws, unsigned blocks, cudaStream_t st, Args... args)
 {
     const size_t smem = ws ? 4 * WarpRecords<PT, NV>::kBytesPerWarp : 0;
-    if (ws) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (ws) allow_smem(kernel, smem);
     kernel<<<blocks, 128, smem, st>>>(args...);
 }
 
@@ -780,7 +780,7 @@ static picasso_status launch_pp_p2g_form(const MeshP& mp, const TileP& tp, int64
     using C = PPStreams<ORDER, STAG ? 1 : NC, R>;
     auto kern = polypic_p2g_kernel<ORDER, NC, STAG, PT, R, FIXED>;
     const size_t smem = kPPWarps * C::kBytes;
-    PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_CUDA_TRY(allow_smem(kern, smem));
     int64_t tables = n / (148 * 16) / C::P;
     if (tables < 1) tables = 1;
     if (tables > 8) tables = 8;

@@ -195,7 +195,7 @@ static picasso_status launch_p2g_tiled(const P2GArgs& args, const FusedUpdate* f
     const size_t smem = p2g_warp_bytes(ORDER, A.tp.P, STAG);
     const int64_t items = item_bound(A.tp, n);
     auto launch = [&](auto kern, const FusedUpdate& F) -> picasso_status {
-        PB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PB_CUDA_TRY(allow_smem(kern, smem));
         kern<<<(unsigned)(items ? items : 1), 32, smem, st>>>(A, F, n);
         return check_launch();
     };
@@ -211,8 +211,7 @@ template <int ORDER, bool ADV, bool REC, bool STAG>
 static picasso_status launch_g2p_tiled(const G2PArgs& A, int64_t n, cudaStream_t st)
 {
     const size_t smem = sizeof(float4) * (size_t)A.tp.nodes;
-    PB_CUDA_TRY(cudaFuncSetAttribute(g2p_tiled_kernel<ORDER, ADV, REC, STAG>,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PB_CUDA_TRY(allow_smem(g2p_tiled_kernel<ORDER, ADV, REC, STAG>, smem));
     const int64_t items = item_bound(A.tp, n);
     g2p_tiled_kernel<ORDER, ADV, REC, STAG>
         <<<(unsigned)(items ? items : 1), G2PThreads<ORDER>::value, smem, st>>>(A, n);
