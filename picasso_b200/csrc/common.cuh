@@ -27,12 +27,12 @@ picasso_status check_launch();  // reads cudaGetLastError after a launch
     } while (0)
 
 // Lets a launch of `kernel` have `bytes` of dynamic shared memory.  Up to 48 KB
-// (with the static part, below 8 KB in every kernel here) needs no attribute, whose
-// call costs as much as a small launch's arguments.
+// together with the static part (15 KB at most in the kernels launched this way)
+// needs no attribute, whose call costs as much as a small launch's arguments.
 template <class Kernel>
 inline cudaError_t allow_smem(Kernel kernel, size_t bytes)
 {
-    if (bytes <= 40 * 1024) return cudaSuccess;
+    if (bytes <= 32 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
