@@ -53,6 +53,7 @@ struct BInst {
     double thr, inv_m, inv_mu;
     int64_t n;
     int order;
+    int g2p_tile;  // FP64: the node tile fits in shared memory
     uint32_t nitems[kPhases];
 };
 
@@ -181,8 +182,9 @@ static int warp_p2g_bytes(int order)
     return d * (int)sizeof(double);
 }
 
-// FP64 G2P item (g2p_item_f64); smem: a WarpRows buffer per warp, then the node
-// tile.  CG: u_i was written in this launch.
+// FP64 G2P item; smem: a WarpRows buffer per warp, then the node tile
+// (g2p_item_f64).  An instance whose tile does not fit in shared memory gathers from
+// global memory (apic_g2p_warp).  CG: u_i was written in this launch.
 constexpr int kWarpG2PBytes = WarpRows<3, false>::DOUBLES * (int)sizeof(double);
 
 template <int ORDER, int NT, bool CG>
@@ -191,6 +193,13 @@ __device__ __noinline__ void g2p_f64_call(const BInst& I, int64_t t, int64_t a, 
 {
     double* rows = reinterpret_cast<double*>(smem);
     double* nodes = rows + NT / 32 * WarpRows<3, false>::DOUBLES;
+    if (!I.g2p_tile) {
+        for (int64_t p0 = a + (tid & ~31); p0 < b; p0 += NT)
+            apic_g2p_warp<ORDER, 3, false, CG, false, false, true>(
+                I.g2p.mp, p0, (int)min((int64_t)32, b - p0), I.x, I.gu, I.c, -1, I.g2p.err, nullptr,
+                rows + (tid >> 5) * WarpRows<3, false>::DOUBLES);
+        return;
+    }
     g2p_item_f64<ORDER, NT, CG, false>(I.g2p.mp, I.g2p.tp, t, a, b, I.x, I.gu, I.c, I.g2p.err,
                                        nullptr, nodes, rows, tid);
 }
@@ -460,6 +469,9 @@ picasso_status enqueue_step(const picasso_batch* b, cudaStream_t s)
     return check_launch();
 }
 
+// FP64 CTAs of the phased transfers run several warps, each with its buffer.
+constexpr int kF64Warps = BatchShape<false, 0x2>::threads / 32;
+
 // Validates one instance and fills its device descriptor; raises *smem to
 // the instance's shared-memory need.
 picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* I,
@@ -538,7 +550,9 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
         *smem_g2p = std::max(*smem_g2p, (int)(sizeof(float4) * (size_t)tp.nodes));
     } else {
         *smem_p2g = std::max(*smem_p2g, warp_p2g_bytes(order));  // one warp's
-        *smem_g2p = std::max(*smem_g2p, 3 * (int)sizeof(double) * tp.nodes);  // the tile's
+        const int64_t tile = 3 * (int64_t)sizeof(double) * tp.nodes;
+        I->g2p_tile = tile + kF64Warps * kWarpG2PBytes <= device_smem_optin();
+        if (I->g2p_tile) *smem_g2p = std::max(*smem_g2p, (int)tile);
     }
     return PICASSO_OK;
 }
@@ -560,8 +574,6 @@ extern "C" picasso_status picasso_batch_create(const picasso_batch_instance* ins
         picasso_status st = make_instance(instances[i], f32, &hinst[i], &smem_p2g, &smem_g2p);
         if (st) return st;
     }
-    // FP64 CTAs of the phased transfers run several warps, each with its buffer
-    constexpr int kF64Warps = BatchShape<false, 0x2>::threads / 32;
     const int p2g_bytes = f32 ? smem_p2g : kF64Warps * smem_p2g;
     const int g2p_bytes = f32 ? smem_g2p : kF64Warps * kWarpG2PBytes + smem_g2p;
     const int fused_bytes = std::max(smem_p2g, f32 ? smem_g2p : kWarpG2PBytes + smem_g2p);

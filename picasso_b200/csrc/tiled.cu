@@ -67,7 +67,7 @@ static void choose_strides(const int NT[3], int K, int* SJ, int* SI)
             for (int r0 = 0; r0 < K * K; r0 += 8) {
                 unsigned banks = 0;
                 for (int r = r0; r < r0 + 8 && r < K * K; ++r) banks |= 1u << ((r / K * si + r % K * sj) & 7);
-                for (; banks; banks &= banks - 1) ++distinct;
+                distinct += __builtin_popcount(banks);
             }
             if (distinct > best || (distinct == best && si < size)) {
                 best = distinct;
@@ -131,8 +131,17 @@ bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n,
     tp->nodes = tp->NT[0] * tp->NT[1] * tp->NT[2];
     tp->SJ = tp->NT[2];
     tp->SI = tp->NT[1] * tp->NT[2];
-    if (p2g_strides) choose_strides(tp->NT, K, &tp->SJ, &tp->SI);
-    tp->P = tp->NT[0] * tp->SI;
+    tp->P = tp->nodes;
+    if (p2g_strides) {
+        int sj, si;
+        choose_strides(tp->NT, K, &sj, &si);
+        // (a tile that the padding pushes out of shared memory stays unpadded)
+        if ((int64_t)p2g_warp_bytes(order, tp->NT[0] * si) <= device_smem_optin()) {
+            tp->SJ = sj;
+            tp->SI = si;
+            tp->P = tp->NT[0] * si;
+        }
+    }
     tp->ntiles = nt;
     tp->off = bins.tile_offset;
     tp->items = bins.tile_items;
