@@ -77,11 +77,11 @@ __device__ __forceinline__ void inverse3(const R a[9], R inv[9])
 // read once per lane group and particle: 64 % of the pipe in FP32, 70 % in FP64)
 // next to the FMAs of the sums (about 100 per node with 3 components) and, in fixed
 // point, 16 instructions per node for the four roundings (57 % of the issue slots);
-// linear, the instructions around the few FMAs: 83 per particle, a third of them for
-// the table, the copies and the moved stencils.  Against one thread per particle
+// linear, the instructions around the few FMAs, 57 per particle (57 % of the issue
+// slots), and 18 L1 wavefronts (69 %).  Against one thread per particle
 // with a shared integer tile (FP32) or grid atomics per node (FP64), cell-sorted
 // particles: quadratic FP32 96^3 cells 8 per cell 2.50 -> 1.89 ms, FP64 48^3 0.73 ->
-// 0.44 ms, linear FP32 101 x 67 x 83 0.278 -> 0.276 ms.  Quadratic warps hold 10
+// 0.44 ms, linear FP32 101 x 67 x 83 0.278 -> 0.240 ms.  Quadratic warps hold 10
 // (FP64: 6) particles per stream in the table and half of them in each of the two
 // coefficient chunks; other splits of the shared memory between table and chunks
 // took 1 to 9 % longer.
@@ -105,8 +105,13 @@ struct PPStreams {
     static constexpr int E_ALPHA = 9, E_DZ = 12, E_WZ = 16, E_DX = 20, E_DY = 20 + K, E_W = 20 + 2 * K;
     static constexpr int ENTRY = 36;
     static_assert(E_W + KK <= ENTRY, "a particle's entry");
-    static constexpr int CHUNK = S * H * CN;  // coefficients of a chunk
-    static constexpr size_t kBytes = sizeof(R) * (2 * CHUNK + P * ENTRY) + sizeof(int4) * P;  // per warp
+    // A stream's entries and coefficients, with linear splines 16 bytes apart: the
+    // 8 streams' reads, 4 lanes of one address each, then fall on distinct banks
+    // (without: 4 and 8 on one, 0.276 instead of 0.240 ms).
+    static constexpr int GAP = ORDER == 1 ? 16 / (int)sizeof(R) : 0;
+    static constexpr int SE = B * ENTRY + GAP, SC = H * CN + GAP;
+    static constexpr int CHUNK = S * SC;  // coefficients of a chunk
+    static constexpr size_t kBytes = sizeof(R) * (2 * CHUNK + S * SE) + sizeof(int4) * P;  // per warp
 };
 
 // Consecutive values of shared memory from a 16-byte aligned address.
@@ -145,7 +150,7 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     R* cs = reinterpret_cast<R*>(pp_smem + warp * C::kBytes);
     R* table = cs + 2 * C::CHUNK;
-    int4* meta = reinterpret_cast<int4*>(table + C::P * C::ENTRY);
+    int4* meta = reinterpret_cast<int4*>(table + S * C::SE);
     const int64_t a = ((int64_t)blockIdx.x * kPPWarps + warp) * seg;
     if (a >= n) return;
     const int64_t b = min(a + seg, n);
@@ -238,7 +243,7 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
             int left = len - s0;  // particles from the stream's next one on
 #pragma unroll 1
             for (int q = 0; q < S; ++q, left -= U, src += (int64_t)U * NVAL,
-                     dst += (unsigned)sizeof(R) * C::H * C::CN) {
+                     dst += (unsigned)sizeof(R) * C::SC) {
 #pragma unroll
                 for (int pl = 0; pl < C::H; ++pl) {
                     if (pl >= here || pl >= left) break;
@@ -260,7 +265,7 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
                     for (int v = 0; v < VPL; ++v) {
                         const int e = lane + 32 * v, r = e / NCU, comp = e - r * NCU;
                         if (e < NVAL)
-                            copy(dst + (unsigned)sizeof(R) * (q * C::H + pl) * C::CN + to[v],
+                            copy(dst + (unsigned)sizeof(R) * (q * C::SC + pl * C::CN) + to[v],
                                  src + (int64_t)(r * ncp + (STAG ? max(col, 0) : comp)) * c.comp_stride);
                     }
                 }
@@ -279,7 +284,7 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
         }
         if (lane < C::P) {
             int4 at = make_int4(-1, -1, -1, 0);
-            R* e = table + lane * C::ENTRY;
+            R* e = table + eg * C::SE + es * C::ENTRY;
             if (s0 + es < ecnt) {
                 const int64_t p = p_first + s0 + es;
                 Spline1D<ORDER, R> sp[3];
@@ -347,7 +352,7 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
         asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this chunk has landed
         __syncwarp();  // ... for every lane, and the table is written
         const int steps = min(C::H, U - (s0 + h * C::H));
-        const R* chunk = cs + (ci & 1) * C::CHUNK + g * C::H * C::CN;
+        const R* chunk = cs + (ci & 1) * C::CHUNK + g * C::SC;
 #pragma unroll 1
         for (int q = 0; q < steps; ++q) {
             const int slot = g * B + h * C::H + q;
@@ -371,7 +376,7 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
             }
             __syncwarp();
             if (!live) continue;
-            const R* e = table + slot * C::ENTRY;
+            const R* e = table + g * C::SE + (h * C::H + q) * C::ENTRY;
             R ia[12], dz[4], wz[4];  // A^-1 and alpha, d_z, w_z
             read_shared(e, ia);
             read_shared(e + C::E_DZ, dz);
