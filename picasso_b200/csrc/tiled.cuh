@@ -267,9 +267,13 @@ struct P2GCfg {
     // lanes fall on distinct banks.
     static constexpr int ENTRY = 20, WZ = 4 * NV, AT = WZ + K + (ORDER == 1 ? 1 : 0);
     static_assert(AT < ENTRY, "a particle's entry");
+    // entries of a stream; linear and cubic ones 4 floats further apart, so that the
+    // streams' reads (16 bytes, one address each) fall on distinct banks
+    static constexpr int SE = B * ENTRY + (ORDER == 2 ? 0 : 4);
+    static constexpr int TABLE = ORDER == 2 ? 32 * ENTRY : S * SE;
     // then w_x w_y m per k-row (linear: w_x, w_y) in rows of 33
     static constexpr int WROWS = ORDER == 1 ? 2 * K : KK, WROW = 33;
-    static constexpr int TILE_OFF = (32 * ENTRY + WROWS * WROW + 3) & ~3;
+    static constexpr int TILE_OFF = (TABLE + WROWS * WROW + 3) & ~3;
 };
 
 // Single-warp CTAs per SM the P2G register budget is sized for.
@@ -421,7 +425,7 @@ __device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, floa
     const TileP& tp = A.tp;
     const int lane = threadIdx.x & 31;
     float* table = warp_smem;
-    float* wrow = warp_smem + 32 * C::ENTRY;
+    float* wrow = warp_smem + C::TABLE;
     float* tile = warp_smem + C::TILE_OFF;
 
     int ob[3];
@@ -478,7 +482,7 @@ __device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, floa
         }
     };
     auto evaluate = [&](int s0) {
-        float* e = table + lane * C::ENTRY;
+        float* e = table + eg * C::SE + es * C::ENTRY;
         float out[C::ENTRY], wxy[C::WROWS];
 #pragma unroll
         for (int v = 0; v < C::ENTRY; ++v) out[v] = 0.f;
@@ -605,7 +609,7 @@ __device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, floa
         __syncwarp();
         fetch(s0 + B);
         const int steps = min(B, U - s0);
-        const float* e = table + g * B * C::ENTRY;
+        const float* e = table + g * C::SE;
         const float* w = wrow + g * B;
         // a particle's entry as the lane reads it, one step ahead of its use
         // (past the last step: the words after the entries, not used)
