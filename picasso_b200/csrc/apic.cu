@@ -183,7 +183,7 @@ static picasso_status launch_g2p_tiled_f64(const MeshP& mp, const TileP& tp, int
     if ((int64_t)(smem + rows) > device_smem_optin()) return PICASSO_OK;
     *handled = true;
     const bool packed = packed_rows_f64(x, c, 12, adv != nullptr);
-    const int64_t items = item_bound(tp, n);
+    const int64_t items = item_bound(tp);
     auto launch = [&](auto kern) -> picasso_status {
         PB_CUDA_TRY(allow_smem(kern, smem));
         kern<<<(unsigned)items, 128, smem, st>>>(mp, tp, n, x, u, c, err, adv ? *adv : Advect{}, packed);
@@ -231,20 +231,6 @@ picasso_status apic_g2p_plain(const MeshP& mp, int order, int stag, int ncomp, b
     }
     return check_launch();
 }
-
-// Tiled kernels for binned particles (tiled.cu).
-struct FusedUpdate;
-struct HaloPeers;
-picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, int64_t n,
-                              const PField& x, const PField& m, const PField& c, const GField& gm,
-                              const GField& gmu, const picasso_bins& bins, int* err,
-                              cudaStream_t st, bool* handled, const FusedUpdate* fu = nullptr,
-                              int stag = -1, const HaloPeers* hp = nullptr);
-picasso_status apic_g2p_tiled(const MeshP& mp, int order, int ncomp, bool f32, int64_t n,
-                              const PField& x, const GField& u, const PField& c,
-                              const picasso_bins& bins, int* err, const Advect* adv,
-                              cudaStream_t st, bool* handled, int stag = -1,
-                              const HaloPeers* hp = nullptr);
 
 }  // namespace pb
 

@@ -498,7 +498,7 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     const int order = in.spline.order;
     if (f32 && !valid_lanes(order, bins.p2g_lanes)) return PICASSO_ERR_INVALID_ARGUMENT;
     TileP tp;
-    if (!make_tilep(mp, order, bins, in.num_particles, &tp, f32)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, order, bins, in.num_particles, &tp, f32, true)) return PICASSO_ERR_INVALID_ARGUMENT;
 
     std::memset(static_cast<void*>(I), 0, sizeof(BInst));
     I->p2g.mp = mp;
@@ -537,7 +537,7 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     I->inv_mu = f32 ? ldexp(1.0, -in.mu_i.fixed_bits) : 1.0;
     I->n = in.num_particles;
     I->order = order;
-    const int64_t work = in.num_particles ? item_bound(tp, in.num_particles) : 0;
+    const int64_t work = in.num_particles ? item_bound(tp) : 0;
     const int64_t fill = (I->full.count() + kNodeItem - 1) / kNodeItem;
     const int64_t vel = (I->owned.count() + kNodeItem - 1) / kNodeItem;
     if (work > (1LL << 30) || fill > (1LL << 30)) return PICASSO_ERR_OUT_OF_RANGE;
@@ -708,8 +708,19 @@ extern "C" picasso_status picasso_batch_step_sequential(picasso_batch* b, void* 
         picasso_status st;
         if ((st = picasso_grid_fill(&in.spline.mesh, 1, in.m_i, 0.0, &ex_nobins))) return st;
         if ((st = picasso_grid_fill(&in.spline.mesh, 3, in.mu_i, 0.0, &ex_nobins))) return st;
-        if ((st = picasso_apic_p2g(&in.spline, in.num_particles, 3, in.x_p, in.m_p, in.c_p,
-                                   in.m_i, in.mu_i, &ex)))
+        // FP32 form: the items in the batch's parts, whose sums round alike
+        bool handled = false;
+        if (b->f32 && in.num_particles > 0) {
+            MeshP mp;
+            if ((st = make_mesh(&in.spline, &mp))) return st;
+            if ((st = apic_p2g_tiled(mp, in.spline.order, 3, Form::F32Fixed, in.num_particles,
+                                     make_pfield(in.x_p), make_pfield(in.m_p), make_pfield(in.c_p),
+                                     make_gfield(in.m_i), make_gfield(in.mu_i), in.bins, in.error_count,
+                                     static_cast<cudaStream_t>(stream), &handled, nullptr, -1, nullptr, true)))
+                return st;
+        }
+        if (!handled && (st = picasso_apic_p2g(&in.spline, in.num_particles, 3, in.x_p, in.m_p, in.c_p,
+                                               in.m_i, in.mu_i, &ex)))
             return st;
         picasso_grid_field none{};
         if ((st = picasso_grid_velocity(&in.spline.mesh, 3, in.m_i, in.mu_i, in.mass_threshold,

@@ -748,7 +748,7 @@ static picasso_status launch_pp_g2p_tiled(const MeshP& mp, const TileP& tp, int6
     const bool ws = packed_record<ORDER, NC, float>(c);
     const size_t smem = ((sizeof(float4) * tp.nodes + 15) & ~size_t(15)) +
                         (ws ? 4 * WarpRecords<float, NV>::kBytesPerWarp : 0);
-    const int64_t items = item_bound(tp, n);
+    const int64_t items = item_bound(tp);
     if (ws) {
         auto kern = polypic_g2p_tiled_kernel<ORDER, NC, true>;
         PB_CUDA_TRY(allow_smem(kern, smem));

@@ -88,29 +88,45 @@ bool valid_lanes(int order, int lanes, bool stag)
     return lanes == 1 || lanes == 2 || (lanes == 4 && !stag);
 }
 
-// Parts an item of the bins is cut into: 1 where the items give every SM 4 warps;
-// less particles than that are latency-bound (12^3 cells of 4, quadratic FP32
-// form: 12 items, one warp each: P2G 69 us, G2P 21 us; 8 parts: 20 and 9 us), so
-// their items are cut into up to 8 parts of at least 64 particles on average.  A
-// function of the sizes alone: every call on the same bins, single or batched,
-// cuts the same way and sums in the same order.
-static int item_split(int64_t ntiles, int64_t n, int chunk)
+// Cuts the items of n particles into parts, each of equal size within its item, so
+// that small sets fill the GPU and a dense tile is not one warp's work: at least
+// 1 / 9 of an SM's share of the particles (about the warps of one wave at 14 per SM
+// where no item is filled), in sets below 300 000 particles down to 64.  Where most items are
+// shorter, the empty parts behind them (1.5 ns each) stay below a tenth of the time.
+// 2 M quadratic particles (P2G): 16 per cell, 546 items 194 -> 110 us; 8 per cell, 1152
+// items 134 -> 114 us; 4 per cell clustered 226 -> 165 us; 300 000: 75 -> 37 us, clustered
+// 159 -> 48 us.  12^3 cells of 4: 69 -> 19 us.
+// A batch fills the GPU by its number of instances: there items are cut only where an
+// instance has less than 592, into at most 8 parts (24 instances up to 64^3 with the
+// other rule 1.92, so 1.76 ms).  Both are functions of the sizes alone, so that every
+// call on the same bins sums in the same order.
+static void set_parts(TileP* tp, int64_t n, bool batched)
 {
-    const int64_t items = ntiles + n / chunk;
-    if (items >= 148 * 4) return 1;
-    const int64_t parts = std::min<int64_t>(148 * 4 / items, n / ntiles / 64);
-    return (int)std::max<int64_t>(1, std::min<int64_t>(parts, 8));
+    const int64_t items = tp->ntiles + (n + tp->chunk - 1) / tp->chunk;
+    const int64_t few = 148 * 4;
+    int64_t part, parts;
+    if (batched) {
+        part = 64;
+        parts = std::min<int64_t>({few / items, n / tp->ntiles / part, 8});
+    } else {
+        part = std::max<int64_t>({n / (148 * 9), std::min<int64_t>(256, n / few), 64});
+        parts = std::min<int64_t>({(std::min<int64_t>(tp->chunk, n) + part - 1) / part,
+                                   1 + (1024 + n / 256) / items, 16});
+    }
+    tp->items_max = items;
+    tp->part = (int)std::min<int64_t>(part, tp->chunk);
+    tp->split = (int)std::max<int64_t>(1, parts);
 }
 
-int64_t item_bound(const TileP& tp, int64_t n)
+int64_t item_bound(const TileP& tp)
 {
-    return (tp.ntiles + (n + tp.chunk - 1) / tp.chunk) * tp.split;
+    return tp.items_max * tp.split;
 }
 
 // Tile geometry for the bins of n particles, with the strides of the P2G node
 // tile if asked.
 bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n, TileP* tp,
-                bool p2g_strides)
+                bool p2g_strides, bool batched)
 {
     const int K = order + 1;
     int64_t nt = 1;
@@ -147,7 +163,7 @@ bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n,
     tp->items = bins.tile_items;
     tp->chunk = bins.chunk;
     if (!bins.tile_offset || !bins.tile_items || bins.chunk < 32) return false;
-    tp->split = item_split(nt, n, bins.chunk);
+    set_parts(tp, n, batched);
     return true;
 }
 
@@ -202,7 +218,7 @@ static picasso_status launch_p2g_tiled(const P2GArgs& args, const FusedUpdate* f
     // the bulk flush rounds rows into the table: one k-row at least must fit
     if (P2GCfg<ORDER, STAG>::TILE_OFF / 8 < A.tp.NT[2]) A.bulk_flush = 0;
     const size_t smem = p2g_warp_bytes(ORDER, A.tp.P, STAG);
-    const int64_t items = item_bound(A.tp, n);
+    const int64_t items = item_bound(A.tp);
     auto launch = [&](auto kern, const FusedUpdate& F) -> picasso_status {
         PB_CUDA_TRY(allow_smem(kern, smem));
         kern<<<(unsigned)(items ? items : 1), 32, smem, st>>>(A, F, n);
@@ -221,7 +237,7 @@ static picasso_status launch_g2p_tiled(const G2PArgs& A, int64_t n, cudaStream_t
 {
     const size_t smem = sizeof(float4) * (size_t)A.tp.nodes;
     PB_CUDA_TRY(allow_smem(g2p_tiled_kernel<ORDER, ADV, REC, STAG>, smem));
-    const int64_t items = item_bound(A.tp, n);
+    const int64_t items = item_bound(A.tp);
     g2p_tiled_kernel<ORDER, ADV, REC, STAG>
         <<<(unsigned)(items ? items : 1), G2PThreads<ORDER>::value, smem, st>>>(A, n);
     return check_launch();
@@ -251,7 +267,7 @@ picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, 
                               const PField& x, const PField& m, const PField& c, const GField& gm,
                               const GField& gmu, const picasso_bins& bins, int* err,
                               cudaStream_t st, bool* handled, const FusedUpdate* fu, int stag,
-                              const HaloPeers* hp)
+                              const HaloPeers* hp, bool batched)
 {
     *handled = false;
     if (form != Form::F32Fixed || ncomp != 3 || !packed_x(x) || !packed_m(m) || !packed_c(c))
@@ -259,7 +275,7 @@ picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, 
     const bool sg = stag >= 0;
     if (!valid_lanes(order, bins.p2g_lanes, sg)) return PICASSO_ERR_INVALID_ARGUMENT;
     P2GArgs A;
-    if (!make_tilep(mp, order, bins, n, &A.tp, true)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, order, bins, n, &A.tp, true, batched)) return PICASSO_ERR_INVALID_ARGUMENT;
     A.rec = bins_records(bins);
     const bool rec = A.rec != nullptr;
     const size_t smem = p2g_warp_bytes(order, A.tp.P, sg);

@@ -51,7 +51,9 @@ struct TileP {
                  // that a plane's nodes fall on distinct banks
     int P;       // node slots of the P2G tile (NT0 * SI)
     int chunk;
-    int split;       // parts an item of the bins is cut into (item_split)
+    int split;       // parts an item of the bins is cut into at most (set_parts)
+    int part;        // particles of a part, if `split` parts suffice
+    int64_t items_max;  // items of the bins, at most
     int tsh[3];      // log2(T[d]) when T[d] is a power of two, else -1
     uint32_t tsize;  // bins per tile (sort keys of tile t start at t * tsize)
     int64_t ntiles;
@@ -154,29 +156,37 @@ __device__ __forceinline__ int node_global(const MeshP& mp, const TileP& tp, int
     return g;
 }
 
-// Work item w -- part w % split of item w / split of the bins -> tile t (-1 past
-// the last item) and particle range [a, b).  False if it has no particles.
+// Work item w -- part w / items_max of item w % items_max of the bins, so that the
+// parts beyond an item's last are launched after the others -> tile t (-1 past the
+// last item) and particle range [a, b); called by whole warps.  False if it has
+// no particles.  The tile is searched 32 at a time: the dependent loads of a binary
+// search (11 for 1224 tiles) are what an empty part costs.
 __device__ __forceinline__ bool item_range(const TileP& tp, int64_t w, int64_t& t, int64_t& a,
                                            int64_t& b)
 {
     int part = 0;
     if (tp.split > 1) {
-        part = (int)(w % tp.split);
-        w /= tp.split;
+        part = (int)(w / tp.items_max);
+        w -= part * tp.items_max;
     }
     t = -1;
-    if (w >= (int64_t)__ldg(tp.items + tp.ntiles)) return false;
+    const int lane = threadIdx.x & 31;
+    const int64_t items = (int64_t)__ldg(tp.items + tp.ntiles);
     int64_t lo = 0, hi = tp.ntiles - 1;  // last t with items[t] <= w
     while (lo < hi) {
-        const int64_t mid = (lo + hi + 1) >> 1;
-        if ((int64_t)__ldg(tp.items + mid) <= w) lo = mid;
-        else hi = mid - 1;
+        const int64_t step = (hi - lo + 32) >> 5;
+        const int64_t at = lo + lane * step;
+        const unsigned below = __ballot_sync(0xFFFFFFFFu, at <= hi && (int64_t)__ldg(tp.items + at) <= w);
+        lo += (__popc(below | 1u) - 1) * step;
+        hi = min(hi, lo + step - 1);
     }
+    if (w >= items) return false;
     t = lo;
     a = __ldg(tp.off + t) + (w - (int64_t)__ldg(tp.items + t)) * tp.chunk;
     b = min(a + (int64_t)tp.chunk, (int64_t)__ldg(tp.off + t + 1));
-    if (tp.split > 1) {  // parts of whole warps
-        const int64_t len = ((b - a + tp.split - 1) / tp.split + 31) & ~int64_t(31);
+    if (tp.split > 1) {  // equal parts of whole warps, the rest empty
+        const int np = max(1, min(tp.split, (int)((b - a + tp.part - 1) / tp.part)));
+        const int64_t len = ((b - a + np - 1) / np + 31) & ~int64_t(31);
         a += part * len;
         b = min(a + len, b);
     }
@@ -1112,13 +1122,25 @@ __device__ void g2p_item(const G2PArgs& A, int64_t t, int64_t a, int64_t b, floa
 // host helpers (tiled.cu)
 bool fused_update_fits(const TileP& tp, int order);
 bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n, TileP* tp,
-                bool p2g_strides = false);
-int64_t item_bound(const TileP& tp, int64_t n);  // items (parts) of n particles, at most
+                bool p2g_strides = false, bool batched = false);
+int64_t item_bound(const TileP& tp);  // parts of all items, at most
 int device_smem_optin();
 bool packed_x(const PField& x);
 bool packed_m(const PField& m);
 bool packed_c(const PField& c);
 bool valid_lanes(int order, int lanes, bool stag = false);
 size_t p2g_warp_bytes(int order, int P, bool stag = false);
+// Tiled kernels of a call (tiled.cu); *handled stays false where they do not take it.
+// batched: an instance's items as the batched launches cut them (set_parts).
+picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, int64_t n,
+                              const PField& x, const PField& m, const PField& c, const GField& gm,
+                              const GField& gmu, const picasso_bins& bins, int* err,
+                              cudaStream_t st, bool* handled, const FusedUpdate* fu = nullptr,
+                              int stag = -1, const HaloPeers* hp = nullptr, bool batched = false);
+picasso_status apic_g2p_tiled(const MeshP& mp, int order, int ncomp, bool f32, int64_t n,
+                              const PField& x, const GField& u, const PField& c,
+                              const picasso_bins& bins, int* err, const Advect* adv,
+                              cudaStream_t st, bool* handled, int stag = -1,
+                              const HaloPeers* hp = nullptr);
 
 }  // namespace pb
