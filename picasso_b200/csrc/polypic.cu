@@ -33,6 +33,22 @@ __device__ __forceinline__ R quad_alpha(R p, R h)
     return p * (h * h - R(4) * p * p) / (h * h);
 }
 
+// a[i] for a register array and a run-time i (a select chain, no local memory).
+template <int K, class T>
+__device__ __forceinline__ T pick(const T (&a)[K], int i)
+{
+    T v = a[0];
+#pragma unroll
+    for (int q = 1; q < K; ++q) v = (i == q) ? a[q] : v;
+    return v;
+}
+
+template <class R>
+__device__ __forceinline__ R mode1d(int deg, R r, R h, R alpha)
+{
+    return deg == 0 ? R(1) : (deg == 1 ? r : r * r - R(0.25) * h * h - alpha * r);
+}
+
 // 3x3 inverse by cofactors times 1/det (BatchedLinearAlgebra.hpp:4337-4350,
 // 4626-4686); row-major.
 template <class R>
@@ -474,9 +490,6 @@ struct WarpRecords {
     }
 };
 
-// ---------------------------------------------------------------------------
-// G2P: PolyPIC.hpp:236-293 (collocated) and :300-358 (staggered)
-// ---------------------------------------------------------------------------
 // Spline and stencil indices of a particle on the whole local mesh (periodic
 // wrap, bounds check): the placement of the plain kernels.
 template <int ORDER, class R>
@@ -495,6 +508,144 @@ struct MeshPlace {
     }
 };
 
+// One particle.  place(xp, sp, idx) evaluates the spline and the stencil's
+// grid indices (false: skip the particle); acc(f, i, j, k, v) adds v to grid
+// field f (0 mass, 1 + d momentum component d); mode(v) returns c_p value v
+// (element v of the particle's record).
+template <int ORDER, int NC, bool STAG, class PT, class R, class Place, class Acc, class Mode>
+__device__ __forceinline__ void polypic_p2g_particle(const MeshP& mp, int64_t p, const PField& x,
+                                                     const PField& m, const PField& u, R dt,
+                                                     int col, int* err, Place&& place, Acc&& acc,
+                                                     Mode&& mode)
+{
+    constexpr int K = SplineTraits<ORDER>::K;
+    {
+        Spline1D<ORDER, R> sp[3];
+        int idx[3][K];
+        const double xp[3] = {x.get<double>(p, 0), x.get<double>(p, 1), x.get<double>(p, 2)};
+        if (!place(xp, sp, idx)) {
+            if (err) atomicAdd(err, 1);
+            return;
+        }
+        const R mass = (R)m.get<PT>(p, 0);
+        // affine material motion operator and its inverse (PolyPIC.hpp:81-87)
+        R am[9], ai[9];
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int b = 0; b < 3; ++b) {
+                const R v = dt * (R)u.get<PT>(p, (1 + a) * 3 + b);
+                am[3 * a + b] = (a == b) ? R(1) + v : v;
+            }
+        inverse3(am, ai);
+        R alpha[3] = {R(0), R(0), R(0)};
+        R h[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            h[d] = (R)mp.dx[d];
+            if (ORDER == 2) alpha[d] = quad_alpha(-sp[d].d[1], h[d]);
+        }
+        // modes of the transferred field: all NC columns, or column `col`
+        constexpr int NCU = STAG ? 1 : NC;
+        constexpr int D = ORDER + 1;  // modes per dimension: degrees 0 .. ORDER
+        const int ncp = STAG ? (col >= 0 ? NC : 1) : NC;
+        // The components are transferred in passes of CB (27 FP64 modes: one
+        // at a time, so that a pass holds 27 mode values rather than 81 in
+        // registers).
+        // The basis sum sum_r c_r b_r(xi) is contracted one dimension at a
+        // time: sum_a f0_a sum_b f1_b sum_c f2_c c_(abc).
+        constexpr int CB = (sizeof(R) == 8 && ORDER == 2) ? 1 : NCU;
+#pragma unroll 1
+        for (int d0 = 0; d0 < NCU; d0 += CB) {
+            R cp[D][D][D][CB];
+            // loop over the modes: their degrees fold to constants
+#pragma unroll
+            for (int r = 0; r < D * D * D; ++r)
+#pragma unroll
+                for (int e = 0; e < CB; ++e)
+                    cp[mode_deg(r, 0)][mode_deg(r, 1)][mode_deg(r, 2)][e] =
+                        (R)mode(r * ncp + (STAG ? col : d0 + e));
+            // quadratic: i-planes one after the other, not unrolled (bounds the
+            // live range of the 9-node plane bodies, which spill in FP64, and
+            // the code size, whose instruction-cache misses stalled the FP32
+            // kernel)
+#pragma unroll(ORDER == 2 ? 1 : K)
+            for (int i = 0; i < K; ++i) {
+                const R wxi = pick<K>(sp[0].w, i), dxi = pick<K>(sp[0].d, i);
+                const int gi = pick<K>(idx[0], i);
+#pragma unroll
+                for (int j = 0; j < K; ++j)
+#pragma unroll
+                    for (int k = 0; k < K; ++k) {
+                        const R wm = mass * wxi * sp[1].w[j] * sp[2].w[k];
+                        const R dist[3] = {dxi, sp[1].d[j], sp[2].d[k]};
+                        // backtracked distance xi = A^-1 d (PolyPIC.hpp:90-106)
+                        R map[3];
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) {
+                            R t = R(0);
+#pragma unroll
+                            for (int v = 0; v < 3; ++v) t += ai[3 * q + v] * dist[v];
+                            map[q] = t;
+                        }
+                        R f[3][D];
+#pragma unroll
+                        for (int q = 0; q < 3; ++q)
+#pragma unroll
+                            for (int g = 0; g < D; ++g)
+                                f[q][g] = (ORDER == 1) ? (g == 0 ? R(1) : map[q])
+                                                       : mode1d(g, map[q], h[q], alpha[q]);
+#pragma unroll
+                        for (int e = 0; e < CB; ++e) {
+                            R sa = R(0);
+#pragma unroll
+                            for (int a = 0; a < D; ++a) {
+                                R sb = R(0);
+#pragma unroll
+                                for (int b = 0; b < D; ++b) {
+                                    R sc = R(0);
+#pragma unroll
+                                    for (int cc = 0; cc < D; ++cc) sc += f[2][cc] * cp[a][b][cc][e];
+                                    sb += f[1][b] * sc;
+                                }
+                                sa += f[0][a] * sb;
+                            }
+                            acc(1 + d0 + e, gi, idx[1][j], idx[2][k], wm * sa);
+                        }
+                        if (d0 == 0) acc(0, gi, idx[1][j], idx[2][k], wm);
+                    }
+            }
+        }
+    }
+}
+
+// FP64 P2G of particles in no known order: one thread per particle, every
+// contribution added to the grid by itself, bound by the L2's additions (108 per
+// quadratic particle, 180 G/s).  In random order a stream of the kernel above moves
+// its stencil with nearly every particle and adds as much, on top of its tables: 1 M
+// particles, quadratic 0.69 to 0.73 ms there and 0.60 here, linear 0.236 and 0.196 ms.
+// Exchanging the sums so that four lanes add a whole node cost more than it saved
+// (quadratic 1.07 ms).  In the order of a cell sort the streams win: quadratic 3 to 14
+// per cell 0.49 and 0.46 ms against 0.68 and 1.56 ms.
+template <int ORDER, int NC, bool STAG>
+__global__ void __launch_bounds__(128)
+polypic_p2g_plain_kernel(MeshP mp, int64_t n, PField x, PField m, PField u, PField c, GField gmu,
+                   GField gm, double dt, int col, int* err)
+{
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    const MeshPlace<ORDER, double> place{mp};
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
+        polypic_p2g_particle<ORDER, NC, STAG, double, double>(
+            mp, p, x, m, u, dt, col, err, place,
+            [&](int f, int i, int j, int k, double v) {
+                atomicAdd(f == 0 ? gm.ptr<double>(i, j, k, 0) : gmu.ptr<double>(i, j, k, f - 1), v);
+            },
+            [&](int v) { return c.get<double>(p, v); });
+}
+
+// ---------------------------------------------------------------------------
+// G2P: PolyPIC.hpp:236-293 (collocated) and :300-358 (staggered)
+// ---------------------------------------------------------------------------
 // One particle; emit(v, value) receives c_p value v (element v of the
 // particle's record).  False if the particle was skipped (stencil outside a
 // non-periodic mesh): then nothing is emitted.
@@ -797,11 +948,16 @@ static picasso_status launch_pp_p2g_form(const MeshP& mp, const TileP& tp, int64
 }
 
 template <int ORDER, int NC, bool STAG>
-static picasso_status launch_pp_p2g(int form, const MeshP& mp, const TileP& tp, int64_t n, const PField& x,
+static picasso_status launch_pp_p2g(int form, bool sorted, const MeshP& mp, const TileP& tp, int64_t n, const PField& x,
                                     const PField& m, const PField& u, const PField& c,
                                     const GField& gmu, const GField& gm, double dt, int col, int* err,
                                     cudaStream_t st)
 {
+    if (form == 0 && !sorted) {
+        polypic_p2g_plain_kernel<ORDER, NC, STAG>
+            <<<grid_for(n, 128, 148LL * 128), 128, 0, st>>>(mp, n, x, m, u, c, gmu, gm, dt, col, err);
+        return check_launch();
+    }
     if (form == 0)
         return launch_pp_p2g_form<ORDER, NC, STAG, double, double, false>(
             mp, tp, n, x, m, u, c, gmu, gm, dt, col, 0.0, 0.0, err, st);
@@ -917,16 +1073,25 @@ extern "C" picasso_status picasso_polypic_p2g(const picasso_spline* sd, int64_t 
     const bool p2g_ok = form == 1 && stag < 0 && exec && exec->bins && exec->bins->chunk <= 65536;
     if ((st = polypic_tiles(sd, exec, num_particles, p2g_ok, mp, 12 * (1 + ncomp), &tiled, &tp))) return st;
     if (!tiled) tp.off = nullptr;
+    // The bins tell that the particles are in the order of their stencils; with linear
+    // splines and less than two per stencil the streams gain nothing by it (1 M
+    // particles, 1 per cell: 0.187 ms, plain 0.183; 3 per cell 0.151 and 0.205).
+    bool sorted = exec && exec->bins;
+    if (sorted && sd->order == 1) {
+        double stencils = 1.0;
+        for (int d = 0; d < 3; ++d) stencils *= exec->bins->bin_extent[d];
+        sorted = num_particles >= 2 * stencils;
+    }
     if (sd->order == 1) {
         if (stag >= 0) {
             PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, true>(
-                                       form, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
+                                       form, sorted, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
         } else {
             PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, false>(
-                                       form, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
+                                       form, sorted, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
         }
     }
-    PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<2, NC_, false>(form, mp, tp, num_particles, x, m, u, c,
+    PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<2, NC_, false>(form, sorted, mp, tp, num_particles, x, m, u, c,
                                                                gmu, gm, dt, col, err, s));
     return PICASSO_OK;
 }

@@ -131,3 +131,29 @@ def test_particles_out_of_their_tile_are_counted(cuda, order, tile):
     gm2, gmu2, _ = _p2g(mesh, loc, order, "fp32", xs[stays], m[stays], u[stays], u[stays], False)
     assert err == int((~stays).sum())
     assert torch.equal(gm.raw, gm2.raw) and torch.equal(gmu.raw, gmu2.raw)
+
+
+@pytest.mark.parametrize("case", [c for c in CASES if c[5] == "packed"], ids=lambda c: "-".join(map(str, c)))
+def test_fp64_streams_of_sorted_particles(cuda, case):
+    """FP64 grids take the streams when the call has bins (linear splines: from 2
+    particles per stencil on, here by repeating them); the tolerance of test_streams."""
+    order, nc, kind, where, n, _ = case
+    mesh, hi = _mesh(kind)
+    loc = FieldLocation.Node if where == "node" else FieldLocation.Face(1)
+    rng = np.random.default_rng(n)
+    n = n if order == 2 else n + 2 * int(np.prod(mesh.extent(loc)))
+    x = torch.as_tensor(rng.random((n, 3)) * hi, device="cuda")
+    _, perm, bins = cell_sort(create_spline(loc, order, mesh, x), (4, 4, 8), chunk=64)
+    x = permute_members(perm, x)[0].cpu().numpy()
+    nm = 8 if order == 1 else 27
+    m = rng.uniform(0.5, 1.5, n)
+    u = rng.standard_normal((n, nm, 3))
+    u[:, 1:] *= 0.05
+    c = np.ascontiguousarray(u[..., :nc])
+    gm, gmu, err = _p2g(mesh, loc, order, "fp64", x, m, u, c, False, bins)
+    ext = mesh.extent(loc)
+    gm_o, gmu_o = np.zeros(ext), np.zeros(ext + ((nc,) if where == "node" else ()))
+    oracle.polypic_p2g(create_spline(loc, order, mesh, None).desc, x, m, u, c, gmu_o, gm_o, DT)
+    assert err == 0
+    assert rel_err(gm.cpu().numpy(), gm_o) <= 1e-12
+    assert rel_err(gmu.cpu().numpy(), gmu_o) <= 1e-12
