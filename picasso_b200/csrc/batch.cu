@@ -498,7 +498,9 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     const int order = in.spline.order;
     if (f32 && !valid_lanes(order, bins.p2g_lanes)) return PICASSO_ERR_INVALID_ARGUMENT;
     TileP tp;
-    if (!make_tilep(mp, order, bins, in.num_particles, &tp, f32, true)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, order, bins, in.num_particles, &tp,
+                    f32 ? TileUse::batch_streams : TileUse::batch_other))
+        return PICASSO_ERR_INVALID_ARGUMENT;
 
     std::memset(static_cast<void*>(I), 0, sizeof(BInst));
     I->p2g.mp = mp;

@@ -6,7 +6,9 @@
 // 4-warp CTA would wait for its slowest warp).
 // G2P runs 128-thread CTAs sharing one node tile.
 #include <algorithm>
+#include <mutex>
 
+#include "run_p2g.cuh"
 #include "tiled.cuh"
 
 namespace pb {
@@ -31,6 +33,23 @@ p2g_tiled_kernel(P2GArgs A, FusedUpdate F, int64_t n)
     int64_t t, a, b;
     const bool any = item_range(A.tp, blockIdx.x, t, a, b);
     if (any) p2g_item<ORDER, REC, STAG>(A, t, a, b, smem);
+    if constexpr (FUSED) {
+        if (t >= 0) fused_update_arrive<ORDER>(A, F, t);
+    }
+}
+
+template <int ORDER, bool REC, bool FUSED>
+__global__ void __launch_bounds__(32, kRunOccupancy)
+p2g_runs_kernel(P2GArgs A, FusedUpdate F, int64_t n)
+{
+    extern __shared__ __align__(16) float smem[];
+    __shared__ int base[32];
+    if (blockIdx.x == 0 && threadIdx.x == 0 && A.err) {
+        const int64_t n_valid = __ldg(A.tp.off + A.tp.ntiles);
+        if (n > n_valid) atomicAdd(A.err, (int)(n - n_valid));
+    }
+    int64_t t, a, b;
+    if (item_range(A.tp, blockIdx.x, t, a, b)) run_p2g_item<ORDER, REC>(A, t, a, b, smem, base);
     if constexpr (FUSED) {
         if (t >= 0) fused_update_arrive<ORDER>(A, F, t);
     }
@@ -78,6 +97,78 @@ static void choose_strides(const int NT[3], int K, int* SJ, int* SI)
         }
 }
 
+// Node-tile strides of the P2G in runs: value lane + 32 r of a staged lane (4 fields of
+// K^3 nodes) lands at f P + a SI + b SJ + c; the smallest padding that puts the most of
+// a merge round's 32 values on distinct banks.  The search takes a fraction of a
+// millisecond, so the last shapes are kept.
+struct RunStrides {
+    int NT[3], K, SJ, SI, P;
+};
+
+static void search_run_strides(RunStrides* s)
+{
+    const int K = s->K, KKK = K * K * K, FS = (KKK + 3) & ~3, SV = 4 * FS;
+    int best = -1;
+    long size = 0;
+    for (int sj = s->NT[2]; sj < s->NT[2] + 8; ++sj)
+        for (int si = s->NT[1] * sj; si < s->NT[1] * sj + 16; ++si)
+            for (int pp = s->NT[0] * si; pp < s->NT[0] * si + 16; ++pp) {
+                int distinct = 0;
+                for (int r = 0; r < SV; r += 32) {
+                    unsigned banks = 0;
+                    for (int v = r; v < r + 32 && v < SV; ++v) {
+                        const int n = v % FS;
+                        if (n < KKK)
+                            banks |= 1u << ((v / FS * pp + n / (K * K) * si + n / K % K * sj + n % K) & 31);
+                    }
+                    distinct += __builtin_popcount(banks);
+                }
+                if (distinct > best || (distinct == best && pp < size)) {
+                    best = distinct;
+                    size = pp;
+                    s->SJ = sj;
+                    s->SI = si;
+                    s->P = pp;
+                }
+            }
+}
+
+static RunStrides run_strides(const int NT[3], int K)
+{
+    constexpr int kSlots = 64;
+    static std::mutex mu;
+    static RunStrides kept[kSlots];
+    static int used = 0, next = 0;
+    RunStrides s{{NT[0], NT[1], NT[2]}, K, 0, 0, 0};
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        for (int i = 0; i < used; ++i)
+            if (kept[i].K == K && std::equal(NT, NT + 3, kept[i].NT)) return kept[i];
+    }
+    search_run_strides(&s);
+    std::lock_guard<std::mutex> lock(mu);
+    kept[used < kSlots ? used++ : next++ % kSlots] = s;
+    return s;
+}
+
+// Sets whose FP32 P2G keeps its sums in runs (run_p2g.cuh) instead of streams.
+// Positions are FP64 and move by FP32 velocities, so the rounding of the node sums
+// shows in them: sums in another order put the advected positions of a step (dt 0.1
+// cells) 0.7e-9 to 2.4e-9 apart with linear splines, whose gradients make the
+// velocities several times the drawn ones, and with quadratic splines 1.4e-9 at one
+// particle per cell, 1.1e-9 at two, 0.9e-9 at three and 0.8e-9 at four (relative to
+// their norm).  A program that continues a run repeats its positions to 1e-9 only if
+// such sets are summed in the same order as ever.  Cubic ones stay below 0.9e-9.
+// (The streams would take 0.6 to 0.9 times as long on them.)  A batch, which moves no
+// particle, and staggered fields take the streams.
+static bool run_sums(int order, const picasso_bins& bins, int64_t n)
+{
+    if (order != 2) return order == 1;
+    double cells = 1.0;
+    for (int d = 0; d < 3; ++d) cells *= bins.bin_extent[d];
+    return n < 4.0 * cells;
+}
+
 // Values of picasso_bins.p2g_lanes a call accepts (the P2G's lanes per particle
 // follow from the order: one per k-row of the stencil): orders 1 and 2 take 1, 2
 // or 4 (staggered locations 1 or 2), order 3 takes 4; 0 always.
@@ -100,12 +191,16 @@ bool valid_lanes(int order, int lanes, bool stag)
 // instance has less than 592, into at most 8 parts (24 instances up to 64^3 with the
 // other rule 1.92, so 1.76 ms).  Both are functions of the sizes alone, so that every
 // call on the same bins sums in the same order.
-static void set_parts(TileP* tp, int64_t n, bool batched)
+// The runs of a whole item are 32 already: they are not cut.
+static void set_parts(TileP* tp, int64_t n, TileUse use)
 {
     const int64_t items = tp->ntiles + (n + tp->chunk - 1) / tp->chunk;
     const int64_t few = 148 * 4;
     int64_t part, parts;
-    if (batched) {
+    if (use == TileUse::runs) {
+        part = tp->chunk;
+        parts = 1;
+    } else if (use == TileUse::batch_streams || use == TileUse::batch_other) {
         part = 64;
         parts = std::min<int64_t>({few / items, n / tp->ntiles / part, 8});
     } else {
@@ -126,7 +221,7 @@ int64_t item_bound(const TileP& tp)
 // Tile geometry for the bins of n particles, with the strides of the P2G node
 // tile if asked.
 bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n, TileP* tp,
-                bool p2g_strides, bool batched)
+                TileUse use)
 {
     const int K = order + 1;
     int64_t nt = 1;
@@ -148,7 +243,13 @@ bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n,
     tp->SJ = tp->NT[2];
     tp->SI = tp->NT[1] * tp->NT[2];
     tp->P = tp->nodes;
-    if (p2g_strides) {
+    tp->runs = use == TileUse::runs;
+    if (tp->runs) {
+        const RunStrides s = run_strides(tp->NT, K);
+        tp->SJ = s.SJ;
+        tp->SI = s.SI;
+        tp->P = s.P;
+    } else if (use == TileUse::streams || use == TileUse::batch_streams) {
         int sj, si;
         choose_strides(tp->NT, K, &sj, &si);
         // (a tile that the padding pushes out of shared memory stays unpadded)
@@ -163,7 +264,7 @@ bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n,
     tp->items = bins.tile_items;
     tp->chunk = bins.chunk;
     if (!bins.tile_offset || !bins.tile_items || bins.chunk < 32) return false;
-    set_parts(tp, n, batched);
+    set_parts(tp, n, use);
     return true;
 }
 
@@ -208,6 +309,32 @@ size_t p2g_warp_bytes(int order, int P, bool stag)
                        : order == 2 ? (stag ? p2g_warp_floats<2, true>(P) : p2g_warp_floats<2>(P))
                                     : (stag ? p2g_warp_floats<3, true>(P) : p2g_warp_floats<3>(P));
     return sizeof(float) * (size_t)floats;
+}
+
+// (with 128 bytes of static shared memory beside it)
+static size_t run_warp_bytes(int order, bool rec, int P)
+{
+    const int floats = order == 1 ? (rec ? run_warp_floats<1, true>(P) : run_warp_floats<1, false>(P))
+                                  : (rec ? run_warp_floats<2, true>(P) : run_warp_floats<2, false>(P));
+    return sizeof(float) * (size_t)floats + 128;
+}
+
+template <int ORDER, bool REC>
+static picasso_status launch_p2g_runs(const P2GArgs& args, const FusedUpdate* fu, int64_t n,
+                                      cudaStream_t st)
+{
+    P2GArgs A = args;
+    // (as below: one k-row at least must fit)
+    if (RunCfg<ORDER, REC>::TILE_OFF / 8 < A.tp.NT[2]) A.bulk_flush = 0;
+    const size_t smem = sizeof(float) * (size_t)run_warp_floats<ORDER, REC>(A.tp.P);
+    const int64_t items = item_bound(A.tp);
+    auto launch = [&](auto kern, const FusedUpdate& F) -> picasso_status {
+        PB_CUDA_TRY(allow_smem(kern, smem));
+        kern<<<(unsigned)(items ? items : 1), 32, smem, st>>>(A, F, n);
+        return check_launch();
+    };
+    if (fu) return launch(p2g_runs_kernel<ORDER, REC, true>, *fu);
+    return launch(p2g_runs_kernel<ORDER, REC, false>, FusedUpdate{});
 }
 
 template <int ORDER, bool REC, bool STAG>
@@ -275,10 +402,13 @@ picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, 
     const bool sg = stag >= 0;
     if (!valid_lanes(order, bins.p2g_lanes, sg)) return PICASSO_ERR_INVALID_ARGUMENT;
     P2GArgs A;
-    if (!make_tilep(mp, order, bins, n, &A.tp, true, batched)) return PICASSO_ERR_INVALID_ARGUMENT;
+    const TileUse use = batched ? TileUse::batch_streams
+                                : !sg && run_sums(order, bins, n) ? TileUse::runs : TileUse::streams;
+    if (!make_tilep(mp, order, bins, n, &A.tp, use)) return PICASSO_ERR_INVALID_ARGUMENT;
     A.rec = bins_records(bins);
     const bool rec = A.rec != nullptr;
-    const size_t smem = p2g_warp_bytes(order, A.tp.P, sg);
+    const size_t smem = A.tp.runs ? run_warp_bytes(order, rec, A.tp.P)
+                                  : p2g_warp_bytes(order, A.tp.P, sg);
     if ((int64_t)smem > device_smem_optin()) return PICASSO_OK;  // tile too large: plain path
     *handled = true;
     A.mp = mp;
@@ -295,6 +425,11 @@ picasso_status apic_p2g_tiled(const MeshP& mp, int order, int ncomp, Form form, 
     // the fused update counts its arrivals after element-wise reductions; a
     // neighbour's rows take element-wise reductions too
     A.bulk_flush = !sg && !fu && !A.hp.on && packed_accumulator(gm, gmu);
+    if (A.tp.runs) {
+        if (order == 1)
+            return rec ? launch_p2g_runs<1, true>(A, fu, n, st) : launch_p2g_runs<1, false>(A, fu, n, st);
+        return rec ? launch_p2g_runs<2, true>(A, fu, n, st) : launch_p2g_runs<2, false>(A, fu, n, st);
+    }
 #define PB_CASE(O)                                                                         \
     if (order == O)                                                                        \
         return sg ? (rec ? launch_p2g_tiled<O, true, true>(A, fu, n, st)                   \

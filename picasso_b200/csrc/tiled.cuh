@@ -6,7 +6,8 @@
 // Work items are chunks of at most `chunk` particles of one tile (the sort
 // writes the per-tile item prefix).
 //
-// P2G item (one warp): the item's sorted particles are cut into S contiguous
+// P2G item (one warp; linear splines and sparse quadratic sets: run_p2g.cuh): the item's
+// sorted particles are cut into S contiguous
 // streams (3 for quadratic, 2 for cubic, 8 for linear splines) that the warp
 // sweeps side by side.  The lanes first evaluate the next 32 / S particles of
 // every stream, one particle each (splines, the affine velocity relative to the
@@ -49,7 +50,8 @@ struct TileP {
     int nodes;   // NT0 * NT1 * NT2
     int SJ, SI;  // P2G node-tile strides along j and i (k stride 1), padded so
                  // that a plane's nodes fall on distinct banks
-    int P;       // node slots of the P2G tile (NT0 * SI)
+    int P;       // node slots of the P2G tile (NT0 * SI, in runs padded too)
+    bool runs;   // P2G in runs (run_p2g.cuh)
     int chunk;
     int split;       // parts an item of the bins is cut into at most (set_parts)
     int part;        // particles of a part, if `split` parts suffice
@@ -349,10 +351,10 @@ __device__ __forceinline__ bool locate_record(const MeshP& mp, const TileP& tp, 
 // reduction (two where it wraps around a periodic boundary; rows and nodes
 // past a non-periodic mesh end are left out -- no stencil reaches them).
 // The integer sums do not depend on the order of the reductions.
-template <int ORDER>
-__device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, const float* tile, int i_lo,
-                                                int i_hi, const int ob[3], float* buf_f,
-                                                int buf_nodes, int lane)
+template <int ORDER, class Values>
+__device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, Values&& values, int i_lo, int i_hi,
+                                                const int ob[3], float* buf_f, int buf_nodes,
+                                                int lane)
 {
     constexpr int K = SplineTraits<ORDER>::K;
     const MeshP& mp = A.mp;
@@ -378,8 +380,8 @@ __device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, const float* t
             const int row = r0 + q;
             const int i = i_lo + row / e1, j = row - (row / e1) * e1;
             const int idx = i * tp.SI + j * tp.SJ + k;
-            const float4 v = reinterpret_cast<const float4*>(tile)[idx];
-            const float x[4] = {v.x, v.y, v.z, v.w};
+            float x[4];
+            values(idx, x);
             long long w[4];
 #pragma unroll
             for (int f = 0; f < 4; ++f)
@@ -410,6 +412,83 @@ __device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, const float* t
     __syncwarp();
 }
 
+// A P2G item's node box (values(idx, x): the NF fields at tile index idx), rounded to
+// fixed point and added to HBM: by bulk reductions of whole k-rows into a packed
+// accumulator (`buf`, room for buf_nodes nodes, holds the rounded rows), else node by
+// node (nodes that received nothing are skipped).  any: the item added something.
+template <int ORDER, int NF, class Values>
+__device__ __forceinline__ void flush_tile(const P2GArgs& A, Values&& values, bool any, int i_lo,
+                                           int i_hi, const int ob[3], float* buf, int buf_nodes,
+                                           int lane)
+{
+    constexpr int K = SplineTraits<ORDER>::K;
+    const MeshP& mp = A.mp;
+    const TileP& tp = A.tp;
+    if (!any) return;
+    if (NF == 4 && A.bulk_flush) {
+        if constexpr (NF == 4) flush_rows_bulk<ORDER>(A, values, i_lo, i_hi, ob, buf, buf_nodes, lane);
+        return;
+    }
+    const int e1 = tp.NT[1], e2 = tp.NT[2];
+    const int total = (i_hi - i_lo + K) * e1 * e2;
+    for (int e = lane; e < total; e += 32) {
+        const int k = e % e2;
+        const int j = (e / e2) % e1;
+        const int i = i_lo + e / (e1 * e2);
+        const int idx = i * tp.SI + j * tp.SJ + k;
+        const int gi = node_global(mp, tp, 0, ob[0], i);
+        const int gj = node_global(mp, tp, 1, ob[1], j);
+        const int gk = node_global(mp, tp, 2, ob[2], k);
+        // this rank's grids, or the neighbour's that owns plane gi
+        int gx_m, gx_mu;
+        char* bm = halo_route(A.hp, 0, A.gm.data, gi, gx_m);
+        char* bmu = halo_route(A.hp, 1, A.gmu.data, gi, gx_mu);
+        float v[NF];
+        values(idx, v);
+#pragma unroll
+        for (int f = 0; f < NF; ++f) {
+            if (v[f] != 0.f) {
+                const long long q =
+                    to_fixed(f == 0 ? A.gm : A.gmu, v[f] * (f == 0 ? A.scale_m : A.scale_mu));
+                unsigned long long* dst =
+                    f == 0 ? reinterpret_cast<unsigned long long*>(bm) + A.gm.index(gx_m, gj, gk, 0)
+                           : reinterpret_cast<unsigned long long*>(bmu) +
+                                 A.gmu.index(gx_mu, gj, gk, NF == 2 ? 0 : f - 1);
+                atomicAdd(dst, (unsigned long long)q);
+            }
+        }
+    }
+}
+
+// Bin rows [i_lo, i_hi] spanned by an item's particles [a, b) (keys are i-major within
+// a tile): the first and last particle bound them; the item's node box is these rows
+// plus the halo, over the whole tile along j and k.
+template <int ORDER, bool REC>
+__device__ __forceinline__ void p2g_rows(const P2GArgs& A, int64_t t, int64_t a, int64_t b,
+                                         const int ob[3], int& i_lo, int& i_hi)
+{
+    const MeshP& mp = A.mp;
+    const TileP& tp = A.tp;
+    i_lo = 0;
+    i_hi = tp.T[0] - 1;
+    int la[3], lz[3];
+    bool oka, okb;
+    if constexpr (REC) {
+        oka = bin_of_key(tp, t, __float_as_uint(__ldg(A.rec + 4 * a + 3)), la);
+        okb = bin_of_key(tp, t, __float_as_uint(__ldg(A.rec + 4 * (b - 1) + 3)), lz);
+    } else {
+        Spline1D<ORDER, float> sp[3];
+        const double xa[3] = {A.x[3 * a], A.x[3 * a + 1], A.x[3 * a + 2]};
+        const double xb[3] = {A.x[3 * (b - 1)], A.x[3 * (b - 1) + 1], A.x[3 * (b - 1) + 2]};
+        oka = locate<ORDER>(mp, tp, xa, ob, sp, la);
+        okb = locate<ORDER>(mp, tp, xb, ob, sp, lz);
+    }
+    if (oka && okb && lz[0] >= la[0]) {
+        i_lo = la[0];
+        i_hi = lz[0];
+    }
+}
+
 // One P2G work item (tile t, particles [a, b)) by the calling warp.  `warp_smem`
 // holds p2g_warp_floats<ORDER, STAG>(P) floats (16-byte aligned).  REC: the
 // particles' positions arrive as spline records (in-cell fraction of the
@@ -438,30 +517,9 @@ __device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, floa
     float* wrow = warp_smem + C::TABLE;
     float* tile = warp_smem + C::TILE_OFF;
 
-    int ob[3];
+    int ob[3], i_lo, i_hi;
     tile_origin(tp, t, ob);
-    // bin rows spanned by the item (keys are i-major within a tile): the
-    // first and last particle bound them; the item's node box is these rows
-    // plus the halo, over the whole tile along j and k
-    int i_lo = 0, i_hi = tp.T[0] - 1;
-    {
-        int la[3], lz[3];
-        bool oka, okb;
-        if constexpr (REC) {
-            oka = bin_of_key(tp, t, __float_as_uint(__ldg(A.rec + 4 * a + 3)), la);
-            okb = bin_of_key(tp, t, __float_as_uint(__ldg(A.rec + 4 * (b - 1) + 3)), lz);
-        } else {
-            Spline1D<ORDER, float> sp[3];
-            const double xa[3] = {A.x[3 * a], A.x[3 * a + 1], A.x[3 * a + 2]};
-            const double xb[3] = {A.x[3 * (b - 1)], A.x[3 * (b - 1) + 1], A.x[3 * (b - 1) + 2]};
-            oka = locate<ORDER>(mp, tp, xa, ob, sp, la);
-            okb = locate<ORDER>(mp, tp, xb, ob, sp, lz);
-        }
-        if (oka && okb && lz[0] >= la[0]) {
-            i_lo = la[0];
-            i_hi = lz[0];
-        }
-    }
+    p2g_rows<ORDER, REC>(A, t, a, b, ob, i_lo, i_hi);
 
     for (int i = lane; i < NF * tp.P / 2; i += 32)
         reinterpret_cast<float2*>(tile)[i] = make_float2(0.f, 0.f);
@@ -686,42 +744,16 @@ __device__ void p2g_item(const P2GArgs& A, int64_t t, int64_t a, int64_t b, floa
     }
     const unsigned last = __ballot_sync(kFull, cur >= 0);
     if (last) merge(last, cur >= 0, false);
-    // the item's node box, rounded to fixed point and added to HBM: by bulk
-    // reductions of whole k-rows into a packed accumulator (the table holds the
-    // rounded rows), else node by node (nodes that received nothing are skipped)
-    if (!STAG && A.bulk_flush && last) {
-        flush_rows_bulk<ORDER>(A, tile, i_lo, i_hi, ob, warp_smem, C::TILE_OFF / 8, lane);
-    } else if (last) {
-        const int e1 = tp.NT[1], e2 = tp.NT[2];
-        const int total = (i_hi - i_lo + K) * e1 * e2;
-        for (int e = lane; e < total; e += 32) {
-            const int k = e % e2;
-            const int j = (e / e2) % e1;
-            const int i = i_lo + e / (e1 * e2);
-            const int idx = i * tp.SI + j * tp.SJ + k;
-            const int gi = node_global(mp, tp, 0, ob[0], i);
-            const int gj = node_global(mp, tp, 1, ob[1], j);
-            const int gk = node_global(mp, tp, 2, ob[2], k);
-            // this rank's grids, or the neighbour's that owns plane gi
-            int gx_m, gx_mu;
-            char* bm = halo_route(A.hp, 0, A.gm.data, gi, gx_m);
-            char* bmu = halo_route(A.hp, 1, A.gmu.data, gi, gx_mu);
-#pragma unroll
-            for (int f = 0; f < NF; ++f) {
-                const float v = tile[NF * idx + f];
-                if (v != 0.f) {
-                    const long long q =
-                        to_fixed(f == 0 ? A.gm : A.gmu, v * (f == 0 ? A.scale_m : A.scale_mu));
-                    unsigned long long* dst =
-                        f == 0 ? reinterpret_cast<unsigned long long*>(bm) +
-                                     A.gm.index(gx_m, gj, gk, 0)
-                               : reinterpret_cast<unsigned long long*>(bmu) +
-                                     A.gmu.index(gx_mu, gj, gk, STAG ? 0 : f - 1);
-                    atomicAdd(dst, (unsigned long long)q);
-                }
-            }
+    auto values = [&](int idx, float (&x)[NF]) {
+        if constexpr (NF == 4) {
+            const float4 v = reinterpret_cast<const float4*>(tile)[idx];
+            x[0] = v.x, x[1] = v.y, x[NF - 2] = v.z, x[NF - 1] = v.w;
+        } else {
+            const float2 v = reinterpret_cast<const float2*>(tile)[idx];
+            x[0] = v.x, x[1] = v.y;
         }
-    }
+    };
+    flush_tile<ORDER, NF>(A, values, last != 0, i_lo, i_hi, ob, warp_smem, C::TILE_OFF / 8, lane);
     __syncwarp();
 }
 
@@ -896,8 +928,9 @@ __device__ __forceinline__ float add_term(int n, float w, float v, float sum)
 }
 
 // Term n of S0 = sum w_n v_n and S1 = sum (n - n0) w_n v_n, n0 the stencil's centre
-// knot (0 linear, else 1), in the fewest instructions: 2 (linear), 4 (quadratic)
-// and 6 (cubic) for all terms.
+// knot (0 linear, else 1), in few instructions: 3 (linear), 4 (quadratic) and 6 (cubic)
+// for all terms.  (Linear: the product twice, once in the sum's FMA, as the velocities
+// that advected positions follow have always been rounded; run_sums in tiled.cu.)
 template <int ORDER>
 __device__ __forceinline__ void add_moments(int n, float w, float v, float& S0, float& S1)
 {
@@ -906,7 +939,7 @@ __device__ __forceinline__ void add_moments(int n, float w, float v, float& S0, 
             S0 = __fmul_rn(w, v);
         } else {
             S1 = __fmul_rn(w, v);
-            S0 = __fadd_rn(S0, S1);
+            S0 = fmaf(w, v, S0);
         }
     } else {
         if (n == 0) {
@@ -1121,8 +1154,11 @@ __device__ void g2p_item(const G2PArgs& A, int64_t t, int64_t a, int64_t b, floa
 
 // host helpers (tiled.cu)
 bool fused_update_fits(const TileP& tp, int order);
+// What a tile is made for: `streams` and `runs` set the strides of the P2G's node tile
+// (p2g_item, run_p2g_item); a batch's items are cut by a rule of their own (set_parts).
+enum class TileUse { other, streams, batch_streams, runs, batch_other };
 bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n, TileP* tp,
-                bool p2g_strides = false, bool batched = false);
+                TileUse use = TileUse::other);
 int64_t item_bound(const TileP& tp);  // parts of all items, at most
 int device_smem_optin();
 bool packed_x(const PField& x);
