@@ -780,17 +780,11 @@ struct FusedUpdate {
 };
 
 // Local node range [lo, hi) of the region part `low` of tile q along d.
-__device__ __forceinline__ void region_range(const MeshP& mp, const TileP& tp, int d, int q,
-                                             int low, int K, int& lo, int& hi)
+__device__ __forceinline__ void region_range(const TileP& tp, int d, int q, int low, int K, int& lo,
+                                             int& hi)
 {
-    const int teff = min(tp.T[d], tp.nb[d] - q * tp.T[d]);
-    if (low) {
-        lo = 0;
-        hi = K - 1;
-    } else {
-        lo = K - 1;
-        hi = teff + ((!mp.periodic[d] && q == tp.nt[d] - 1) ? K - 1 : 0);
-    }
+    lo = low ? 0 : K - 1;
+    hi = low ? K - 1 : min(tp.T[d], tp.nb[d] - q * tp.T[d]);
 }
 
 __device__ __forceinline__ uint32_t tile_items_of(const TileP& tp, int64_t s)
@@ -877,7 +871,7 @@ __device__ void fused_update_arrive(const P2GArgs& A, const FusedUpdate& F, int6
         const int cq[3] = {(int)(ct / ((int64_t)tp.nt[1] * tp.nt[2])),
                            (int)((ct / tp.nt[2]) % tp.nt[1]), (int)(ct % tp.nt[2])};
         int lo[3], hi[3];
-        for (int d = 0; d < 3; ++d) region_range(mp, tp, d, cq[d], (cr >> d) & 1, K, lo[d], hi[d]);
+        for (int d = 0; d < 3; ++d) region_range(tp, d, cq[d], (cr >> d) & 1, K, lo[d], hi[d]);
         const int n1 = hi[1] - lo[1], n2 = hi[2] - lo[2];
         const int total = (hi[0] - lo[0]) * n1 * n2;
         for (int e = lane; e < total; e += 32) {
@@ -904,7 +898,7 @@ __global__ void zero_untouched_regions_kernel(MeshP mp, TileP tp, FusedUpdate F)
                           (int)((t / tp.nt[2]) % tp.nt[1]), (int)(t % tp.nt[2])};
         if (region_items(mp, tp, q, reg) != 0) continue;
         int lo[3], hi[3];
-        for (int d = 0; d < 3; ++d) region_range(mp, tp, d, q[d], (reg >> d) & 1, K, lo[d], hi[d]);
+        for (int d = 0; d < 3; ++d) region_range(tp, d, q[d], (reg >> d) & 1, K, lo[d], hi[d]);
         for (int i = lo[0]; i < hi[0]; ++i)
             for (int j = lo[1]; j < hi[1]; ++j)
                 for (int k = lo[2]; k < hi[2]; ++k) {
