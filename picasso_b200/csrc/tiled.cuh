@@ -147,12 +147,18 @@ __device__ __forceinline__ int bin_of(const MeshP& mp, const TileP& tp, int d, i
     return s0;
 }
 
+// Node of the tile with bin origin ob along d.  (A tile with its halo can span several
+// periods of a thin mesh.)
 __device__ __forceinline__ int node_global(const MeshP& mp, const TileP& tp, int d, int ob,
                                            int local)
 {
     int g = ob + local;
     if (mp.periodic[d]) {
-        if (g >= tp.nb[d]) g -= tp.nb[d];
+        const int nb = tp.nb[d];
+        if (g >= nb) {
+            g -= nb;
+            if (g >= nb) g %= nb;
+        }
         return mp.own_lo[d] + g;
     }
     return g;
@@ -348,8 +354,8 @@ __device__ __forceinline__ bool locate_record(const MeshP& mp, const TileP& tp, 
 // whole tile along j and k) into a packed accumulator: the box's k-rows are
 // rounded to fixed point into `buf` (room for buf_nodes nodes of 4 words, a
 // group of rows at a time) and each row is added to HBM by one bulk
-// reduction (two where it wraps around a periodic boundary; rows and nodes
-// past a non-periodic mesh end are left out -- no stencil reaches them).
+// reduction (one more for every time it wraps around a periodic boundary; rows and
+// nodes past a non-periodic mesh end are left out -- no stencil reaches them).
 // The integer sums do not depend on the order of the reductions.
 template <int ORDER, class Values>
 __device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, Values&& values, int i_lo, int i_hi,
@@ -366,8 +372,7 @@ __device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, Values&& value
     // nodes of a row before the periodic wrap or the mesh end along k
     const int gk0 = node_global(mp, tp, 2, ob[2], 0);
     const int n0 = mp.periodic[2] ? min(e2, tp.nb[2] - ob[2]) : min(e2, mp.ext[2] - gk0);
-    const bool wraps = mp.periodic[2] && n0 < e2;
-    const int gk1 = wraps ? node_global(mp, tp, 2, ob[2], n0) : 0;
+    const int nk = mp.periodic[2] ? e2 : n0;  // nodes of a row to add
     for (int r0 = 0; r0 < rows; r0 += per) {
         const int nr = min(per, rows - r0);
         if (r0 > 0) {  // the previous group's rows have been read
@@ -403,8 +408,9 @@ __device__ __forceinline__ void flush_rows_bulk(const P2GArgs& A, Values&& value
                 continue;
             const long long* src = buf + (size_t)q * e2 * 4;
             if (n0 > 0) bulk_add_u64(A.gm.ptr<long long>(gi, gj, gk0, 0), src, n0 * 32);
-            if (wraps)
-                bulk_add_u64(A.gm.ptr<long long>(gi, gj, gk1, 0), src + 4 * n0, (e2 - n0) * 32);
+            for (int k = n0; k < nk; k += tp.nb[2])
+                bulk_add_u64(A.gm.ptr<long long>(gi, gj, mp.own_lo[2], 0), src + 4 * k,
+                             min(nk - k, tp.nb[2]) * 32);
         }
         bulk_commit();
     }
