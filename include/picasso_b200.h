@@ -231,7 +231,11 @@ PICASSO_API picasso_status picasso_apic_g2p(const picasso_spline* sd, int64_t nu
  * library documentation for its definition.  u_p is the 8 (27) x 3 velocity
  * mode matrix defining the affine material motion, c_p the 8 (27) x ncomp
  * field modes (u_p == c_p when the field is the velocity).  Adds into mu_i
- * and m_i. */
+ * and m_i.  With exec->bins the collocated FP32 form counts particles that have
+ * left the tile they were sorted into (exec->error_count) instead of adding
+ * them, if the bins' chunk is at most 65536 and a tile of 12 (1 + ncomp) bytes
+ * per node, next to 41 KB, fits in shared memory; other bins only tell that the
+ * particles are sorted. */
 PICASSO_API picasso_status picasso_polypic_p2g(const picasso_spline* sd, int64_t num_particles,
                                    int32_t ncomp, picasso_particle_field x_p,
                                    picasso_particle_field m_p, picasso_particle_field u_p,

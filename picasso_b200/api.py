@@ -407,8 +407,11 @@ class PolyPIC:
     def p2g(m_p, u_p, c_p, mu_i, m_i, dt, sd, stream=None, error_count=None, bins=None,
             overflow_count=None):
         """PolyPIC::p2g(m_p, u_p, c_p, mu_i, m_i, dt, sd) -- field before mass.
-        With bins (cell-sorted particles) the FP32 form counts particles that
-        have left the tile they were sorted into instead of adding them."""
+        With bins (cell-sorted particles) the collocated FP32 form counts
+        particles that have left the tile they were sorted into instead of
+        adding them, if the bins have work items of at most 65536 particles
+        and a tile of 12 (1 + ncomp) bytes per node, next to 41 KB, fits in
+        shared memory; other bins only tell the particles' order."""
         ncomp = c_p.shape[2]
         _check_grid_extent(m_i, sd.desc.mesh)
         _check_grid_extent(mu_i, sd.desc.mesh)

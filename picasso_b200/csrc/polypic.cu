@@ -10,6 +10,7 @@
 //   c_r = sum_i w_i s_r(r_i) u_i / sum_i w_i s_r(r_i)^2
 // (for linear splines these reduce to w and dw/dx, PolyPIC.hpp:269-284).
 #include "common.cuh"
+#include "g2p_f64.cuh"
 #include "tiled.cuh"
 #include "transfer.cuh"
 
@@ -27,10 +28,16 @@ __host__ __device__ __forceinline__ constexpr int mode_deg(int r, int d)
                   (2 * r)) & 3ull);
 }
 
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// (Here and in inverse3 every rounding is written out: the kernels of the fixed-point
+// P2G have to agree in every bit, and a sum of two products can be fused in two ways.)
 template <class R>
 __device__ __forceinline__ R quad_alpha(R p, R h)
 {
-    return p * (h * h - R(4) * p * p) / (h * h);
+    const R hh = mul_rn(h, h);
+    return mul_rn(p, fma(R(-4) * p, p, hh)) / hh;
 }
 
 // a[i] for a register array and a run-time i (a select chain, no local memory).
@@ -54,18 +61,34 @@ __device__ __forceinline__ R mode1d(int deg, R r, R h, R alpha)
 template <class R>
 __device__ __forceinline__ void inverse3(const R a[9], R inv[9])
 {
-    const R det = a[0] * a[4] * a[8] + a[1] * a[5] * a[6] + a[2] * a[3] * a[7] -
-                  a[2] * a[4] * a[6] - a[1] * a[3] * a[8] - a[0] * a[5] * a[7];
-    const R r = R(1) / det;
-    inv[0] = (a[4] * a[8] - a[5] * a[7]) * r;
-    inv[1] = (a[2] * a[7] - a[1] * a[8]) * r;
-    inv[2] = (a[1] * a[5] - a[2] * a[4]) * r;
-    inv[3] = (a[5] * a[6] - a[3] * a[8]) * r;
-    inv[4] = (a[0] * a[8] - a[2] * a[6]) * r;
-    inv[5] = (a[2] * a[3] - a[0] * a[5]) * r;
-    inv[6] = (a[3] * a[7] - a[4] * a[6]) * r;
-    inv[7] = (a[1] * a[6] - a[0] * a[7]) * r;
-    inv[8] = (a[0] * a[4] - a[1] * a[3]) * r;
+    auto minor = [&](int p, int q, int r, int s) { return fma(a[p], a[q], -mul_rn(a[r], a[s])); };
+    const R c0 = minor(4, 8, 5, 7), c1 = minor(5, 6, 3, 8), c2 = minor(3, 7, 4, 6);
+    const R r = R(1) / fma(a[0], c0, fma(a[1], c1, mul_rn(a[2], c2)));
+    inv[0] = c0 * r;
+    inv[1] = minor(2, 7, 1, 8) * r;
+    inv[2] = minor(1, 5, 2, 4) * r;
+    inv[3] = c1 * r;
+    inv[4] = minor(0, 8, 2, 6) * r;
+    inv[5] = minor(2, 3, 0, 5) * r;
+    inv[6] = c2 * r;
+    inv[7] = minor(1, 6, 0, 7) * r;
+    inv[8] = minor(0, 4, 1, 3) * r;
+}
+
+// The P2G's spline: eval_spline, in FP64 with the weights of g2p_spline.
+template <int ORDER, class R>
+__device__ __forceinline__ void pp_spline(double x, double lo, double dx, double rdx,
+                                          Spline1D<ORDER, R>& sp)
+{
+    if constexpr (std::is_same<R, double>::value) {
+        double dist0;
+        g2p_spline<ORDER>(x, lo, dx, rdx, sp.s0, sp.w, dist0);
+#pragma unroll
+        for (int n = 0; n < SplineTraits<ORDER>::K; ++n)
+            sp.d[n] = __dsub_rn(fma((double)(sp.s0 + n), dx, lo), x);
+    } else {
+        eval_spline<ORDER>(x, lo, dx, rdx, sp);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -87,7 +110,7 @@ __device__ __forceinline__ void inverse3(const R a[9], R inv[9])
 // order, nor on how they are cut into segments and streams.
 //
 // With the bins of cell-sorted particles, one that is not in the tile it was sorted
-// into is counted instead, as the G2P does.
+// into is counted instead, as the G2P does (where polypic_tiles takes the bins).
 //
 // Bound: quadratic, the shared-memory wavefronts of the coefficients (81 values are
 // read once per lane group and particle: 64 % of the pipe in FP32, 70 % in FP64)
@@ -308,7 +331,7 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
                 bool ok = true;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
-                    eval_spline<ORDER>(x.get<double>(p, d), mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
+                    pp_spline<ORDER>(x.get<double>(p, d), mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
                     ok = stencil_start<K>(mp, d, sp[d].s0, st[d]) && ok;
                 }
                 int64_t t_lo = 0, t_hi = n;  // particles sorted into its tile
@@ -330,10 +353,9 @@ polypic_p2g_kernel(MeshP mp, TileP tp, int64_t n, int64_t seg, PField x, PField 
 #pragma unroll
                     for (int q = 0; q < 3; ++q)
 #pragma unroll
-                        for (int r = 0; r < 3; ++r) {
-                            const R v = dt * (R)u.get<PT>(p, (1 + q) * 3 + r);
-                            am[3 * q + r] = (q == r) ? R(1) + v : v;
-                        }
+                        for (int r = 0; r < 3; ++r)
+                            am[3 * q + r] =
+                                fma(dt, (R)u.get<PT>(p, (1 + q) * 3 + r), R(q == r ? 1 : 0));
                     inverse3(am, ai);
 #pragma unroll
                     for (int q = 0; q < 9; ++q) e[q] = ai[q];
@@ -491,8 +513,8 @@ struct WarpRecords {
 };
 
 // Spline and stencil indices of a particle on the whole local mesh (periodic
-// wrap, bounds check): the placement of the plain kernels.
-template <int ORDER, class R>
+// wrap, bounds check): the placement of the plain kernels.  STREAM: pp_spline's.
+template <int ORDER, class R, bool STREAM = false>
 struct MeshPlace {
     const MeshP& mp;
     __device__ __forceinline__ bool operator()(const double xp[3], Spline1D<ORDER, R> sp[3],
@@ -501,7 +523,8 @@ struct MeshPlace {
         bool ok = true;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            eval_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
+            if constexpr (STREAM) pp_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
+            else eval_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], sp[d]);
             ok = ok && resolve_stencil<SplineTraits<ORDER>::K>(mp, d, sp[d].s0, idx[d]);
         }
         return ok;
@@ -511,12 +534,15 @@ struct MeshPlace {
 // One particle.  place(xp, sp, idx) evaluates the spline and the stencil's
 // grid indices (false: skip the particle); acc(f, i, j, k, v) adds v to grid
 // field f (0 mass, 1 + d momentum component d); mode(v) returns c_p value v
-// (element v of the particle's record).
-template <int ORDER, int NC, bool STAG, class PT, class R, class Place, class Acc, class Mode>
+// (element v of the particle's record).  STREAM: every value in the operations of the
+// streams above, in their order, and times 2^fixed_bits of its field (scale_mu,
+// scale_m), so that a fixed-point grid has the same bits whichever kernel filled it.
+template <int ORDER, int NC, bool STAG, bool STREAM, class PT, class R, class Place, class Acc,
+          class Mode>
 __device__ __forceinline__ void polypic_p2g_particle(const MeshP& mp, int64_t p, const PField& x,
                                                      const PField& m, const PField& u, R dt,
-                                                     int col, int* err, Place&& place, Acc&& acc,
-                                                     Mode&& mode)
+                                                     int col, R scale_mu, R scale_m, int* err,
+                                                     Place&& place, Acc&& acc, Mode&& mode)
 {
     constexpr int K = SplineTraits<ORDER>::K;
     {
@@ -533,10 +559,8 @@ __device__ __forceinline__ void polypic_p2g_particle(const MeshP& mp, int64_t p,
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                const R v = dt * (R)u.get<PT>(p, (1 + a) * 3 + b);
-                am[3 * a + b] = (a == b) ? R(1) + v : v;
-            }
+            for (int b = 0; b < 3; ++b)
+                am[3 * a + b] = fma(dt, (R)u.get<PT>(p, (1 + a) * 3 + b), R(a == b ? 1 : 0));
         inverse3(am, ai);
         R alpha[3] = {R(0), R(0), R(0)};
         R h[3];
@@ -577,24 +601,31 @@ __device__ __forceinline__ void polypic_p2g_particle(const MeshP& mp, int64_t p,
                 for (int j = 0; j < K; ++j)
 #pragma unroll
                     for (int k = 0; k < K; ++k) {
-                        const R wm = mass * wxi * sp[1].w[j] * sp[2].w[k];
+                        const R wab = mass * wxi * sp[1].w[j];
+                        const R wm = STREAM ? wab * scale_m * sp[2].w[k] : wab * sp[2].w[k];
+                        const R wmu = STREAM ? wab * scale_mu * sp[2].w[k] : wm;
                         const R dist[3] = {dxi, sp[1].d[j], sp[2].d[k]};
-                        // backtracked distance xi = A^-1 d (PolyPIC.hpp:90-106)
-                        R map[3];
-#pragma unroll
-                        for (int q = 0; q < 3; ++q) {
-                            R t = R(0);
-#pragma unroll
-                            for (int v = 0; v < 3; ++v) t += ai[3 * q + v] * dist[v];
-                            map[q] = t;
-                        }
+                        // backtracked distance xi = A^-1 d (PolyPIC.hpp:90-106) and
+                        // its modes
                         R f[3][D];
 #pragma unroll
-                        for (int q = 0; q < 3; ++q)
+                        for (int q = 0; q < 3; ++q) {
+                            f[q][0] = R(1);
+                            if constexpr (STREAM) {
+                                f[q][1] = fma(ai[3 * q + 2], dist[2],
+                                              fma(ai[3 * q + 1], dist[1], ai[3 * q] * dist[0]));
+                                if (ORDER == 2)
+                                    f[q][D - 1] = fma(f[q][1], f[q][1] - alpha[q],
+                                                      -(R(0.25) * h[q] * h[q]));
+                            } else {
+                                R t = R(0);
 #pragma unroll
-                            for (int g = 0; g < D; ++g)
-                                f[q][g] = (ORDER == 1) ? (g == 0 ? R(1) : map[q])
-                                                       : mode1d(g, map[q], h[q], alpha[q]);
+                                for (int v = 0; v < 3; ++v) t += ai[3 * q + v] * dist[v];
+#pragma unroll
+                                for (int g = 1; g < D; ++g)
+                                    f[q][g] = ORDER == 1 ? t : mode1d(g, t, h[q], alpha[q]);
+                            }
+                        }
 #pragma unroll
                         for (int e = 0; e < CB; ++e) {
                             R sa = R(0);
@@ -603,14 +634,19 @@ __device__ __forceinline__ void polypic_p2g_particle(const MeshP& mp, int64_t p,
                                 R sb = R(0);
 #pragma unroll
                                 for (int b = 0; b < D; ++b) {
-                                    R sc = R(0);
+                                    R sc = STREAM ? cp[a][b][0][e] : R(0);
 #pragma unroll
-                                    for (int cc = 0; cc < D; ++cc) sc += f[2][cc] * cp[a][b][cc][e];
-                                    sb += f[1][b] * sc;
+                                    for (int cc = STREAM ? 1 : 0; cc < D; ++cc) {
+                                        if (STREAM) sc = fma(f[2][cc], cp[a][b][cc][e], sc);
+                                        else sc += f[2][cc] * cp[a][b][cc][e];
+                                    }
+                                    if (STREAM) sb = b == 0 ? sc : fma(f[1][b], sc, sb);
+                                    else sb += f[1][b] * sc;
                                 }
-                                sa += f[0][a] * sb;
+                                if (STREAM) sa = a == 0 ? sb : fma(f[0][a], sb, sa);
+                                else sa += f[0][a] * sb;
                             }
-                            acc(1 + d0 + e, gi, idx[1][j], idx[2][k], wm * sa);
+                            acc(1 + d0 + e, gi, idx[1][j], idx[2][k], wmu * sa);
                         }
                         if (d0 == 0) acc(0, gi, idx[1][j], idx[2][k], wm);
                     }
@@ -619,28 +655,30 @@ __device__ __forceinline__ void polypic_p2g_particle(const MeshP& mp, int64_t p,
     }
 }
 
-// FP64 P2G of particles in no known order: one thread per particle, every
-// contribution added to the grid by itself, bound by the L2's additions (108 per
-// quadratic particle, 180 G/s).  In random order a stream of the kernel above moves
-// its stencil with nearly every particle and adds as much, on top of its tables: 1 M
-// particles, quadratic 0.69 to 0.73 ms there and 0.60 here, linear 0.236 and 0.196 ms.
-// Exchanging the sums so that four lanes add a whole node cost more than it saved
-// (quadratic 1.07 ms).  In the order of a cell sort the streams win: quadratic 3 to 14
-// per cell 0.49 and 0.46 ms against 0.68 and 1.56 ms.
-template <int ORDER, int NC, bool STAG>
+// P2G of particles in no known order: one thread per particle, every contribution
+// added to the grid by itself, bound by the L2's additions (108 per quadratic particle,
+// 180 G/s).  In random order a stream of the kernel above moves its stencil with nearly
+// every particle and adds as much, on top of its tables; in the order of a cell sort
+// the streams win (pp_kernel).
+template <int ORDER, int NC, bool STAG, class R, bool FIXED>
 __global__ void __launch_bounds__(128)
 polypic_p2g_plain_kernel(MeshP mp, int64_t n, PField x, PField m, PField u, PField c, GField gmu,
-                   GField gm, double dt, int col, int* err)
+                         GField gm, R dt, int col, R scale_mu, R scale_m, int* err)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    const MeshPlace<ORDER, double> place{mp};
+    const MeshPlace<ORDER, R, FIXED> place{mp};
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
-        polypic_p2g_particle<ORDER, NC, STAG, double, double>(
-            mp, p, x, m, u, dt, col, err, place,
-            [&](int f, int i, int j, int k, double v) {
-                atomicAdd(f == 0 ? gm.ptr<double>(i, j, k, 0) : gmu.ptr<double>(i, j, k, f - 1), v);
+        polypic_p2g_particle<ORDER, NC, STAG, FIXED, R, R>(
+            mp, p, x, m, u, dt, col, scale_mu, scale_m, err, place,
+            [&](int f, int i, int j, int k, R v) {
+                if constexpr (FIXED)
+                    atomicAdd(f == 0 ? gm.ptr<unsigned long long>(i, j, k, 0)
+                                     : gmu.ptr<unsigned long long>(i, j, k, f - 1),
+                              (unsigned long long)to_fixed(f == 0 ? gm : gmu, v));
+                else
+                    atomicAdd(f == 0 ? gm.ptr<double>(i, j, k, 0) : gmu.ptr<double>(i, j, k, f - 1), v);
             },
-            [&](int v) { return c.get<double>(p, v); });
+            [&](int v) { return c.get<R>(p, v); });
 }
 
 // ---------------------------------------------------------------------------
@@ -832,6 +870,94 @@ __device__ __forceinline__ void count_unsorted(const TileP& tp, int64_t n, int* 
     }
 }
 
+// P2G of sparse cell-sorted sets: the contributions of an item, rounded to fixed point,
+// are summed in a shared-memory node tile with 32-bit integer atomics, either on three
+// slices of each value (q = hi 2^32 + mid 2^16 + lo with mid, lo in [0, 2^16): the lo
+// and mid sums of at most 65536 contributions are exact, the hi sum is exact modulo
+// 2^32) or on two words (the low word's carries, read from the atomics' old values,
+// added to the high word), so that the recombined 64-bit total is the sum modulo 2^64;
+// then the tile is added to the grid, with one grid atomic per touched node and field.
+template <int ORDER, int NC>
+__global__ void __launch_bounds__(128, ORDER == 2 ? 3 : 1)
+polypic_p2g_tiled_kernel(MeshP mp, TileP tp, int64_t n, PField x, PField m, PField u, PField c,
+                         GField gmu, GField gm, float dt, float scale_mu, float scale_m, int* err)
+{
+    extern __shared__ __align__(16) unsigned int pp_tacc[];  // 2 or 3 slices x (1 + NC) x nodes
+    count_unsorted(tp, n, err);
+    int64_t t, a, b;
+    if (!item_range(tp, blockIdx.x, t, a, b)) return;  // CTA-uniform
+    // Linear: two words (128^3 8 per cell 2.11 -> 1.52 ms); quadratic, where a run per
+    // thread leaves few conflicts: three slices without returned values (the returning
+    // atomic measured 6.20 -> 7.27 ms there).
+    constexpr bool TWO = ORDER == 1;
+    const int nodes = tp.nodes, slice = (1 + NC) * nodes;
+    for (int e = threadIdx.x; e < (TWO ? 2 : 3) * slice; e += blockDim.x) pp_tacc[e] = 0u;
+    __syncthreads();
+    int ob[3];
+    tile_origin(tp, t, ob);
+    const TilePlace<ORDER> place{mp, tp, ob};
+    // Quadratic: each thread sweeps its own contiguous run of the item, so that the lanes
+    // of a warp sit in different cells.  Linear (8 nodes, little arithmetic) keeps
+    // consecutive particles per warp for coalesced loads.
+    const int64_t U = ORDER == 2 ? (b - a + blockDim.x - 1) / blockDim.x : 1;
+    const int64_t r0 = a + (int64_t)threadIdx.x * U;
+    const int64_t r1 = ORDER == 2 ? min(r0 + U, b) : b;
+    const int64_t step = ORDER == 2 ? 1 : blockDim.x;
+    for (int64_t p = r0; p < r1; p += step)
+        polypic_p2g_particle<ORDER, NC, false, true, float, float>(
+            mp, p, x, m, u, dt, -1, scale_mu, scale_m, err, place,
+            [&](int f, int i, int j, int k, float v) {
+                const unsigned long long q = (unsigned long long)to_fixed(f == 0 ? gm : gmu, v);
+                const int e = f * nodes + (i * tp.NT[1] + j) * tp.NT[2] + k;
+                if constexpr (TWO) {
+                    const unsigned lo = (unsigned)q;
+                    const unsigned old = atomicAdd(&pp_tacc[e], lo);
+                    const unsigned hi = (unsigned)(q >> 32) + (old + lo < old ? 1u : 0u);
+                    if (hi) atomicAdd(&pp_tacc[slice + e], hi);
+                } else {
+                    atomicAdd(&pp_tacc[e], (unsigned)(q & 0xFFFF));
+                    atomicAdd(&pp_tacc[slice + e], (unsigned)((q >> 16) & 0xFFFF));
+                    atomicAdd(&pp_tacc[2 * slice + e], (unsigned)(q >> 32));
+                }
+            },
+            [&](int v) { return c.get<float>(p, v); });
+    __syncthreads();
+    for (int e = threadIdx.x; e < nodes; e += blockDim.x) {
+        const int k = e % tp.NT[2], j = (e / tp.NT[2]) % tp.NT[1], i = e / (tp.NT[1] * tp.NT[2]);
+        const int gi = node_global(mp, tp, 0, ob[0], i);
+        const int gj = node_global(mp, tp, 1, ob[1], j);
+        const int gk = node_global(mp, tp, 2, ob[2], k);
+#pragma unroll
+        for (int f = 0; f <= NC; ++f) {
+            const int q = f * nodes + e;
+            const unsigned long long v =
+                TWO ? ((unsigned long long)pp_tacc[slice + q] << 32) + (unsigned long long)pp_tacc[q]
+                    : ((unsigned long long)pp_tacc[2 * slice + q] << 32) +
+                          ((unsigned long long)pp_tacc[slice + q] << 16) +
+                          (unsigned long long)pp_tacc[q];
+            if (v)
+                atomicAdd(f == 0 ? gm.ptr<unsigned long long>(gi, gj, gk, 0)
+                                 : gmu.ptr<unsigned long long>(gi, gj, gk, f - 1),
+                          v);
+        }
+    }
+}
+
+template <int ORDER, int NC>
+static picasso_status launch_pp_p2g_tiled(const MeshP& mp, const TileP& tp, int64_t n,
+                                          const PField& x, const PField& m, const PField& u,
+                                          const PField& c, const GField& gmu, const GField& gm,
+                                          double dt, int* err, cudaStream_t st)
+{
+    const size_t smem = (ORDER == 1 ? 2 : 3) * sizeof(unsigned) * (1 + NC) * (size_t)tp.nodes;
+    auto kern = polypic_p2g_tiled_kernel<ORDER, NC>;
+    PB_CUDA_TRY(allow_smem(kern, smem));
+    kern<<<(unsigned)item_bound(tp), 128, smem, st>>>(mp, tp, n, x, m, u, c, gmu, gm, (float)dt,
+                                                      ldexpf(1.f, gmu.fixed_bits),
+                                                      ldexpf(1.f, gm.fixed_bits), err);
+    return check_launch();
+}
+
 // G2P: the tile's node velocities are staged once per item in shared memory;
 // packed c_p records leave through WarpRecords.
 template <int ORDER, int NC, bool WS>
@@ -925,8 +1051,36 @@ static void launch_staged(Kern kernel, bool ws, unsigned blocks, cudaStream_t st
     kernel<<<blocks, 128, smem, st>>>(args...);
 }
 
+// The three P2G kernels: particles in no known order go one per thread; the bins tell
+// that the particles are in the order of their stencils, where streams win unless there
+// is about one particle per stencil.  1 M particles, ms:
+//   without bins, streams / particles: random order FP32 linear 0.178 / 0.169, clustered
+//   0.274 / 0.240, quadratic clustered 0.930 / 0.881; fixed point of FP64 particles
+//   linear 0.217 / 0.199, quadratic 0.785 / 0.587 (only particles that happen to be in
+//   cell order would gain: FP32 linear 8 per cell 0.076 / 0.215);
+//   sorted FP32, streams / tile: linear 1 per cell 0.145 / 0.124, 2 per cell 0.097 /
+//   0.110; quadratic 1 per cell 0.452 / 0.406, 2 per cell 0.330 / 0.354, but 0.1 M of 1
+//   per cell 0.045 / 0.049;
+//   sorted FP64, streams / particles: linear 1 per cell 0.187 / 0.183, 3 per cell 0.151
+//   / 0.205; fixed point 1 per cell linear 0.185 / 0.178, quadratic 0.604 / 0.594, but
+//   clustered 0.159 / 0.560 and 0.577 / 1.69.
+enum class PPKernel { streams, particles, tile };
+
+static PPKernel pp_kernel(int form, int order, int64_t n, const picasso_bins* bins, bool tiled)
+{
+    if (!bins) return PPKernel::particles;
+    double cells = 1.0;
+    for (int d = 0; d < 3; ++d) cells *= bins->bin_extent[d];
+    if (form == 0 && order == 1 && n < 2.0 * cells) return PPKernel::particles;
+    if (tiled && n < 1.5 * cells && (order == 1 || n >= 500000)) return PPKernel::tile;
+    return PPKernel::streams;
+}
+
 // Particles per warp: up to 8 tables (a run's end at a segment's costs as much as
-// a stencil), less when that would not give every SM 16 warps.
+// a stencil), as few as leave the warps in the same number of whole waves: with a rule
+// by the particles alone 1 M linear FP32 particles were 2.2 waves of 8 tables, now 3 of
+// 6 (3 per cell 0.100 -> 0.095 ms; 0.4 M 0.055 -> 0.039 ms; quadratic 0.4 M 0.145 ->
+// 0.131 ms).
 template <int ORDER, int NC, bool STAG, class PT, class R, bool FIXED>
 static picasso_status launch_pp_p2g_form(const MeshP& mp, const TileP& tp, int64_t n, const PField& x,
                                          const PField& m, const PField& u, const PField& c,
@@ -937,9 +1091,14 @@ static picasso_status launch_pp_p2g_form(const MeshP& mp, const TileP& tp, int64
     auto kern = polypic_p2g_kernel<ORDER, NC, STAG, PT, R, FIXED>;
     const size_t smem = kPPWarps * C::kBytes;
     PB_CUDA_TRY(allow_smem(kern, smem));
-    int64_t tables = n / (148 * 16) / C::P;
-    if (tables < 1) tables = 1;
-    if (tables > 8) tables = 8;
+    static const int ctas_per_sm = [&] {
+        int v = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, kern, 32 * kPPWarps, smem);
+        return v > 0 ? v : 1;
+    }();
+    const int64_t slots = (int64_t)148 * kPPWarps * ctas_per_sm * C::P;
+    const int64_t waves = (n + 8 * slots - 1) / (8 * slots);
+    const int64_t tables = (n + waves * slots - 1) / (waves * slots);
     const int64_t seg = tables * C::P;
     const int64_t ctas = (n + seg * kPPWarps - 1) / (seg * kPPWarps);
     kern<<<(unsigned)ctas, 32 * kPPWarps, smem, st>>>(mp, tp, n, seg, x, m, u, c, gmu, gm, dt, col, smu, sm,
@@ -947,16 +1106,38 @@ static picasso_status launch_pp_p2g_form(const MeshP& mp, const TileP& tp, int64
     return check_launch();
 }
 
-template <int ORDER, int NC, bool STAG>
-static picasso_status launch_pp_p2g(int form, bool sorted, const MeshP& mp, const TileP& tp, int64_t n, const PField& x,
-                                    const PField& m, const PField& u, const PField& c,
-                                    const GField& gmu, const GField& gm, double dt, int col, int* err,
-                                    cudaStream_t st)
+template <int ORDER, int NC, bool STAG, class R, bool FIXED>
+static picasso_status launch_pp_p2g_plain(const MeshP& mp, int64_t n, const PField& x, const PField& m,
+                                          const PField& u, const PField& c, const GField& gmu,
+                                          const GField& gm, double dt, int col, int* err,
+                                          cudaStream_t st)
 {
-    if (form == 0 && !sorted) {
-        polypic_p2g_plain_kernel<ORDER, NC, STAG>
-            <<<grid_for(n, 128, 148LL * 128), 128, 0, st>>>(mp, n, x, m, u, c, gmu, gm, dt, col, err);
-        return check_launch();
+    polypic_p2g_plain_kernel<ORDER, NC, STAG, R, FIXED>
+        <<<grid_for(n, 128, 148LL * 128), 128, 0, st>>>(
+            mp, n, x, m, u, c, gmu, gm, (R)dt, col, (R)ldexp(1.0, gmu.fixed_bits),
+            (R)ldexp(1.0, gm.fixed_bits), err);
+    return check_launch();
+}
+
+template <int ORDER, int NC, bool STAG>
+static picasso_status launch_pp_p2g(int form, PPKernel kernel, const MeshP& mp, const TileP& tp,
+                                    int64_t n, const PField& x, const PField& m, const PField& u,
+                                    const PField& c, const GField& gmu, const GField& gm, double dt,
+                                    int col, int* err, cudaStream_t st)
+{
+    if (kernel == PPKernel::particles) {
+        if (form == 0)
+            return launch_pp_p2g_plain<ORDER, NC, STAG, double, false>(mp, n, x, m, u, c, gmu, gm, dt,
+                                                                       col, err, st);
+        if (form == 1)
+            return launch_pp_p2g_plain<ORDER, NC, STAG, float, true>(mp, n, x, m, u, c, gmu, gm, dt,
+                                                                     col, err, st);
+        return launch_pp_p2g_plain<ORDER, NC, STAG, double, true>(mp, n, x, m, u, c, gmu, gm, dt, col,
+                                                                  err, st);
+    }
+    if constexpr (!STAG) {
+        if (kernel == PPKernel::tile)
+            return launch_pp_p2g_tiled<ORDER, NC>(mp, tp, n, x, m, u, c, gmu, gm, dt, err, st);
     }
     if (form == 0)
         return launch_pp_p2g_form<ORDER, NC, STAG, double, double, false>(
@@ -1019,19 +1200,20 @@ static picasso_status polypic_common(const picasso_spline* sd, int64_t n, int32_
 }
 
 // Tiled path for sorted particles (picasso_exec.bins): FP32 form, collocated
-// locations; the bins must match the spline.  *tiled stays false (plain
-// kernels) when not eligible or when the node tile of `node_bytes` per node
-// does not fit in shared memory.
+// locations; the bins must match the spline.  *tiled stays false when not
+// eligible or when the node tile of `node_bytes` per node does not fit in
+// shared memory: then particles that have left the tile they were sorted into
+// are transferred like the others, else they are counted.
 static picasso_status polypic_tiles(const picasso_spline* sd, const picasso_exec* exec, int64_t n,
-                                    bool eligible, const MeshP& mp, int node_bytes, bool* tiled,
-                                    TileP* tp)
+                                    bool eligible, const MeshP& mp, int node_bytes, TileUse use,
+                                    bool* tiled, TileP* tp)
 {
     *tiled = false;
     if (!exec || !exec->bins) return PICASSO_OK;
     if (exec->bins->order != sd->order || exec->bins->location != sd->location)
         return PICASSO_ERR_INVALID_ARGUMENT;
     if (!eligible) return PICASSO_OK;
-    if (!make_tilep(mp, sd->order, *exec->bins, n, tp)) return PICASSO_ERR_INVALID_ARGUMENT;
+    if (!make_tilep(mp, sd->order, *exec->bins, n, tp, use)) return PICASSO_ERR_INVALID_ARGUMENT;
     // records of four warps on top of the node tile in the G2P (at most)
     const int64_t extra = 4 * 32 * 82 * 4;
     if ((int64_t)node_bytes * tp->nodes + extra > device_smem_optin()) return PICASSO_OK;
@@ -1070,28 +1252,26 @@ extern "C" picasso_status picasso_polypic_p2g(const picasso_spline* sd, int64_t 
     gmu.overflow = gm.overflow = exec ? exec->overflow_count : nullptr;
     bool tiled = false;
     TileP tp;
+    // (the tile kernel's 32-bit sums are exact for work items of at most 65536 particles)
     const bool p2g_ok = form == 1 && stag < 0 && exec && exec->bins && exec->bins->chunk <= 65536;
-    if ((st = polypic_tiles(sd, exec, num_particles, p2g_ok, mp, 12 * (1 + ncomp), &tiled, &tp))) return st;
+    if ((st = polypic_tiles(sd, exec, num_particles, p2g_ok, mp, 12 * (1 + ncomp), TileUse::whole,
+                            &tiled, &tp)))
+        return st;
     if (!tiled) tp.off = nullptr;
-    // The bins tell that the particles are in the order of their stencils; with linear
-    // splines and less than two per stencil the streams gain nothing by it (1 M
-    // particles, 1 per cell: 0.187 ms, plain 0.183; 3 per cell 0.151 and 0.205).
-    bool sorted = exec && exec->bins;
-    if (sorted && sd->order == 1) {
-        double stencils = 1.0;
-        for (int d = 0; d < 3; ++d) stencils *= exec->bins->bin_extent[d];
-        sorted = num_particles >= 2 * stencils;
-    }
+    const PPKernel kernel =
+        pp_kernel(form, sd->order, num_particles, exec ? exec->bins : nullptr, tiled);
     if (sd->order == 1) {
         if (stag >= 0) {
-            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, true>(
-                                       form, sorted, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
+            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, true>(form, kernel, mp, tp, num_particles,
+                                                                      x, m, u, c, gmu, gm, dt, col,
+                                                                      err, s));
         } else {
-            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, false>(
-                                       form, sorted, mp, tp, num_particles, x, m, u, c, gmu, gm, dt, col, err, s));
+            PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<1, NC_, false>(form, kernel, mp, tp,
+                                                                       num_particles, x, m, u, c, gmu,
+                                                                       gm, dt, col, err, s));
         }
     }
-    PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<2, NC_, false>(form, sorted, mp, tp, num_particles, x, m, u, c,
+    PB_PP_NC_SWITCH(ncomp, return launch_pp_p2g<2, NC_, false>(form, kernel, mp, tp, num_particles, x, m, u, c,
                                                                gmu, gm, dt, col, err, s));
     return PICASSO_OK;
 }
@@ -1116,7 +1296,7 @@ extern "C" picasso_status picasso_polypic_g2p(const picasso_spline* sd, int64_t 
     GField u = make_gfield(u_i);
     bool tiled = false;
     TileP tp;
-    if ((st = polypic_tiles(sd, exec, num_particles, f32 && stag < 0, mp, 16, &tiled, &tp))) return st;
+    if ((st = polypic_tiles(sd, exec, num_particles, f32 && stag < 0, mp, 16, TileUse::other, &tiled, &tp))) return st;
     if (tiled) {
         if (sd->order == 1) {
             PB_PP_NC_SWITCH(ncomp, return launch_pp_g2p_tiled<1, NC_>(mp, tp, num_particles, x, u,

@@ -191,13 +191,13 @@ bool valid_lanes(int order, int lanes, bool stag)
 // instance has less than 592, into at most 8 parts (24 instances up to 64^3 with the
 // other rule 1.92, so 1.76 ms).  Both are functions of the sizes alone, so that every
 // call on the same bins sums in the same order.
-// The runs of a whole item are 32 already: they are not cut.
+// Runs (32 per item already) and the PolyPIC P2G's tiles are not cut.
 static void set_parts(TileP* tp, int64_t n, TileUse use)
 {
     const int64_t items = tp->ntiles + (n + tp->chunk - 1) / tp->chunk;
     const int64_t few = 148 * 4;
     int64_t part, parts;
-    if (use == TileUse::runs) {
+    if (use == TileUse::runs || use == TileUse::whole) {
         part = tp->chunk;
         parts = 1;
     } else if (use == TileUse::batch_streams || use == TileUse::batch_other) {

@@ -1155,8 +1155,9 @@ __device__ void g2p_item(const G2PArgs& A, int64_t t, int64_t a, int64_t b, floa
 // host helpers (tiled.cu)
 bool fused_update_fits(const TileP& tp, int order);
 // What a tile is made for: `streams` and `runs` set the strides of the P2G's node tile
-// (p2g_item, run_p2g_item); a batch's items are cut by a rule of their own (set_parts).
-enum class TileUse { other, streams, batch_streams, runs, batch_other };
+// (p2g_item, run_p2g_item); a batch's items are cut by a rule of their own, those of
+// `whole` and `runs` not at all (set_parts).
+enum class TileUse { other, whole, streams, runs, batch_other, batch_streams };
 bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n, TileP* tp,
                 TileUse use = TileUse::other);
 int64_t item_bound(const TileP& tp);  // parts of all items, at most
