@@ -59,20 +59,28 @@ apic_g2p_tiled_f64_kernel(MeshP mp, TileP tp, int64_t n, PField x, GField u, PFi
     using R = WarpRows<3, ADV>;
     extern __shared__ __align__(16) double g2p_nodes[];  // 3 per tile node
     __shared__ double rows[4][R::DOUBLES];
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5;
     int64_t t, a, b;
     if (item_range(tp, blockIdx.x, t, a, b)) {
         b = min(b, n);
         if (a < b)
             g2p_item_f64<ORDER, 128, false, ADV>(mp, tp, t, a, b, x, u, c, err, &adv, g2p_nodes,
-                                                       packed ? rows[0] : nullptr, tid);
+                                                 packed ? rows[0] : nullptr, tid);
     }
-    const int64_t rest = __ldg(tp.off + tp.ntiles) + (int64_t)blockIdx.x * 128 + tid;
-    for (int64_t p = rest; p < n; p += (int64_t)gridDim.x * 128) {
-        const double xp[3] = {x.get<double>(p, 0), x.get<double>(p, 1), x.get<double>(p, 2)};
-        double up[3], B[3][3];
-        if (g2p_stray<ORDER, false>(mp, xp, u, up, B)) g2p_set<ADV>(p, xp, up, B, x, c, &adv);
-        else if (err) atomicAdd(err, 1);
+    // (32 particles per warp; their rows go through the warp's buffer)
+    for (int64_t p0 = __ldg(tp.off + tp.ntiles) + (int64_t)blockIdx.x * 128 + warp * 32; p0 < n;
+         p0 += (int64_t)gridDim.x * 128) {
+        const int64_t p = p0 + (tid & 31);
+        bool ok = p < n;
+        double xp[3] = {0.0, 0.0, 0.0}, up[3], B[3][3];
+        if (ok) {
+#pragma unroll
+            for (int d = 0; d < 3; ++d) xp[d] = x.get<double>(p, d);
+            ok = g2p_stray<ORDER, false>(mp, xp, u, up, B);
+            if (!ok && err) atomicAdd(err, 1);
+        }
+        g2p_store<3, false, ADV>(p0, tid & 31, ok, xp, up, B, x, c, -1, &adv,
+                                 packed ? rows[warp] : nullptr);
     }
 }
 
@@ -169,8 +177,11 @@ static void launch_g2p(bool f32, const MeshP& mp, int64_t n, const PField& x, co
         mp, n, x, u, c, stag, err, a);
 }
 
-// FP64 G2P with bins (3 collocated components); *handled stays false when the
-// node tile does not fit in shared memory.
+// FP64 G2P with bins (3 collocated components); *handled stays false where gathering
+// from global memory is faster: g2p_tiles_pay, and sets that leave the tiles' CTAs about
+// a wave (tile / global memory, sorted, 8 per cell, ms: quadratic 0.15 M 0.019 / 0.013,
+// 0.5 M 0.035 / 0.031, 1 M 0.063 / 0.066, 2 M 0.104 / 0.120; cubic 0.5 M 0.052 / 0.054,
+// 1 M 0.084 / 0.107).
 template <int ORDER>
 static picasso_status launch_g2p_tiled_f64(const MeshP& mp, const TileP& tp, int64_t n,
                                            const PField& x, const GField& u, const PField& c,
@@ -181,6 +192,7 @@ static picasso_status launch_g2p_tiled_f64(const MeshP& mp, const TileP& tp, int
     const size_t rows = 4 * sizeof(double) * (size_t)(adv ? WarpRows<3, true>::DOUBLES
                                                           : WarpRows<3, false>::DOUBLES);
     if ((int64_t)(smem + rows) > device_smem_optin()) return PICASSO_OK;
+    if (n < (ORDER == 3 ? 1000000 : 1500000) || !g2p_tiles_pay(tp, ORDER, n)) return PICASSO_OK;
     *handled = true;
     const bool packed = packed_rows_f64(x, c, 12, adv != nullptr);
     const int64_t items = item_bound(tp);

@@ -53,7 +53,7 @@ struct BInst {
     double thr, inv_m, inv_mu;
     int64_t n;
     int order;
-    int g2p_tile;  // FP64: the node tile fits in shared memory
+    int g2p_tile;  // FP64: the G2P stages node tiles
     uint32_t nitems[kPhases];
 };
 
@@ -183,8 +183,8 @@ static int warp_p2g_bytes(int order)
 }
 
 // FP64 G2P item; smem: a WarpRows buffer per warp, then the node tile
-// (g2p_item_f64).  An instance whose tile does not fit in shared memory gathers from
-// global memory (apic_g2p_warp).  CG: u_i was written in this launch.
+// (g2p_item_f64).  An instance whose tiles do not fit in shared memory, or do not pay,
+// gathers from global memory (apic_g2p_warp).  CG: u_i was written in this launch.
 constexpr int kWarpG2PBytes = WarpRows<3, false>::DOUBLES * (int)sizeof(double);
 
 template <int ORDER, int NT, bool CG>
@@ -553,7 +553,8 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
     } else {
         *smem_p2g = std::max(*smem_p2g, warp_p2g_bytes(order));  // one warp's
         const int64_t tile = 3 * (int64_t)sizeof(double) * tp.nodes;
-        I->g2p_tile = tile + kF64Warps * kWarpG2PBytes <= device_smem_optin();
+        I->g2p_tile = tile + kF64Warps * kWarpG2PBytes <= device_smem_optin() &&
+                      g2p_tiles_pay(tp, order, in.num_particles);
         if (I->g2p_tile) *smem_g2p = std::max(*smem_g2p, (int)tile);
     }
     return PICASSO_OK;

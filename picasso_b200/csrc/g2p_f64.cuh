@@ -14,8 +14,9 @@
 //   * particles in any order read u_i from global memory, in the order of their
 //     stencils inside a warp where they have little locality (64^3 cells of 8:
 //     0.214 ms as they come, 0.167 ms ordered, 90 % of the L1 data pipe);
-//   * cell-sorted particles (bins) read it from a node tile in shared memory
-//     (128^3 8 per cell clustered: 0.92 ms from global memory, 0.71 ms).
+//   * large dense sets of cell-sorted particles (bins; g2p_tiles_pay) read it from a
+//     node tile in shared memory (128^3 8 per cell clustered: 0.92 ms from global
+//     memory, 0.71 ms).
 // Against the form it replaces (node by node, every thread storing its row):
 // sorted quadratic 128^3 1.28 -> 0.71 ms, cubic with advection 64^3 0.44 -> 0.17
 // ms, unsorted quadratic 64^3 0.224 -> 0.165 ms, the faces of a 45 x 38 x 53 box
@@ -184,10 +185,42 @@ __device__ __forceinline__ void g2p_store(int64_t p0, int at, bool ok, const dou
     }
 }
 
-// Particles p0 .. p0 + cnt - 1 (cnt <= 32) by a whole warp.  CG: u_i is read
-// through L2 only (written earlier in the same launch).  UNIT: the components of
-// u_i are adjacent.  ORDERED: the particles come in the order of their stencils.
-// rows: see g2p_store.
+// u_p and B_p of a particle at xp gathered from u_i in global memory.  False (counted in
+// err) if the stencil leaves a non-periodic mesh.  CG: u_i is read through L2 only
+// (written earlier in the same launch).  UNIT: the components of u_i are adjacent.
+template <int ORDER, int NU, bool CG, bool UNIT>
+__device__ __forceinline__ bool g2p_gather(const MeshP& mp, const double (&xp)[3], const GField& u,
+                                           int* err, double (&up)[NU], double (&B)[NU][3])
+{
+    constexpr int K = SplineTraits<ORDER>::K;
+    double w[3][K], dist0[3];
+    int idx[3][K];
+    bool ok = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        int s0;
+        g2p_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], s0, w[d], dist0[d]);
+        ok = resolve_stencil<K>(mp, d, s0, idx[d]) && ok;
+    }
+    if (!ok) {
+        if (err) atomicAdd(err, 1);
+        return false;
+    }
+    int64_t nk[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) nk[k] = (int64_t)idx[2][k] * u.s[2];
+    const int64_t sc = UNIT ? 1 : u.s[3];
+    g2p_contract<ORDER, NU>(mp, w, dist0, up, B, [&](int i, int j, int k, int d) {
+        const double* a = reinterpret_cast<const double*>(u.data) +
+                          (int64_t)idx[0][i] * u.s[0] +
+                          (int64_t)idx[1][j] * u.s[1] + nk[k] + d * sc;
+        return CG ? __ldcg(a) : __ldg(a);
+    });
+    return true;
+}
+
+// Particles p0 .. p0 + cnt - 1 (cnt <= 32) by a whole warp, gathered from global memory.
+// ORDERED: the particles come in the order of their stencils.  rows: see g2p_store.
 template <int ORDER, int NC, bool STAG, bool CG, bool ADV, bool UNIT, bool ORDERED>
 __device__ __forceinline__ void apic_g2p_warp(const MeshP& mp, int64_t p0, int cnt, const PField& x,
                                               const GField& u, const PField& c, int stag, int* err,
@@ -217,31 +250,11 @@ __device__ __forceinline__ void apic_g2p_warp(const MeshP& mp, int64_t p0, int c
                                       ((unsigned)s[0] * (unsigned)mp.ext[1] + (unsigned)s[1]) *
                                               (unsigned)mp.ext[2] + (unsigned)s[2]) & 31;
     }
-    const int64_t p = p0 + at;
     double up[NU], B[NU][3], xp[3] = {0.0, 0.0, 0.0};
     if (ok) {
-        double w[3][K], dist0[3];
-        int idx[3][K];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            int s0;
-            xp[d] = x.get<double>(p, d);
-            g2p_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], s0, w[d], dist0[d]);
-            ok = resolve_stencil<K>(mp, d, s0, idx[d]) && ok;
-        }
-        if (!ok && err) atomicAdd(err, 1);
-        if (ok) {
-            int64_t nk[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) nk[k] = (int64_t)idx[2][k] * u.s[2];
-            const int64_t sc = UNIT ? 1 : u.s[3];
-            g2p_contract<ORDER, NU>(mp, w, dist0, up, B, [&](int i, int j, int k, int d) {
-                const double* a = reinterpret_cast<const double*>(u.data) +
-                                  (int64_t)idx[0][i] * u.s[0] + (int64_t)idx[1][j] * u.s[1] + nk[k] +
-                                  d * sc;
-                return CG ? __ldcg(a) : __ldg(a);
-            });
-        }
+        for (int d = 0; d < 3; ++d) xp[d] = x.get<double>(p0 + at, d);
+        ok = g2p_gather<ORDER, NU, CG, UNIT>(mp, xp, u, err, up, B);
     }
     g2p_store<NC, STAG, ADV>(p0, at, ok, xp, up, B, x, c, stag, adv, rows);
 }
@@ -255,9 +268,14 @@ struct NodeTile {
     int i_lo, i_hi;  // bin rows staged
 };
 
-// u_p and B_p of one particle at xp gathered node by node from global memory,
-// in rolled loops: for the few particles that are not in the tile they were
-// sorted into.  False if the stencil leaves a non-periodic mesh.
+// u_p and B_p of one particle at xp gathered from global memory, the rows of its stencil
+// in a loop (the same operations as g2p_contract, in few registers): for the particles
+// that are not in the tile they were sorted into.  False if the stencil leaves a
+// non-periodic mesh.  (A row at a time, its values in flight together; node by node
+// quadratic sets of 8 per cell that had drifted since the sort took 1.6 times as long: 5 M
+// drifted by 0.1 cells 0.75 ms, now 0.46, from global memory alone 0.32; as a loop of its
+// own over the warps concerned, or with g2p_contract, the tile's gather spills and sorted
+// sets lose 5 to 40 %.)
 template <int ORDER, bool CG>
 __device__ __forceinline__ bool g2p_stray(const MeshP& mp, const double xp[3], const GField& u,
                                           double (&up)[3], double (&B)[3][3])
@@ -267,50 +285,60 @@ __device__ __forceinline__ bool g2p_stray(const MeshP& mp, const double xp[3], c
     double w[3][K], dist0[3];
     int idx[3][K];
     bool ok = true;
+#pragma unroll
     for (int d = 0; d < 3; ++d) {
         int s0;
         g2p_spline<ORDER>(xp[d], mp.lo[d], mp.dx[d], mp.rdx[d], s0, w[d], dist0[d]);
         ok = resolve_stencil<K>(mp, d, s0, idx[d]) && ok;
     }
     if (!ok) return false;
+    double M[3][3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) up[d] = B[d][0] = B[d][1] = B[d][2] = 0.0;
+    for (int d = 0; d < 3; ++d) up[d] = M[d][0] = M[d][1] = M[d][2] = 0.0;
+    double A0[3] = {0.0, 0.0, 0.0}, A1[3] = {0.0, 0.0, 0.0}, A2[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
-    for (int e = 0; e < K * K * K; ++e) {
-        const int n[3] = {e / (K * K), e / K % K, e % K};
-        const double wn = w[0][n[0]] * w[1][n[1]] * w[2][n[2]];
+    for (int e = 0; e < K * K; ++e) {
+        const int i = e / K, j = e - i * K;
+        const double* row = reinterpret_cast<const double*>(u.data) +
+                            (int64_t)select<K>(idx[0], i) * u.s[0] + (int64_t)select<K>(idx[1], j) * u.s[1];
+        double v[K][3];
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const double* a = row + (int64_t)idx[2][k] * u.s[2] + d * u.s[3];
+                v[k][d] = CG ? __ldcg(a) : __ldg(a);
+            }
+        const double wy = select<K>(w[1], j), wj = wy * (double)(j - N0);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            const double* a = u.ptr<double>(idx[0][n[0]], idx[1][n[1]], idx[2][n[2]], d);
-            const double wu = wn * (CG ? __ldcg(a) : __ldg(a));
-            up[d] += wu;
+            double S0 = 0.0, S1 = 0.0;
 #pragma unroll
-            for (int q = 0; q < 3; ++q) B[d][q] = fma(wu, mp.dx[q] * (n[q] - N0), B[d][q]);
+            for (int k = 0; k < K; ++k) {
+                S0 = fma(w[2][k], v[k][d], S0);
+                if (k != N0) S1 = fma(w[2][k] * (double)(k - N0), v[k][d], S1);
+            }
+            A0[d] = fma(wy, S0, A0[d]);
+            if (j != N0) A1[d] = fma(wj, S0, A1[d]);
+            A2[d] = fma(wy, S1, A2[d]);
+        }
+        if (j == K - 1) {
+            const double wx = select<K>(w[0], i), wi = wx * (double)(i - N0);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                up[d] = fma(wx, A0[d], up[d]);
+                if (i != N0) M[d][0] = fma(wi, A0[d], M[d][0]);
+                M[d][1] = fma(wx, A1[d], M[d][1]);
+                M[d][2] = fma(wx, A2[d], M[d][2]);
+                A0[d] = A1[d] = A2[d] = 0.0;
+            }
         }
     }
 #pragma unroll
     for (int d = 0; d < 3; ++d)
 #pragma unroll
-        for (int q = 0; q < 3; ++q) B[d][q] = fma(dist0[q], up[d], B[d][q]);
+        for (int q = 0; q < 3; ++q) B[d][q] = fma(mp.dx[q], M[d][q], __dmul_rn(dist0[q], up[d]));
     return true;
-}
-
-// Results of one particle to its own row.
-template <bool ADV>
-__device__ __forceinline__ void g2p_set(int64_t p, const double xp[3], const double (&up)[3],
-                                        const double (&B)[3][3], const PField& x, const PField& c,
-                                        const Advect* adv)
-{
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        c.set<double>(p, d, up[d]);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) c.set<double>(p, (1 + q) * 3 + d, B[d][q]);
-    }
-    if constexpr (ADV) {
-        const double uo[3] = {up[0], up[1], up[2]};
-        advect_particle(*adv, p, xp, uo, [&](int d, double v) { x.set<double>(p, d, v); });
-    }
 }
 
 // Particles p0 .. p0 + cnt - 1 of a tile, three components, by a whole warp:
@@ -423,6 +451,21 @@ __device__ __forceinline__ void g2p_item_f64(const MeshP& mp, const TileP& tp, i
     for (int64_t p0 = a + (tid & ~31); p0 < b; p0 += NTHR)
         g2p_tile_warp<ORDER, CG, ADV>(mp, nt, p0, (int)min((int64_t)32, b - p0), x, u, c, err, adv,
                                       mine);
+}
+
+// Whether the bins' node tiles pay against gathering from global memory: enough particles
+// per staged node, and tiles small enough for 4 CTAs on an SM.  2 M sorted particles,
+// tile / global memory, ms: linear tile (4, 8, 8) 8 per cell 0.077 / 0.084 and 4 per cell
+// (2.5 per node) 0.084 / 0.084; quadratic 4 per cell (1.7) 0.107 / 0.123, 2 per cell
+// 0.137 / 0.139, 1 per cell 0.211 / 0.164, tile (4, 4, 8) 4 per cell (1.4) 0.121 / 0.122,
+// (2, 2, 2) 1 per cell 1.98 / 0.17; cubic 2 per cell (0.6) 0.197 / 0.219, tile (4, 4, 8)
+// 2 per cell (0.5) 0.230 / 0.218; (8, 16, 16), 2 CTAs, 8 per cell, quadratic 0.176 /
+// 0.121.
+inline bool g2p_tiles_pay(const TileP& tp, int order, int64_t n)
+{
+    const double per_node = (double)n / ((double)tp.ntiles * tp.nodes);
+    return 3 * sizeof(double) * (size_t)tp.nodes <= 40 * 1024 &&
+           per_node >= (order == 1 ? 4.5 : order == 2 ? 1.5 : 0.55);
 }
 
 // c_p (ncv values per particle) and, with adv, x_p are packed rows.
