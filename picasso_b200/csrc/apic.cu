@@ -102,12 +102,13 @@ apic_p2g_warp_kernel(MeshP mp, int64_t n, int64_t seg, PField x, PField m, PFiel
 }
 
 // Particles per warp: 256 (long enough that the flush at a segment's end is a
-// small part, 108 grid additions per quadratic segment), less -- at least 8 --
-// when the particles would not give every SM 16 warps.
-static int64_t warp_segment(int64_t n)
+// small part, 108 grid additions per quadratic segment), less -- at least 8, or
+// with one momentum component, whose lanes may add a particle each, 32 -- when the
+// particles would not give every SM 16 warps.
+static int64_t warp_segment(int64_t n, int64_t least)
 {
     const int64_t seg = (n / (148 * 16) + 7) / 8 * 8;
-    return seg < 8 ? 8 : (seg > 32 ? (seg > 256 ? 256 : seg / 32 * 32) : seg);
+    return seg < least ? least : (seg > 32 ? (seg > 256 ? 256 : seg / 32 * 32) : seg);
 }
 
 // ---------------------------------------------------------------------------
@@ -121,7 +122,7 @@ static void launch_p2g(Form form, const MeshP& mp, int64_t n, const PField& x, c
     const int threads = 256;
     const unsigned blocks = grid_for(n, threads);
     if (form == Form::F64) {
-        const int64_t seg = warp_segment(n);
+        const int64_t seg = warp_segment(n, STAG || NC == 1 ? 32 : 8);
         const int64_t ctas = (n + seg * kWarpP2GWarps - 1) / (seg * kWarpP2GWarps);
         apic_p2g_warp_kernel<ORDER, NC, STAG><<<(unsigned)ctas, 32 * kWarpP2GWarps, 0, st>>>(
             mp, n, seg, x, m, c, wide_rows<STAG ? 3 : NC>(c), gm, gmu, stag, err);

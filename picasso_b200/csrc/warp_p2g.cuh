@@ -93,6 +93,16 @@ struct WarpP2G {
     // straight to the grid: a run costs 290-400 ps more than its particles, the
     // direct way about 250 ps per particle with 4 fields and 190 ps with 2.
     static constexpr int kDirectNum = NT == 2 ? 5 : 3, kDirectDen = 8;
+    // With one momentum component, particles in few rows (i, j) of which many move the
+    // stencil are added by the lanes of their own: neighbouring lanes' nodes then lie
+    // along k and an addition of the warp covers whole sectors.  Of 32 particles at most
+    // kLaneRows rows, more than kLaneMoves moves.  1 M particles of a face field in cell
+    // order, ms, as runs or node by node / this way / one thread per particle: linear 1
+    // per cell 0.104 / 0.073 / 0.067, 8 per cell 0.131 / 0.080 / 0.083, 32 per cell 0.092
+    // / 0.110 / 0.156; quadratic 1 per cell 0.240 / 0.151 / 0.156, 4 per cell 0.266 /
+    // 0.174 / 0.217, 12 per cell 0.167 / 0.209 / 0.376; cubic 1 per cell 0.450 / 0.447 /
+    // 0.400, 6 per cell 0.687 / 0.418 / 0.588.
+    static constexpr int kLaneRows = 10, kLaneMoves = ORDER == 1 ? 4 : 9;
 };
 
 // c_p packed (rows of 4 x NCI doubles, a multiple of 16 bytes) from a 16-byte
@@ -322,7 +332,7 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
         }
         // stencil changes against the previous particle, and the changes by
         // one node along k
-        unsigned chg, step;
+        unsigned chg, step, rows;
         auto changes = [&] {
             int pv[3];
 #pragma unroll
@@ -334,6 +344,7 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
             const bool live = lane < cnt;
             chg = __ballot_sync(kAll, live && !(same2 && s[2] == pv[2]));
             step = __ballot_sync(kAll, live && same2 && s[0] >= 0 && s[2] == pv[2] + 1);
+            rows = __ballot_sync(kAll, live && !same2);
         };
         changes();
         if (__popc(chg & ~step) > 8) {
@@ -442,6 +453,59 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
         }
         const unsigned valid = __ballot_sync(kAll, s[0] >= 0);
         __syncwarp();
+        if constexpr (NV == 1) {
+            // every lane its own particle (kLaneRows)
+            if (__popc(rows) <= W::kLaneRows && __popc(chg) * 32 > cnt * W::kLaneMoves) {
+                if (cur >= -1) flush(false);
+                cur = -2;
+                if (s[0] >= 0) {
+                    int node[3][K];  // grid indices of the stencil
+#pragma unroll
+                    for (int d = 0; d < 3; ++d)
+#pragma unroll
+                        for (int q = 0; q < K; ++q) {
+                            int g = s[d] + q;
+                            while (g >= lim[d]) g -= lim[d];
+                            node[d][q] = g + off[d];
+                        }
+                    const double* wt = sm + lane;
+                    const double c0 = coef[CS * 0 + (ORDER == 1 ? ROW : 0) + lane],
+                                 c1 = coef[CS * 1 + (ORDER == 1 ? ROW : 0) + lane],
+                                 c2 = coef[CS * 2 + (ORDER == 1 ? ROW : 0) + lane],
+                                 c3 = coef[CS * 3 + (ORDER == 1 ? ROW : 0) + lane];
+#pragma unroll 1
+                    for (int i = 0; i < K; ++i) {
+                        const int gi = select<K>(node[0], i);
+#pragma unroll
+                        for (int j = 0; j < K; ++j) {
+                            double* pm = gm.ptr<double>(gi, node[1][j], 0, 0);
+                            double* pmu = gmu.ptr<double>(gi, node[1][j], 0, 0);
+#pragma unroll
+                            for (int k = 0; k < K; ++k) {
+                                double w, v;
+                                if constexpr (ORDER == 1) {  // linear_value of both fields
+                                    const double wx = wt[i * ROW], wy = wt[(2 + j) * ROW],
+                                                 wz = wt[(4 + k) * ROW];
+                                    const double x1 = i ? c1 : -c1, y1 = j ? c2 : -c2, z1 = k ? c3 : -c3;
+                                    w = coef[lane] * (wx * (wy * wz));
+                                    v = fma(fma(wx, c0, x1), wy * wz, wx * fma(z1, wy, y1 * wz));
+                                } else {  // (D0, D1, D2 = j, k, i)
+                                    w = ORDER == 3 ? wt[(j * K + k) * ROW] * wt[(KK + i) * ROW]
+                                                   : wt[(i * KK + j * K + k) * ROW];
+                                    v = w * fma((double)(i - 1), c3,
+                                                add_steps_f64(k - 1, fma((double)(j - 1), c1, c0), c2));
+                                }
+                                atomicAdd(pm + (int64_t)node[2][k] * gm.s[2], w);
+                                atomicAdd(pmu + (int64_t)node[2][k] * gmu.s[2], v);
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int d = 0; d < 3; ++d) last[d] = -1;  // no run to continue
+                continue;
+            }
+        }
         // table row of the weight of the lane's node number t (cubic: of its pair)
         auto wrow = [&](int t) {
             if (ORDER == 3) return ((t & 1) * 8 + lg) * ROW;
