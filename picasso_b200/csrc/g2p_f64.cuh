@@ -12,8 +12,9 @@
 // time, in whole lines.  What bounds it are the L1 wavefronts of the gather, 81
 // loads per quadratic particle:
 //   * particles in any order read u_i from global memory, in the order of their
-//     stencils inside a warp where they have little locality (64^3 cells of 8:
-//     0.214 ms as they come, 0.167 ms ordered, 90 % of the L1 data pipe);
+//     stencils inside a warp where they have little locality (linear, quadratic;
+//     64^3 cells of 8: 0.214 ms as they come, 0.167 ms ordered, 90 % of the L1 data
+//     pipe);
 //   * large dense sets of cell-sorted particles (bins; g2p_tiles_pay) read it from a
 //     node tile in shared memory (128^3 8 per cell clustered: 0.92 ms from global
 //     memory, 0.71 ms).
@@ -220,7 +221,7 @@ __device__ __forceinline__ bool g2p_gather(const MeshP& mp, const double (&xp)[3
 }
 
 // Particles p0 .. p0 + cnt - 1 (cnt <= 32) by a whole warp, gathered from global memory.
-// ORDERED: the particles come in the order of their stencils.  rows: see g2p_store.
+// ORDERED: the particles are taken as they come.  rows: see g2p_store.
 template <int ORDER, int NC, bool STAG, bool CG, bool ADV, bool UNIT, bool ORDERED>
 __device__ __forceinline__ void apic_g2p_warp(const MeshP& mp, int64_t p0, int cnt, const PField& x,
                                               const GField& u, const PField& c, int stag, int* err,
