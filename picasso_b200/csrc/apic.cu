@@ -35,7 +35,9 @@ apic_g2p_kernel(MeshP mp, int64_t n, PField x, GField u, PField c, int stag, int
 // FP64 G2P: grid-stride over 32 particles per warp.  Cubic: 3 CTAs, without spills, and
 // the particles as they come: 192 loads of 8 bytes hide their latency by themselves, and
 // 4 CTAs or ordering the lanes only cost (0.1 M clustered in random order 0.051 -> 0.035
-// ms, 4 M 1.53 -> 1.41 ms; in cell order 4 M 0.394 -> 0.406 ms).
+// ms, 4 M 1.53 -> 1.41 ms; in cell order 4 M 0.394 -> 0.406 ms).  Scalar fields, whose
+// results are one sector per particle, neither: linear 1 M in cell order 0.026 -> 0.020
+// ms (one thread per particle 0.021).
 template <int ORDER, int NC, bool STAG, bool ADV, bool UNIT>
 __global__ void __launch_bounds__(128, ORDER == 3 ? 3 : 4)
 apic_g2p_f64_kernel(MeshP mp, int64_t n, PField x, GField u, PField c, int stag, int* err,
@@ -47,7 +49,7 @@ apic_g2p_f64_kernel(MeshP mp, int64_t n, PField x, GField u, PField c, int stag,
     double* mine = packed ? rows[warp] : nullptr;
     const int64_t stride = (int64_t)gridDim.x * 128;
     for (int64_t p0 = (int64_t)blockIdx.x * 128 + warp * 32; p0 < n; p0 += stride)
-        apic_g2p_warp<ORDER, NC, STAG, false, ADV, UNIT, ORDER == 3>(
+        apic_g2p_warp<ORDER, NC, STAG, false, ADV, UNIT, ORDER == 3 || (NC == 1 && !STAG)>(
             mp, p0, (int)min((int64_t)32, n - p0), x, u, c, stag, err, &adv, mine);
 }
 
@@ -148,7 +150,8 @@ static void launch_g2p(bool f32, const MeshP& mp, int64_t n, const PField& x, co
     const Advect a = adv ? *adv : Advect{};
     if (!f32) {
         const unsigned blocks = grid_for(n, 128, 148LL * 64);
-        const bool packed = packed_rows_f64(x, c, 4 * (STAG ? 3 : NC), adv != nullptr);
+        const bool packed =
+            (NC > 1 || STAG) && packed_rows_f64(x, c, 4 * (STAG ? 3 : NC), adv != nullptr);
         auto launch = [&](auto kern) {
             kern<<<blocks, 128, 0, st>>>(mp, n, x, u, c, stag, err, a, packed);
         };

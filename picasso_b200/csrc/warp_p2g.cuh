@@ -93,16 +93,21 @@ struct WarpP2G {
     // straight to the grid: a run costs 290-400 ps more than its particles, the
     // direct way about 250 ps per particle with 4 fields and 190 ps with 2.
     static constexpr int kDirectNum = NT == 2 ? 5 : 3, kDirectDen = 8;
-    // With one momentum component, particles in few rows (i, j) of which many move the
-    // stencil are added by the lanes of their own: neighbouring lanes' nodes then lie
-    // along k and an addition of the warp covers whole sectors.  Of 32 particles at most
-    // kLaneRows rows, more than kLaneMoves moves.  1 M particles of a face field in cell
-    // order, ms, as runs or node by node / this way / one thread per particle: linear 1
-    // per cell 0.104 / 0.073 / 0.067, 8 per cell 0.131 / 0.080 / 0.083, 32 per cell 0.092
-    // / 0.110 / 0.156; quadratic 1 per cell 0.240 / 0.151 / 0.156, 4 per cell 0.266 /
-    // 0.174 / 0.217, 12 per cell 0.167 / 0.209 / 0.376; cubic 1 per cell 0.450 / 0.447 /
-    // 0.400, 6 per cell 0.687 / 0.418 / 0.588.
-    static constexpr int kLaneRows = 10, kLaneMoves = ORDER == 1 ? 4 : 9;
+    // With one or two momentum components, particles in few rows (i, j) of which many
+    // move the stencil are added by the lanes of their own: neighbouring lanes' nodes
+    // then lie along k and an addition of the warp covers whole sectors.  Of 32 particles
+    // at most kLaneRows rows, more than kLaneMoves moves.  1 M particles in cell order,
+    // ms, as runs or node by node / this way / one thread per particle.  A face field:
+    // linear 1 per cell 0.104 / 0.073 / 0.067, 8 per cell 0.131 / 0.080 / 0.083, 32 per
+    // cell 0.092 / 0.110 / 0.156; quadratic 1 per cell 0.240 / 0.151 / 0.156, 4 per cell
+    // 0.266 / 0.174 / 0.217, 12 per cell 0.167 / 0.209 / 0.376; cubic 1 per cell 0.450 /
+    // 0.447 / 0.400, 6 per cell 0.687 / 0.418 / 0.588.  Two components: linear 1 per cell
+    // 0.176 / 0.077 / 0.067; quadratic 2 per cell 0.425 / 0.327 / 0.322, 8 per cell 0.281
+    // / 0.324 / 0.438; cubic 1 per cell 0.936 / 0.560 / 0.533, 2 per cell 0.401 / 0.592 /
+    // 0.617.
+    static constexpr int kLaneRows = 10;
+    static constexpr int kLaneMoves =
+        ORDER == 1 ? 4 : NV == 1 ? 9 : (ORDER == 2 ? 18 : 20);
 };
 
 // c_p packed (rows of 4 x NCI doubles, a multiple of 16 bytes) from a 16-byte
@@ -453,7 +458,7 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
         }
         const unsigned valid = __ballot_sync(kAll, s[0] >= 0);
         __syncwarp();
-        if constexpr (NV == 1) {
+        if constexpr (NV < 3) {
             // every lane its own particle (kLaneRows)
             if (__popc(rows) <= W::kLaneRows && __popc(chg) * 32 > cnt * W::kLaneMoves) {
                 if (cur >= -1) flush(false);
@@ -469,10 +474,12 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
                             node[d][q] = g + off[d];
                         }
                     const double* wt = sm + lane;
-                    const double c0 = coef[CS * 0 + (ORDER == 1 ? ROW : 0) + lane],
-                                 c1 = coef[CS * 1 + (ORDER == 1 ? ROW : 0) + lane],
-                                 c2 = coef[CS * 2 + (ORDER == 1 ? ROW : 0) + lane],
-                                 c3 = coef[CS * 3 + (ORDER == 1 ? ROW : 0) + lane];
+                    double cf[NV][4];
+#pragma unroll
+                    for (int f = 0; f < NV; ++f)
+#pragma unroll
+                        for (int r = 0; r < 4; ++r)
+                            cf[f][r] = coef[r * CS + (ORDER == 1 ? f + 1 : f) * ROW + lane];
 #pragma unroll 1
                     for (int i = 0; i < K; ++i) {
                         const int gi = select<K>(node[0], i);
@@ -482,21 +489,32 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
                             double* pmu = gmu.ptr<double>(gi, node[1][j], 0, 0);
 #pragma unroll
                             for (int k = 0; k < K; ++k) {
-                                double w, v;
-                                if constexpr (ORDER == 1) {  // linear_value of both fields
+                                const int n[3] = {i, j, k};
+                                const int pair = n[D0] * K + n[D1];
+                                double w, v[NV];
+                                if constexpr (ORDER == 1) {  // linear_value of all fields
                                     const double wx = wt[i * ROW], wy = wt[(2 + j) * ROW],
                                                  wz = wt[(4 + k) * ROW];
-                                    const double x1 = i ? c1 : -c1, y1 = j ? c2 : -c2, z1 = k ? c3 : -c3;
                                     w = coef[lane] * (wx * (wy * wz));
-                                    v = fma(fma(wx, c0, x1), wy * wz, wx * fma(z1, wy, y1 * wz));
-                                } else {  // (D0, D1, D2 = j, k, i)
-                                    w = ORDER == 3 ? wt[(j * K + k) * ROW] * wt[(KK + i) * ROW]
-                                                   : wt[(i * KK + j * K + k) * ROW];
-                                    v = w * fma((double)(i - 1), c3,
-                                                add_steps_f64(k - 1, fma((double)(j - 1), c1, c0), c2));
+#pragma unroll
+                                    for (int f = 0; f < NV; ++f) {
+                                        const double x1 = i ? cf[f][1] : -cf[f][1], y1 = j ? cf[f][2] : -cf[f][2],
+                                                     z1 = k ? cf[f][3] : -cf[f][3];
+                                        v[f] = fma(fma(wx, cf[f][0], x1), wy * wz, wx * fma(z1, wy, y1 * wz));
+                                    }
+                                } else {
+                                    w = ORDER == 3 ? wt[pair * ROW] * wt[(KK + n[D2]) * ROW]
+                                                   : wt[(n[D2] * KK + pair) * ROW];
+#pragma unroll
+                                    for (int f = 0; f < NV; ++f)
+                                        v[f] = w * fma((double)(n[D2] - 1), cf[f][3],
+                                                       fma((double)(n[D1] - 1), cf[f][2],
+                                                           fma((double)(n[D0] - 1), cf[f][1], cf[f][0])));
                                 }
                                 atomicAdd(pm + (int64_t)node[2][k] * gm.s[2], w);
-                                atomicAdd(pmu + (int64_t)node[2][k] * gmu.s[2], v);
+#pragma unroll
+                                for (int f = 0; f < NV; ++f)
+                                    atomicAdd(pmu + (int64_t)node[2][k] * gmu.s[2] + f * gmu.s[3], v[f]);
                             }
                         }
                     }
