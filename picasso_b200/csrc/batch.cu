@@ -183,8 +183,8 @@ static int warp_p2g_bytes(int order)
 }
 
 // FP64 G2P item; smem: a WarpRows buffer per warp, then the node tile
-// (g2p_item_f64).  An instance whose tiles do not fit in shared memory, or do not pay,
-// gathers from global memory (apic_g2p_warp).  CG: u_i was written in this launch.
+// (g2p_item_f64).  An instance whose tiles do not pay gathers from global memory
+// (apic_g2p_warp).  CG: u_i was written in this launch.
 constexpr int kWarpG2PBytes = WarpRows<3, false>::DOUBLES * (int)sizeof(double);
 
 template <int ORDER, int NT, bool CG>
@@ -408,12 +408,13 @@ picasso_status configure(picasso_batch* b)
     for (int p = 0; p < kPhases; ++p)
         items[p] = (int)(b->qbegin[(p + 1) * b->count] - b->qbegin[p * b->count]);
     if ((st = configure_kernel<F32, 0x1>(b->smem[0], items[0], &b->blocks[0]))) return st;
-    if ((st = configure_kernel<F32, 0x2>(b->smem[1], items[1], &b->blocks[1]))) return st;
     if ((st = configure_kernel<F32, 0x4>(b->smem[2], items[2], &b->blocks[2]))) return st;
     if ((st = configure_kernel<F32, 0x8>(b->smem[3], items[3], &b->blocks[3]))) return st;
     if ((st = configure_variant<F32, 0>(b))) return st;
     if ((st = configure_variant<F32, 1>(b))) return st;
-    return configure_variant<F32, 2>(b);
+    if ((st = configure_variant<F32, 2>(b))) return st;
+    b->blocks[1] = *std::max_element(b->var_blocks, b->var_blocks + kVariants);
+    return PICASSO_OK;
 }
 
 template <bool F32, int VAR>
@@ -442,7 +443,6 @@ void launch_phase(const picasso_batch* b, int p, cudaStream_t s)
         b->dev, lo, hi, P)
     switch (p) {
         case 0: PB_PHASE(0, 0x1); break;
-        case 1: PB_PHASE(1, 0x2); break;
         case 2: PB_PHASE(2, 0x4); break;
         default: PB_PHASE(3, 0x8); break;
     }
@@ -552,10 +552,8 @@ picasso_status make_instance(const picasso_batch_instance& in, bool f32, BInst* 
         *smem_g2p = std::max(*smem_g2p, (int)(sizeof(float4) * (size_t)tp.nodes));
     } else {
         *smem_p2g = std::max(*smem_p2g, warp_p2g_bytes(order));  // one warp's
-        const int64_t tile = 3 * (int64_t)sizeof(double) * tp.nodes;
-        I->g2p_tile = tile + kF64Warps * kWarpG2PBytes <= device_smem_optin() &&
-                      g2p_tiles_pay(tp, order, in.num_particles);
-        if (I->g2p_tile) *smem_g2p = std::max(*smem_g2p, (int)tile);
+        I->g2p_tile = g2p_tiles_pay(tp, order, in.num_particles);  // (40 KB at most)
+        if (I->g2p_tile) *smem_g2p = std::max(*smem_g2p, 3 * (int)sizeof(double) * tp.nodes);
     }
     return PICASSO_OK;
 }
@@ -580,7 +578,8 @@ extern "C" picasso_status picasso_batch_create(const picasso_batch_instance* ins
     const int p2g_bytes = f32 ? smem_p2g : kF64Warps * smem_p2g;
     const int g2p_bytes = f32 ? smem_g2p : kF64Warps * kWarpG2PBytes + smem_g2p;
     const int fused_bytes = std::max(smem_p2g, f32 ? smem_g2p : kWarpG2PBytes + smem_g2p);
-    if (std::max(std::max(p2g_bytes, g2p_bytes), fused_bytes) > device_smem_optin())
+    if (std::max(std::max(p2g_bytes, g2p_bytes), fused_bytes) >
+        device_smem_optin() - (f32 ? kBatchStaticSmem : 0))
         return PICASSO_ERR_UNSUPPORTED;
 
     picasso_batch* b = new (std::nothrow) picasso_batch();

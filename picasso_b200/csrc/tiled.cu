@@ -253,7 +253,9 @@ bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n,
         int sj, si;
         choose_strides(tp->NT, K, &sj, &si);
         // (a tile that the padding pushes out of shared memory stays unpadded)
-        if ((int64_t)p2g_warp_bytes(order, tp->NT[0] * si) <= device_smem_optin()) {
+        const int64_t limit =
+            device_smem_optin() - (use == TileUse::batch_streams ? kBatchStaticSmem : 0);
+        if ((int64_t)p2g_warp_bytes(order, tp->NT[0] * si) <= limit) {
             tp->SJ = sj;
             tp->SI = si;
             tp->P = tp->NT[0] * si;

@@ -131,6 +131,10 @@ struct G2PArgs {
     HaloPeers hp;
 };
 
+// Static shared memory of the batch's kernels, which copy these arguments there: the
+// launch that runs all phases holds both.
+constexpr int kBatchStaticSmem = (int)((sizeof(P2GArgs) + 15) / 16 * 16 + (sizeof(G2PArgs) + 15) / 16 * 16);
+
 __device__ __forceinline__ int bin_of(const MeshP& mp, const TileP& tp, int d, int s0)
 {
     if (mp.periodic[d]) {
