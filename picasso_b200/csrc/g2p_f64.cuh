@@ -186,6 +186,56 @@ __device__ __forceinline__ void g2p_store(int64_t p0, int at, bool ok, const dou
     }
 }
 
+// B_p of particle p node by node as it is defined, for the components whose u_p (in `up`)
+// is not finite: relative to the centre knot an infinite node velocity makes NaN, inf - inf,
+// of sums that are infinite.  After g2p_store (whose registers it then does not add to),
+// by whole warps.  With advection the particle's position is not finite either, and stays.
+template <int NU>
+__device__ __forceinline__ bool g2p_odd(const double (&up)[NU])
+{
+    unsigned top = 0;
+#pragma unroll
+    for (int d = 0; d < NU; ++d) top = max(top, high_bits(up[d]));
+    return top >= kNotFinite;
+}
+template <int ORDER, int NC, bool STAG, bool CG>
+__device__ __forceinline__ void g2p_store_odd(const MeshP& mp, int64_t p, bool odd, const PField& x,
+                                              const GField& u, const PField& c, int stag)
+{
+    constexpr int K = SplineTraits<ORDER>::K, NU = STAG ? 1 : NC, NCO = STAG ? 3 : NC;
+    if (!__any_sync(0xFFFFFFFFu, odd)) return;  // (and the row has been written)
+    if (!odd) return;
+#pragma unroll 1
+    for (int d = 0; d < NU; ++d) {
+        double up = 0.0, b[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int e = 0; e < K * K * K; ++e) {
+            double w = 1.0, dist[3];
+            int g[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                const int n = q == 0 ? e / (K * K) : (q == 1 ? e / K % K : e % K);
+                const double xq = x.get<double>(p, q);
+                double ws[K], dist0;
+                int s0, idx[K];
+                g2p_spline<ORDER>(xq, mp.lo[q], mp.dx[q], mp.rdx[q], s0, ws, dist0);
+                resolve_stencil<K>(mp, q, s0, idx);
+                w *= select<K>(ws, n);
+                dist[q] = fma((double)(s0 + n), mp.dx[q], mp.lo[q]) - xq;
+                g[q] = select<K>(idx, n);
+            }
+            const double* a = u.ptr<double>(g[0], g[1], g[2], d);
+            const double wu = w * (CG ? __ldcg(a) : __ldg(a));
+            up += wu;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) b[q] = fma(wu, dist[q], b[q]);
+        }
+        if (high_bits(up) < kNotFinite) continue;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) c.set<double>(p, (1 + q) * NCO + (STAG ? stag : d), b[q]);
+    }
+}
+
 // u_p and B_p of a particle at xp gathered from u_i in global memory.  False (counted in
 // err) if the stencil leaves a non-periodic mesh.  CG: u_i is read through L2 only
 // (written earlier in the same launch).  UNIT: the components of u_i are adjacent.
@@ -257,7 +307,9 @@ __device__ __forceinline__ void apic_g2p_warp(const MeshP& mp, int64_t p0, int c
         for (int d = 0; d < 3; ++d) xp[d] = x.get<double>(p0 + at, d);
         ok = g2p_gather<ORDER, NU, CG, UNIT>(mp, xp, u, err, up, B);
     }
+    const bool odd = !ADV && ok && g2p_odd(up);
     g2p_store<NC, STAG, ADV>(p0, at, ok, xp, up, B, x, c, stag, adv, rows);
+    if (!ADV) g2p_store_odd<ORDER, NC, STAG, CG>(mp, p0 + at, odd, x, u, c, stag);
 }
 
 // A tile of node velocities in shared memory: `u` holds NU doubles per node of
@@ -384,7 +436,9 @@ __device__ __forceinline__ void g2p_tile_warp(const MeshP& mp, const NodeTile& n
             if (!ok && err) atomicAdd(err, 1);
         }
     }
+    const bool odd = !ADV && ok && g2p_odd(up);
     g2p_store<3, false, ADV>(p0, lane, ok, xp, up, B, x, c, -1, adv, rows);
+    if (!ADV) g2p_store_odd<ORDER, 3, false, CG>(mp, p0 + lane, odd, x, u, c, -1);
 }
 
 // One work item (tile t, particles [a, b)) of cell-sorted particles by NTHR

@@ -32,6 +32,13 @@ __device__ __forceinline__ R inertial_scaling(double dx0)
     return (R)((ORDER == 2 ? 4.0 : 3.0) / (dx0 * dx0));
 }
 
+// Exponent and leading bits of |v|: kNotFinite and above for infinities and NaN.
+__device__ __forceinline__ unsigned high_bits(double v)
+{
+    return (unsigned)__double2hiint(v) << 1;
+}
+constexpr unsigned kNotFinite = 0xFFE00000u;
+
 // First stencil node of a particle along d, counted from the owned box in a
 // periodic dimension; false if the stencil leaves a non-periodic mesh.
 template <int K>

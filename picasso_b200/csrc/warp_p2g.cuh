@@ -119,6 +119,56 @@ inline bool wide_rows(const PField& c)
            reinterpret_cast<uintptr_t>(c.data) % 16 == 0;
 }
 
+// A particle whose mass or coefficients are not all finite, node by node as it is defined
+// (others: nothing): relative to the centre knot an infinite coefficient would make NaN,
+// inf - inf or 0 inf, of nodes that are infinite.  Called at the segment's end: inside the
+// loop it spills (quadratic 3 M sorted 0.282 -> 0.295 ms, this way 0.289).
+template <int ORDER, int NC, bool STAG>
+__device__ __forceinline__ void p2g_odd_particle(const MeshP& mp, int64_t p, const PField& x,
+                                                 const PField& m, const PField& c,
+                                                 const GField& gm, const GField& gmu, int stag)
+{
+    using W = WarpP2G<ORDER, NC, STAG>;
+    constexpr int K = W::K;
+    const double D = inertial_scaling<ORDER == 1 ? 2 : ORDER, double>(mp.dx[0]);
+    unsigned top = high_bits(m.get<double>(p, 0));
+    for (int q = 0; q < 4; ++q) {
+        for (int d = 0; d < W::NV; ++d)
+            top = max(top, high_bits(c.get<double>(p, q * W::NCI + (STAG ? stag : d))));
+    }
+    if (top < kNotFinite) return;
+#pragma unroll 1
+    for (int e = 0; e < W::KKK; ++e) {
+        double w = m.get<double>(p, 0), dist[3];
+        int g[3];
+        bool ok = true;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int n = d == 0 ? e / W::KK : (d == 1 ? e / K % K : e % K);
+            const double xd = x.get<double>(p, d);
+            const double x0 = logical_coord(xd, mp.lo[d], mp.rdx[d], SplineTraits<ORDER>::shift);
+            Spline1D<ORDER, double> sp;
+            spline_eval_f64<ORDER>(xd, mp.lo[d], mp.dx[d], mp.rdx[d], sp);
+            w *= select<K>(sp.w, n);
+            dist[d] = select<K>(sp.d, n);
+            int idx[K];
+            ok = resolve_stencil<K>(mp, d, (int)floor(x0) + SplineTraits<ORDER>::first, idx) && ok;
+            g[d] = select<K>(idx, n);
+        }
+        if (!ok) return;  // out of the mesh, counted already
+        atomicAdd(gm.ptr<double>(g[0], g[1], g[2], 0), w);
+#pragma unroll 1
+        for (int d = 0; d < W::NV; ++d) {
+            const int col = STAG ? stag : d;
+            double v = 0.0;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) v = fma(c.get<double>(p, (1 + q) * W::NCI + col), dist[q], v);
+            atomicAdd(gmu.ptr<double>(g[0], g[1], g[2], d),
+                      w * fma(D, v, c.get<double>(p, col)));
+        }
+    }
+}
+
 // Adds the particles [a, b) to the grid; called by a whole warp.  sm:
 // WarpP2G::DOUBLES doubles of the warp.  wide: wide_rows(c).
 template <int ORDER, int NC, bool STAG>
@@ -315,6 +365,7 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
     };
 
     int last[3] = {-1, -1, -1};  // stencil start of the previous particle
+    bool odd = false;  // the lane has had a particle that p2g_odd_particle takes
     for (int64_t p0 = a; p0 < b; p0 += 32) {
         const int cnt = (int)min((int64_t)32, b - p0);
         int64_t p = p0 + lane;
@@ -427,6 +478,7 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
                 }
                 const double D =
                     ORDER == 1 ? 1.0 : inertial_scaling<ORDER == 1 ? 2 : ORDER, double>(mp.dx[0]);
+                unsigned top = high_bits(mass);
 #pragma unroll
                 for (int d = 0; d < NV; ++d) {
                     double v[4];
@@ -437,6 +489,8 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
                             v[r] = stag == 0 ? v[r] : (stag == 1 ? cp[r * 3 + 1] : cp[r * 3 + 2]);
                     }
                     if constexpr (ORDER >= 2) {
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) top = max(top, high_bits(v[r]));
                         const double bd =
                             fma(v[3], sp[2].d[1], fma(v[2], sp[1].d[1], v[1] * sp[0].d[1]));
                         v[0] = fma(D, bd, v[0]);
@@ -453,6 +507,13 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
                         coef[r * CS + (ORDER == 1 ? d + 1 : d) * ROW + lane] = v[r];
+                }
+                if constexpr (ORDER >= 2) {
+                    if (top >= kNotFinite) {
+                        odd = true;  // and the table without it
+#pragma unroll 1
+                        for (int r = 0; r < W::WROWS + W::CROWS; ++r) sm[r * ROW + lane] = 0.0;
+                    }
                 }
             }
         }
@@ -620,6 +681,10 @@ __device__ __forceinline__ void apic_p2g_warp(const MeshP& mp, int64_t a, int64_
         for (int d = 0; d < 3; ++d) last[d] = __shfl_sync(kAll, s[d], cnt - 1);
     }
     if (cur >= -1) flush(false);
+    if (ORDER >= 2 && __any_sync(kAll, odd)) {
+        for (int64_t p = a + lane; p < b; p += 32)
+            p2g_odd_particle<ORDER, NC, STAG>(mp, p, x, m, c, gm, gmu, stag);
+    }
 }
 
 }  // namespace pb
