@@ -16,6 +16,9 @@ the particle arrays in pinned host memory, copies included.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
+The printed line holds the headline and one summary per leg (`stdout_line`);
+`--json-out FILE` writes the whole record, kernels and autotuner tables included.
+
 Under torchrun each rank runs its own replica of the workload (no
 collective in the data path); `value` is the sum over ranks of particles
 divided by the slowest rank's time.
@@ -705,10 +708,7 @@ def run_ours(args):
                              "fp64_ms_per_step": adv["fp64"]["ms_per_step"],
                              "speedup_fp32_vs_fp64": adv["speedup_fp32_vs_fp64"]}
     if rank == 0:
-        print(json.dumps(line))
-        if args.json_out:
-            with open(args.json_out, "w") as f:
-                json.dump(line, f, indent=1)
+        emit(line, args.json_out)
     if dist:
         torch.distributed.barrier()
         torch.distributed.destroy_process_group()
@@ -959,6 +959,56 @@ def run_polypic(args, peak):
         del xs, ms, us, modes, perm, sd, sd0, finals
         torch.cuda.empty_cache()
     return res
+
+
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+            "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "impl", "config", "e2e",
+            "gpu_launches", "clocks", "roofline", "speedup_fp32_vs_fp64", "errors_vs_fp64",
+            "cpu_baseline")
+
+
+def stdout_line(record):
+    """One JSON line of the record's headline keys and a summary of the others: every FP64
+    form's value and time, the sort, the legs' times.  A few KB whatever the record holds."""
+    line = {k: record[k] for k in HEADLINE if k in record}
+    for k in ("fp64_plain", "fp64_plain_unsorted"):
+        if k in record:
+            line[k] = {q: record[k][q] for q in ("value", "ms_per_step", "step_frac")}
+    if "step_roofline" in record:
+        line["step_frac"] = record["step_roofline"]["frac"]
+    if "sort" in record:
+        line["sort"] = {k: v for k, v in record["sort"].items() if isinstance(v, (int, float))}
+    if "errors_vs_oracle" in record:
+        line["errors_vs_oracle"] = {form: {k: e["normwise"] for k, e in errors.items()}
+                                    for form, errors in record["errors_vs_oracle"].items()
+                                    if isinstance(errors, dict)}
+    if "advect_cubic" in record:
+        line["advect_cubic_ms"] = {f: record["advect_cubic"][f]["ms_per_step"]
+                                   for f in ("fp32", "fp64")}
+    if "polypic" in record:
+        line["polypic_ms"] = {modes: {f: r[f]["ms_per_step"] for f in ("fp32", "fp64")}
+                              for modes, r in record["polypic"].items() if isinstance(r, dict)}
+    for holder in (record, record.get("batch", {})):
+        if "forms" in holder:
+            line["batch_ms"] = {f: {mode: m["ms_per_step"] for mode, m in r["modes"].items()}
+                                for f, r in holder["forms"].items()}
+
+    def short(v):  # six digits of what the contract does not name
+        if isinstance(v, dict):
+            return {k: short(q) for k, q in v.items()}
+        if isinstance(v, list):
+            return [short(q) for q in v]
+        return float("%.6g" % v) if isinstance(v, float) else v
+
+    exact = ("value", "ms_per_step", "e2e", "clocks")
+    return json.dumps({k: v if k in exact else short(v) for k, v in line.items()})
+
+
+def emit(record, json_out):
+    print(stdout_line(record), flush=True)
+    if json_out:
+        with open(json_out, "w") as f:
+            json.dump(record, f, indent=1)
 
 
 def run_leg_alone(args):
@@ -1240,11 +1290,7 @@ def run_batch(args):
                        "frac": best["modes"]["fused"]["frac_hbm"],
                        "peak_source": peak["source"], "traffic": None}
     out["autotune_measurements"] = meas
-    line = json.dumps(out)
-    print(line)
-    if args.json_out:
-        with open(args.json_out, "w") as f:
-            f.write(line + "\n")
+    emit(out, args.json_out)
 
 
 def main():
