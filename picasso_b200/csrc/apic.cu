@@ -12,24 +12,24 @@ namespace pb {
 // ---------------------------------------------------------------------------
 // kernels: one thread per particle, grid-stride
 // ---------------------------------------------------------------------------
-template <int ORDER, int NC, bool STAG, class PT, class R, class ACC>
+template <int ORDER, int NC, bool STAG, class R>
 __global__ void __launch_bounds__(256)
 apic_p2g_kernel(MeshP mp, int64_t n, PField x, PField m, PField c, GField gm, GField gmu,
                 int stag, R scale_m, R scale_mu, int* err)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
-        apic_p2g_particle<ORDER, NC, STAG, PT, R, ACC>(mp, p, x, m, c, gm, gmu, stag, scale_m,
-                                                       scale_mu, err);
+        apic_p2g_particle<ORDER, NC, STAG, R>(mp, p, x, m, c, gm, gmu, stag, scale_m, scale_mu,
+                                              err);
 }
 
-template <int ORDER, int NC, bool STAG, class GT, class PT, class R, bool ADV>
+template <int ORDER, int NC, bool STAG, bool ADV>
 __global__ void __launch_bounds__(256)
 apic_g2p_kernel(MeshP mp, int64_t n, PField x, GField u, PField c, int stag, int* err, Advect adv)
 {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += stride)
-        apic_g2p_particle<ORDER, NC, STAG, GT, PT, R, ADV>(mp, p, x, u, c, stag, err, &adv);
+        apic_g2p_particle<ORDER, NC, STAG, ADV>(mp, p, x, u, c, stag, err, &adv);
 }
 
 // FP64 G2P: grid-stride over 32 particles per warp.  Cubic: 3 CTAs, without spills, and
@@ -132,11 +132,11 @@ static void launch_p2g(Form form, const MeshP& mp, int64_t n, const PField& x, c
         apic_p2g_warp_kernel<ORDER, NC, STAG><<<(unsigned)ctas, 32 * kWarpP2GWarps, 0, st>>>(
             mp, n, seg, x, m, c, wide_rows<STAG ? 3 : NC>(c), gm, gmu, stag, err);
     } else if (form == Form::F32Fixed) {
-        apic_p2g_kernel<ORDER, NC, STAG, float, float, AccFixed><<<blocks, threads, 0, st>>>(
+        apic_p2g_kernel<ORDER, NC, STAG, float><<<blocks, threads, 0, st>>>(
             mp, n, x, m, c, gm, gmu, stag, ldexpf(1.0f, gm.fixed_bits),
             ldexpf(1.0f, gmu.fixed_bits), err);
     } else {
-        apic_p2g_kernel<ORDER, NC, STAG, double, double, AccFixed><<<blocks, threads, 0, st>>>(
+        apic_p2g_kernel<ORDER, NC, STAG, double><<<blocks, threads, 0, st>>>(
             mp, n, x, m, c, gm, gmu, stag, ldexp(1.0, gm.fixed_bits),
             ldexp(1.0, gmu.fixed_bits), err);
     }
@@ -175,12 +175,12 @@ static void launch_g2p(bool f32, const MeshP& mp, int64_t n, const PField& x, co
     const unsigned blocks = grid_for(n, threads);
     if constexpr (NC == 3 && !STAG) {
         if (adv) {
-            apic_g2p_kernel<ORDER, NC, STAG, float, float, float, true>
+            apic_g2p_kernel<ORDER, NC, STAG, true>
                 <<<blocks, threads, 0, st>>>(mp, n, x, u, c, stag, err, a);
             return;
         }
     }
-    apic_g2p_kernel<ORDER, NC, STAG, float, float, float, false><<<blocks, threads, 0, st>>>(
+    apic_g2p_kernel<ORDER, NC, STAG, false><<<blocks, threads, 0, st>>>(
         mp, n, x, u, c, stag, err, a);
 }
 

@@ -16,9 +16,8 @@ namespace pb {
 // ---------------------------------------------------------------------------
 // NC: field components (collocated); STAG: staggered (Face/Edge) location,
 // scattering c_p column `stag` of a 3-component matrix into component 0.
-// PT: particle storage type of m_p / c_p; R: arithmetic type; ACC: grid
-// accumulation policy (FP64 atomics or 64-bit fixed point).
-template <int ORDER, int NC, bool STAG, class PT, class R, class ACC>
+// R: storage type of m_p / c_p and arithmetic type.  64-bit fixed-point grids.
+template <int ORDER, int NC, bool STAG, class R>
 __device__ __forceinline__ void apic_p2g_particle(const MeshP& mp, int64_t p, const PField& x,
                                                   const PField& m, const PField& c,
                                                   const GField& gm, const GField& gmu, int stag,
@@ -38,12 +37,12 @@ __device__ __forceinline__ void apic_p2g_particle(const MeshP& mp, int64_t p, co
         if (err) atomicAdd(err, 1);
         return;
     }
-    const R mass = (R)m.get<PT>(p, 0);
+    const R mass = m.get<R>(p, 0);
     R cp[4][NCI];
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int d = 0; d < NCI; ++d) cp[r][d] = (R)c.get<PT>(p, r * NCI + d);
+        for (int d = 0; d < NCI; ++d) cp[r][d] = c.get<R>(p, r * NCI + d);
 
     if (ORDER >= 2) {
         // APIC.hpp:94-139 (collocated) and :190-231 (staggered)
@@ -74,17 +73,17 @@ __device__ __forceinline__ void apic_p2g_particle(const MeshP& mp, int64_t p, co
                             R dbd = R(0);
 #pragma unroll
                             for (int a = 0; a < 3; ++a) dbd += DB[d][a] * dist[a];
-                            ACC::add(gmu, idx[0][i], idx[1][j], idx[2][k], d,
+                            AccFixed::add(gmu, idx[0][i], idx[1][j], idx[2][k], d,
                                      wm * (cp[0][d] + dbd), scale_mu);
                         }
                     } else {
                         R bd = R(0);
 #pragma unroll
                         for (int a = 0; a < 3; ++a) bd += DBs[a] * dist[a];
-                        ACC::add(gmu, idx[0][i], idx[1][j], idx[2][k], 0,
+                        AccFixed::add(gmu, idx[0][i], idx[1][j], idx[2][k], 0,
                                  wm * (c0s + bd), scale_mu);
                     }
-                    ACC::add(gm, idx[0][i], idx[1][j], idx[2][k], 0, wm, scale_m);
+                    AccFixed::add(gm, idx[0][i], idx[1][j], idx[2][k], 0, wm, scale_m);
                 }
     } else {
         // order 1, gradient form: APIC.hpp:276-318 and :363-401
@@ -111,17 +110,17 @@ __device__ __forceinline__ void apic_p2g_particle(const MeshP& mp, int64_t p, co
                             R bg = R(0);
 #pragma unroll
                             for (int a = 0; a < 3; ++a) bg += cp[1 + a][d] * gm3[a];
-                            ACC::add(gmu, idx[0][i], idx[1][j], idx[2][k], d,
+                            AccFixed::add(gmu, idx[0][i], idx[1][j], idx[2][k], d,
                                      wm * cp[0][d] + bg, scale_mu);
                         }
                     } else {
                         R bg = R(0);
 #pragma unroll
                         for (int a = 0; a < 3; ++a) bg += Bs[a] * gm3[a];
-                        ACC::add(gmu, idx[0][i], idx[1][j], idx[2][k], 0,
+                        AccFixed::add(gmu, idx[0][i], idx[1][j], idx[2][k], 0,
                                  wm * c0s + bg, scale_mu);
                     }
-                    ACC::add(gm, idx[0][i], idx[1][j], idx[2][k], 0, wm, scale_m);
+                    AccFixed::add(gm, idx[0][i], idx[1][j], idx[2][k], 0, wm, scale_m);
                 }
     }
 }
@@ -129,14 +128,15 @@ __device__ __forceinline__ void apic_p2g_particle(const MeshP& mp, int64_t p, co
 // ---------------------------------------------------------------------------
 // G2P
 // ---------------------------------------------------------------------------
-// GT: grid storage type of u_i; PT: particle storage type of c_p.
-// ADV (collocated, 3 components): then moves the particle, x += dt u_p with
-// the stored (PT-rounded) u_p, exactly as picasso_advect would afterwards.
-template <int ORDER, int NC, bool STAG, class GT, class PT, class R, bool ADV = false>
+// FP32 u_i, c_p and arithmetic.
+// ADV (collocated, 3 components): then moves the particle, x += dt u_p,
+// exactly as picasso_advect would afterwards.
+template <int ORDER, int NC, bool STAG, bool ADV = false>
 __device__ __forceinline__ void apic_g2p_particle(const MeshP& mp, int64_t p, const PField& x,
                                                   const GField& u, const PField& c, int stag,
                                                   int* err, const Advect* adv = nullptr)
 {
+    using R = float;
     constexpr int K = SplineTraits<ORDER>::K;
     constexpr int NCO = STAG ? 3 : NC;
     Spline1D<ORDER, R> sp[3];
@@ -172,7 +172,7 @@ __device__ __forceinline__ void apic_g2p_particle(const MeshP& mp, int64_t p, co
                     R ue[NC];
 #pragma unroll
                     for (int d = 0; d < NC; ++d)
-                        ue[d] = (R)__ldg(u.ptr<GT>(idx[0][i], idx[1][j], idx[2][k], d));
+                        ue[d] = __ldg(u.ptr<R>(idx[0][i], idx[1][j], idx[2][k], d));
 #pragma unroll
                     for (int d = 0; d < NC; ++d) {
                         up[d] = up[d] + w * ue[d];
@@ -181,7 +181,7 @@ __device__ __forceinline__ void apic_g2p_particle(const MeshP& mp, int64_t p, co
                         for (int a = 0; a < 3; ++a) B[d][a] += wu * dist[a];
                     }
                 } else {
-                    const R ue = (R)__ldg(u.ptr<GT>(idx[0][i], idx[1][j], idx[2][k], 0));
+                    const R ue = __ldg(u.ptr<R>(idx[0][i], idx[1][j], idx[2][k], 0));
                     const R wu = w * ue;
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
@@ -196,14 +196,14 @@ __device__ __forceinline__ void apic_g2p_particle(const MeshP& mp, int64_t p, co
     // c_p(0,d) = u_p(d); c_p(1+a,d) = B_p(d,a)  (APIC.hpp:464-471)
 #pragma unroll
     for (int d = 0; d < NCO; ++d) {
-        c.set<PT>(p, 0 * NCO + d, (PT)up[d]);
+        c.set<R>(p, 0 * NCO + d, up[d]);
 #pragma unroll
-        for (int a = 0; a < 3; ++a) c.set<PT>(p, (1 + a) * NCO + d, (PT)B[d][a]);
+        for (int a = 0; a < 3; ++a) c.set<R>(p, (1 + a) * NCO + d, B[d][a]);
     }
     if constexpr (ADV) {
         static_assert(!STAG && NC == 3, "advection needs the 3-component collocated velocity");
         const double xo[3] = {x.get<double>(p, 0), x.get<double>(p, 1), x.get<double>(p, 2)};
-        const double uo[3] = {(double)(PT)up[0], (double)(PT)up[1], (double)(PT)up[2]};
+        const double uo[3] = {(double)up[0], (double)up[1], (double)up[2]};
         advect_particle(*adv, p, xo, uo, [&](int d, double v) { x.set<double>(p, d, v); });
     }
 }

@@ -161,12 +161,18 @@ static RunStrides run_strides(const int NT[3], int K)
 // such sets are summed in the same order as ever.  Cubic ones stay below 0.9e-9.
 // (The streams would take 0.6 to 0.9 times as long on them.)  A batch, which moves no
 // particle, and staggered fields take the streams.
+// Large dense quadratic sets are faster in runs: a run stays long in a stencil and its
+// lane adds a particle in fewer instructions.  Runs / streams, ms: clustered 16 per cell
+// 8 M 0.339 / 0.351, 32 M 1.10 / 1.23, 13 per cell 32 M 1.18 / 1.27, 10 per cell 32 M 1.31
+// / 1.34, 6 per cell 32 M 1.58 / 1.50; uniform 16 per cell 32 M 1.35 / 1.32, 10 per cell
+// 1.31 / 1.21; below 5 M the streams' parts fill the GPU better (clustered 16 per cell 4 M
+// 0.239 / 0.211).
 static bool run_sums(int order, const picasso_bins& bins, int64_t n)
 {
     if (order != 2) return order == 1;
     double cells = 1.0;
     for (int d = 0; d < 3; ++d) cells *= bins.bin_extent[d];
-    return n < 4.0 * cells;
+    return n < 4.0 * cells || (n >= 11.0 * cells && n >= 5000000);
 }
 
 // Values of picasso_bins.p2g_lanes a call accepts (the P2G's lanes per particle
@@ -184,12 +190,16 @@ bool valid_lanes(int order, int lanes, bool stag)
 // 1 / 9 of an SM's share of the particles (about the warps of one wave at 14 per SM
 // where no item is filled), in sets below 300 000 particles down to 64.  Where most items are
 // shorter, the empty parts behind them (1.5 ns each) stay below a tenth of the time.
-// 2 M quadratic particles (P2G): 16 per cell, 546 items 194 -> 110 us; 8 per cell, 1152
-// items 134 -> 114 us; 4 per cell clustered 226 -> 165 us; 300 000: 75 -> 37 us, clustered
-// 159 -> 48 us.  12^3 cells of 4: 69 -> 19 us.
+// P2G streams from 3.5 M particles on: several waves of thirds of a full item, so that the
+// last one is not a wave of whole items (quadratic 8 per cell 6 M 0.335 -> 0.279 ms,
+// clustered 6 M 0.392 -> 0.323, 8 M 0.460 -> 0.405 ms, in runs 0.441; cubic clustered 8 M
+// 0.638 -> 0.533 ms), whole items again from 22 M on.
+// 2 M quadratic particles (P2G of the streams, uncut -> cut): 16 per cell, 546 items 194
+// -> 110 us; 8 per cell, 1152 items 134 -> 114 us (the runs took 111); 4 per cell clustered
+// 226 -> 165 us; 300 000: 75 -> 37 us, clustered 159 -> 48 us.  12^3 cells of 4: 69 -> 19 us.
 // A batch fills the GPU by its number of instances: there items are cut only where an
-// instance has less than 592, into at most 8 parts (24 instances up to 64^3 with the
-// other rule 1.92, so 1.76 ms).  Both are functions of the sizes alone, so that every
+// instance has at most 296 (two parts for each of 592), into at most 8 parts (24 instances
+// up to 64^3 with the other rule 1.92, so 1.76 ms).  Both are functions of the sizes alone, so that every
 // call on the same bins sums in the same order.
 // Runs (32 per item already) and the PolyPIC P2G's tiles are not cut.
 static void set_parts(TileP* tp, int64_t n, TileUse use)
@@ -204,7 +214,10 @@ static void set_parts(TileP* tp, int64_t n, TileUse use)
         part = 64;
         parts = std::min<int64_t>({few / items, n / tp->ntiles / part, 8});
     } else {
-        part = std::max<int64_t>({n / (148 * 9), std::min<int64_t>(256, n / few), 64});
+        const int64_t share = n / (148 * 9);
+        part = std::max<int64_t>({use == TileUse::streams && share > 2600
+                                      ? std::max<int64_t>(1366, share / 4) : share,
+                                  std::min<int64_t>(256, n / few), 64});
         parts = std::min<int64_t>({(std::min<int64_t>(tp->chunk, n) + part - 1) / part,
                                    1 + (1024 + n / 256) / items, 16});
     }
