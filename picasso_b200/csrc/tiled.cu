@@ -193,16 +193,18 @@ bool valid_lanes(int order, int lanes, bool stag)
 // P2G streams from 3.5 M particles on: several waves of thirds of a full item, so that the
 // last one is not a wave of whole items (quadratic 8 per cell 6 M 0.335 -> 0.279 ms,
 // clustered 6 M 0.392 -> 0.323, 8 M 0.460 -> 0.405 ms, in runs 0.441; cubic clustered 8 M
-// 0.638 -> 0.533 ms), whole items again from 22 M on.
+// 0.638 -> 0.533 ms), whole items again from 22 M on.  The linear G2P, whose particles cost
+// little beside the staging of their nodes, takes whole items there (uniform 16 per cell 4 M
+// 0.080 -> 0.068 ms).
 // 2 M quadratic particles (P2G of the streams, uncut -> cut): 16 per cell, 546 items 194
 // -> 110 us; 8 per cell, 1152 items 134 -> 114 us (the runs took 111); 4 per cell clustered
 // 226 -> 165 us; 300 000: 75 -> 37 us, clustered 159 -> 48 us.  12^3 cells of 4: 69 -> 19 us.
 // A batch fills the GPU by its number of instances: there items are cut only where an
 // instance has at most 296 (two parts for each of 592), into at most 8 parts (24 instances
-// up to 64^3 with the other rule 1.92, so 1.76 ms).  Both are functions of the sizes alone, so that every
-// call on the same bins sums in the same order.
+// up to 64^3 with the other rule 1.92, so 1.76 ms).  Both are functions of the sizes alone,
+// so that every call on the same bins sums in the same order.
 // Runs (32 per item already) and the PolyPIC P2G's tiles are not cut.
-static void set_parts(TileP* tp, int64_t n, TileUse use)
+static void set_parts(TileP* tp, int64_t n, TileUse use, int order)
 {
     const int64_t items = tp->ntiles + (n + tp->chunk - 1) / tp->chunk;
     const int64_t few = 148 * 4;
@@ -214,10 +216,10 @@ static void set_parts(TileP* tp, int64_t n, TileUse use)
         part = 64;
         parts = std::min<int64_t>({few / items, n / tp->ntiles / part, 8});
     } else {
-        const int64_t share = n / (148 * 9);
-        part = std::max<int64_t>({use == TileUse::streams && share > 2600
-                                      ? std::max<int64_t>(1366, share / 4) : share,
-                                  std::min<int64_t>(256, n / few), 64});
+        int64_t share = n / (148 * 9);
+        if (share > 2600 && use == TileUse::streams) share = std::max<int64_t>(1366, share / 4);
+        if (share > 2600 && use == TileUse::other && order == 1) share = tp->chunk;
+        part = std::max<int64_t>({share, std::min<int64_t>(256, n / few), 64});
         parts = std::min<int64_t>({(std::min<int64_t>(tp->chunk, n) + part - 1) / part,
                                    1 + (1024 + n / 256) / items, 16});
     }
@@ -279,7 +281,7 @@ bool make_tilep(const MeshP& mp, int order, const picasso_bins& bins, int64_t n,
     tp->items = bins.tile_items;
     tp->chunk = bins.chunk;
     if (!bins.tile_offset || !bins.tile_items || bins.chunk < 32) return false;
-    set_parts(tp, n, use);
+    set_parts(tp, n, use, order);
     return true;
 }
 
