@@ -13,14 +13,14 @@
 // loads per quadratic particle:
 //   * particles in any order read u_i from global memory, in the order of their
 //     stencils inside a warp where they have little locality (linear, quadratic;
-//     64^3 cells of 8: 0.214 ms as they come, 0.167 ms ordered, 90 % of the L1 data
+//     64^3 cells of 8: 0.214 ms as they come, 0.170 ms ordered, 90 % of the L1 data
 //     pipe);
 //   * large dense sets of cell-sorted particles (bins; g2p_tiles_pay) read it from a
-//     node tile in shared memory (128^3 8 per cell clustered: 0.92 ms from global
-//     memory, 0.71 ms).
+//     node tile in shared memory (128^3 8 per cell clustered: 0.97 ms from global
+//     memory, 0.74 ms).
 // Against the form it replaces (node by node, every thread storing its row):
-// sorted quadratic 128^3 1.28 -> 0.71 ms, cubic with advection 64^3 0.44 -> 0.17
-// ms, unsorted quadratic 64^3 0.224 -> 0.165 ms, the faces of a 45 x 38 x 53 box
+// sorted quadratic 128^3 1.28 -> 0.74 ms, cubic with advection 64^3 0.44 -> 0.17
+// ms, unsorted quadratic 64^3 0.224 -> 0.170 ms, the faces of a 45 x 38 x 53 box
 // 0.38 -> 0.14 ms.
 #pragma once
 

@@ -1,6 +1,6 @@
-// FP32 tiled P2G in runs: the P2G of linear splines and of sparse quadratic sets
-// (run_sums in tiled.cu says where and why; the other sets take the streams of
-// p2g_item in tiled.cuh).
+// FP32 tiled P2G in runs: the P2G of linear splines and of sparse and of large dense
+// quadratic sets (run_sums in tiled.cu says where and why; the other sets take the
+// streams of p2g_item in tiled.cuh).
 //
 // A work item's sorted particles are cut into 32 contiguous runs, one per lane.
 // Consecutive particles of a run mostly share a stencil, whose sums (4 fields x K^3

@@ -510,7 +510,7 @@ __device__ __forceinline__ void p2g_rows(const P2GArgs& A, int64_t t, int64_t a,
 // the shared-memory pipe at 14 warps per SM; 20 warps, tile (4, 4, 8), are no
 // faster).  Measured against one lane (cubic: 4) per particle and stream, with
 // up to 108 sums per lane: cubic 128^3 8 per cell 1.52 -> 0.85 ms, quadratic 256^3
-// 8 per cell clustered 5.53 -> 5.24 ms, a batch of 24 small problems 2.16 -> 1.07
+// 8 per cell clustered 5.53 -> 5.33 ms, a batch of 24 small problems 2.16 -> 1.07
 // ms.  The next step's entry is read before the current one is used (quadratic
 // 5.80 -> 5.35 ms, cubic 0.95 -> 0.85 ms).  Not kept: the streams that move found
 // one by one (5.50 ms instead of testing each); packed FP32 pairs, whose

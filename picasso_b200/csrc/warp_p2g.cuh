@@ -22,9 +22,9 @@
 //
 // Measured (B200, against one thread per particle adding every contribution to
 // the grid, which the L2's 200 G additions/s bound): quadratic 128^3 8 per cell
-// clustered and sorted 31.7 -> 1.47 ms, 64^3 unsorted 1.28 -> 0.48 ms, shuffled
+// clustered and sorted 31.7 -> 1.52 ms, 64^3 unsorted 1.28 -> 0.49 ms, shuffled
 // 1.03 -> 0.52 ms (108 additions per particle at 440 G/s: whole sectors);
-// cubic 64^3 sorted 4.83 -> 0.36 ms; linear 128^3 sorted 3.51 -> 1.10 ms; the
+// cubic 64^3 sorted 4.83 -> 0.32 ms; linear 128^3 sorted 3.51 -> 1.10 ms; the
 // faces of a 45 x 38 x 53 box, shuffled, 0.48 -> 0.35 ms.  A sorted quadratic
 // particle costs about 60 ps plus 290 ps per stencil; what bounds it is the
 // latency of a run's chain (table, contraction, node values) at 16 warps per
